@@ -110,7 +110,7 @@ int reinit_run(gb2d_ctx* c, int src, int a, int b) {
   launch_reinit_sign(c->stream, c, c->phi_buf[src], c->sign);
   int cur = src, nxt = a;
   for (int it = 0; it < c->prm.reinit_iterations; ++it) {
-    launch_reinit_sweep(c->stream, c, c->phi_buf[cur], c->phi_buf[nxt], c->sign, dtau, mixed);
+    launch_reinit_sweep(c->stream, c, c->phi_buf[cur], c->phi_buf[nxt], c->sign, dtau, mixed, it < 2);
     int prev = cur;
     cur = nxt;
     nxt = (prev == src) ? b : prev;
@@ -902,7 +902,7 @@ int gb2d_reinit_sweep_apply(gb2d_ctx* c, const double* phi_in, const double* sig
   GB2D_CUDA_TRY(c, cudaMemcpyAsync(c->phi_buf[A], phi_in, nphi * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   GB2D_CUDA_TRY(c, cudaMemcpyAsync(c->sign, sign, ni * nj * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   launch_reinit_sweep(c->stream, c, c->phi_buf[A], c->phi_buf[B], c->sign, c->base.dx / (double)c->prm.reinit_scaling,
-                      c->prm.advection_precision == GB2D_PRECISION_MIXED);
+                      c->prm.advection_precision == GB2D_PRECISION_MIXED, 1);
   GB2D_CUDA_TRY(c, cudaMemcpyAsync(phi_out, c->phi_buf[B], nphi * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   return sync_check(c, "reinit_sweep_apply");
 }

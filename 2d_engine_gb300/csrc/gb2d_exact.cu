@@ -33,6 +33,7 @@ __device__ __forceinline__ bool prod_ge0(double x, double y) {
 // FillGhostCellsFrom (FIELD_STRUCTURE_2D.h:374-449): interior copied, each ghost
 // layer copies the second interior line, corners untouched.
 __global__ void k_fill_ghost_copy(double* dst_a, int gd, const double* __restrict__ src_a, int gs, int nI, int nJ, int g) {
+  pdl_enter();
   DField d = dfield(dst_a, gd, nI, nJ);
   DField s = dfield((double*)src_a, gs, nI, nJ);
   GB_FOR_IJ(ii, jj, nI + 2 * g, nJ + 2 * g) {
@@ -52,6 +53,7 @@ __global__ void k_fill_ghost_copy(double* dst_a, int gd, const double* __restric
 // reference's layer order: left/bottom outermost first (the outer layer reads
 // the previous inner value), right/top innermost first.
 __global__ void k_extrapolate(double* a, int g, int nI, int nJ) {
+  pdl_enter();
   DField f = dfield(a, g, nI, nJ);
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < nJ) {
@@ -91,14 +93,96 @@ struct LSArgs {
   int ni, nj;
   double odx, ody, eps;
   float odx_f, ody_f, eps_f;  // the same in FP32 for the FP32 flux path
+  int fast;                   // epsilon is in weno5_side_fast's range (and dx in [2^-300, 2^300], for dtau s h)
 };
+
+// Reads phi's interior at (i, j), where positions outside it hold the second interior
+// line as in the reference's ghost-filled scratch copy (scalar_field_ghost, ghost 3).
+__device__ __forceinline__ double ghosted(const DField& s, int i, int j) {
+  i = i < 0 ? 1 : (i >= s.nI ? s.nI - 2 : i);
+  j = j < 0 ? 1 : (j >= s.nJ ? s.nJ - 2 : j);
+  return __ldg(&GB_AT(s, i, j));
+}
+
+// One tile of the exact FP64 sweeps: kExX x kExY nodes with every WENO first difference
+// o (q[k+1] - q[k]) formed once (12 per node when each node forms its own, 2.8 to 3.4
+// here); dxs[r][c + k] is difference k of node (c, r) along x, dys[r + k][c] along y.
+constexpr int kExX = 32, kExY = 4;
+struct ExactTile {
+  double ph[kExY + 6][kExX + 6];
+  double dxs[kExY][kExX + 5], dys[kExY + 5][kExX];
+};
+
+// Stages the tile at (i0, j0); true in every thread where all differences are in
+// weno5_side_fast's range.
+__device__ __forceinline__ bool stage_exact(ExactTile& t, const DField& src, const LSArgs& a, int i0, int j0) {
+  constexpr int NT = 2 * kExX * kExY, SW = kExX + 6, DW = kExX + 5;
+  const int tid = threadIdx.x;
+  for (int k = tid; k < SW * (kExY + 6); k += NT) t.ph[k / SW][k % SW] = ghosted(src, i0 - 3 + k % SW, j0 - 3 + k / SW);
+  __syncthreads();
+  bool ok = true;
+  for (int k = tid; k < kExY * DW; k += NT) {
+    const int c = k % DW, r = k / DW;
+    const double d = a.odx * (t.ph[r + 3][c + 1] - t.ph[r + 3][c]);
+    ok = ok && weno5_in_range(d);
+    t.dxs[r][c] = d;
+  }
+  for (int k = tid; k < (kExY + 5) * kExX; k += NT) {
+    const int c = k % kExX, r = k / kExX;
+    const double d = a.ody * (t.ph[r + 1][c + 3] - t.ph[r][c + 3]);
+    ok = ok && weno5_in_range(d);
+    t.dys[r][c] = d;
+  }
+  return __syncthreads_and(ok && a.fast);
+}
+
+// Difference k (0..5) of node (c, r) along direction dir (0: x, 1: y).
+__device__ __forceinline__ double ex_diff(const ExactTile& t, int dir, int c, int r, int k) {
+  return dir == 0 ? t.dxs[r][c + k] : t.dys[r + k][c];
+}
+// One-sided derivative of node (c, r): side 0 the minus, side 1 the plus one.
+template <bool FAST>
+__device__ __forceinline__ double ex_side(const ExactTile& t, int dir, int c, int r, int side, double eps) {
+  const double* d = dir == 0 ? &t.dxs[r][c] : &t.dys[r][c];
+  const int st = dir == 0 ? 1 : kExX, first = side ? 5 * st : 0, step = side ? -st : st;
+  const double a1 = d[first], a2 = d[first + step], a3 = d[first + 2 * step], a4 = d[first + 3 * step], a5 = d[first + 4 * step];
+  if (FAST) return weno5_side_fast(a1, a2, a3, a4, a5, eps);
+  return weno5_side<double>(a1, a2, a3, a4, a5, eps);
+}
+// g g, or 0 for |g| < 2^-400; |g| < 2^500.
+__device__ __forceinline__ double sqr_flush(double g) {
+  return ((unsigned)(__double_as_longlong(g) >> 52) & 0x7ffu) < 1023u - 400u ? 0.0 : mul_rn(g, g);
+}
+// Out of line: the general forms serve differences outside the fast range only.
+__device__ __noinline__ double ex_side_general(const ExactTile& t, int dir, int c, int r, int side, double eps) {
+  return ex_side<false>(t, dir, c, r, side, eps);
+}
+
+// Copies src's ghost ring (width 2) to dst, a block's threads each taking every
+// n-th element from the first-th.
+__device__ __forceinline__ void copy_ring(const DField& src, const DField& dst, int first, int n) {
+  const int W = src.nI + 4, rows = 4 * W, total = rows + 4 * src.nJ;
+  for (int k = first; k < total; k += n) {
+    int i, j;
+    if (k < rows) {
+      const int y = k / W;
+      i = k - y * W - 2;
+      j = y < 2 ? y - 2 : src.nJ + y - 2;
+    } else {
+      const int y = (k - rows) >> 2, x = (k - rows) & 3;
+      i = x < 2 ? x - 2 : src.nI + x - 2;
+      j = y;
+    }
+    GB_AT(dst, i, j) = GB_AT(src, i, j);
+  }
+}
 
 // WENO5th (ADVECTION_METHOD_2D.h:508-663) for the node-grid level set: writes
 // dst's interior from src, copies src's ghost ring (the sweep leaves phi's own
 // ghosts to the caller's extrapolation).
-template <bool MIXED>
-__global__ void k_weno5_advect(const double* __restrict__ src_a, double* __restrict__ dst_a, const double* __restrict__ ua_a,
-                               const double* __restrict__ va_a, LSArgs a, DtArg dt_arg) {
+__global__ void k_weno5_advect_mixed(const double* __restrict__ src_a, double* __restrict__ dst_a, const double* __restrict__ ua_a,
+                                     const double* __restrict__ va_a, LSArgs a, DtArg dt_arg) {
+  pdl_enter();
   int ni = a.ni, nj = a.nj;
   const double dt = dt_arg.get();
   int W = ni + 4, H = nj + 4;
@@ -115,28 +199,53 @@ __global__ void k_weno5_advect(const double* __restrict__ src_a, double* __restr
   double u = (__ldg(&GB_AT(ua, i + 1, j)) + __ldg(&GB_AT(ua, i, j))) * 0.5;
   double v = (__ldg(&GB_AT(va, i, j + 1)) + __ldg(&GB_AT(va, i, j))) * 0.5;
   double fx, fy;
-  if (MIXED) {
-    float m, p;
-    gather_x(src, i, j, q);
-    weno5_pair_f32(q, a.odx_f, a.eps_f, m, p);
-    fx = gtz(u) ? widen(m) : widen(p);
-    gather_y(src, i, j, q);
-    weno5_pair_f32(q, a.ody_f, a.eps_f, m, p);
-    fy = gtz(v) ? widen(m) : widen(p);
-  } else {
-    double m, p;
-    gather_x(src, i, j, q);
-    weno5_pair(q, a.odx, a.eps, m, p);
-    fx = gtz(u) ? m : p;
-    gather_y(src, i, j, q);
-    weno5_pair(q, a.ody, a.eps, m, p);
-    fy = gtz(v) ? m : p;
-  }
+  float m, p;
+  gather_x(src, i, j, q);
+  weno5_pair_f32(q, a.odx_f, a.eps_f, m, p);
+  fx = gtz(u) ? widen(m) : widen(p);
+  gather_y(src, i, j, q);
+  weno5_pair_f32(q, a.ody_f, a.eps_f, m, p);
+  fy = gtz(v) ? widen(m) : widen(p);
   GB_AT(dst, i, j) = GB_AT(src, i, j) - dt * (u * fx + v * fy);
+}
+
+// The exact FP64 sweep, bound by the FP64 pipe: each node evaluates the upwind side
+// only (one WENO derivative per direction instead of two), from differences formed
+// once per tile, the x and y directions on two threads.  The grid's last block row
+// copies the ghost ring.
+__global__ void __launch_bounds__(2 * kExX* kExY) k_weno5_advect_exact(const double* __restrict__ src_a, double* __restrict__ dst_a,
+                                                                     const double* __restrict__ ua_a, const double* __restrict__ va_a,
+                                                                     LSArgs a, DtArg dt_arg) {
+  pdl_enter();
+  constexpr int NN = kExX * kExY;
+  __shared__ ExactTile t;
+  __shared__ double vfy[NN];
+  const DField src = dfield((double*)src_a, 2, a.ni, a.nj), dst = dfield(dst_a, 2, a.ni, a.nj);
+  if (blockIdx.y == gridDim.y - 1) {
+    copy_ring(src, dst, blockIdx.x * (2 * NN) + threadIdx.x, gridDim.x * (2 * NN));
+    return;
+  }
+  const int i0 = (int)blockIdx.x * kExX, j0 = (int)blockIdx.y * kExY;
+  const bool fast = stage_exact(t, src, a, i0, j0);
+  const int node = threadIdx.x & (NN - 1), dir = threadIdx.x / NN;
+  const int c = node & (kExX - 1), r = node / kExX, i = i0 + c, j = j0 + r;
+  const bool in = i < a.ni && j < a.nj;
+  double wf = 0;  // u fx or v fy
+  if (in) {
+    const DField ua = dfield((double*)ua_a, 3, a.ni + 1, a.nj), va = dfield((double*)va_a, 3, a.ni, a.nj + 1);
+    const double w = dir == 0 ? (__ldg(&GB_AT(ua, i + 1, j)) + __ldg(&GB_AT(ua, i, j))) * 0.5
+                              : (__ldg(&GB_AT(va, i, j + 1)) + __ldg(&GB_AT(va, i, j))) * 0.5;
+    const int side = gtz(w) ? 0 : 1;
+    wf = w * (fast ? ex_side<true>(t, dir, c, r, side, a.eps) : ex_side_general(t, dir, c, r, side, a.eps));
+  }
+  if (dir == 1) vfy[node] = wf;
+  __syncthreads();
+  if (in && dir == 0) GB_AT(dst, i, j) = t.ph[r + 3][c + 3] - dt_arg.get() * (wf + vfy[node]);
 }
 
 // Sign function of Reinitialization (EULERIAN_FLUID_SOLVER_2D.h:2431-2435).
 __global__ void k_reinit_sign(const double* __restrict__ phi_a, double* __restrict__ S, int ni, int nj, double dx) {
+  pdl_enter();
   DField phi = dfield((double*)phi_a, 2, ni, nj);
   GB_FOR_IJ(i, j, ni, nj) {
     const size_t t = (size_t)j * ni + i;
@@ -145,10 +254,10 @@ __global__ void k_reinit_sign(const double* __restrict__ phi_a, double* __restri
   }
 }
 
-// WENO5thReinitialization (ADVECTION_METHOD_2D.h:1401-1658).
-template <bool MIXED>
-__global__ void k_reinit_sweep(const double* __restrict__ src_a, double* __restrict__ dst_a, const double* __restrict__ S, LSArgs a,
-                               double dtau) {
+// WENO5thReinitialization (ADVECTION_METHOD_2D.h:1401-1658), the mixed form.
+__global__ void k_reinit_sweep_mixed(const double* __restrict__ src_a, double* __restrict__ dst_a, const double* __restrict__ S, LSArgs a,
+                                     double dtau) {
+  pdl_enter();
   int ni = a.ni, nj = a.nj;
   int W = ni + 4, H = nj + 4;
   int ix = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y * blockDim.y + threadIdx.y;
@@ -162,24 +271,122 @@ __global__ void k_reinit_sweep(const double* __restrict__ src_a, double* __restr
   }
   double q[7];
   double out = old;
-  if (MIXED) {
-    float mx, px, my, py, h;
-    gather_x(src, i, j, q);
-    weno5_pair_f32(q, a.odx_f, a.eps_f, mx, px);
-    gather_y(src, i, j, q);
-    weno5_pair_f32(q, a.ody_f, a.eps_f, my, py);
-    double s = __ldg(&S[i + (size_t)j * ni]);
-    if (godunov_h<float>(narrow(s), mx, px, my, py, h)) out = old - dtau * s * widen(h);
-  } else {
-    double mx, px, my, py, h;
-    gather_x(src, i, j, q);
-    weno5_pair(q, a.odx, a.eps, mx, px);
-    gather_y(src, i, j, q);
-    weno5_pair(q, a.ody, a.eps, my, py);
-    double s = __ldg(&S[i + (size_t)j * ni]);
-    if (godunov_h<double>(s, mx, px, my, py, h)) out = old - dtau * s * h;
-  }
+  float mx, px, my, py, h;
+  gather_x(src, i, j, q);
+  weno5_pair_f32(q, a.odx_f, a.eps_f, mx, px);
+  gather_y(src, i, j, q);
+  weno5_pair_f32(q, a.ody_f, a.eps_f, my, py);
+  double s = __ldg(&S[i + (size_t)j * ni]);
+  if (godunov_h<float>(narrow(s), mx, px, my, py, h)) out = old - dtau * s * widen(h);
   GB_AT(dst, i, j) = out;
+}
+
+// Godunov choice of one direction from certain signs of s and of the one-sided
+// derivatives (godunov_h's cases): 0 the minus side, 1 the plus side, 2 neither
+// (rarefaction), 3 both values are needed (a shock, or a sign that is not certain).
+// With |s| >= 2^-100 and derivatives above weno5_sign's margin no product s m
+// underflows, so the products' signs are the signs' products.
+__device__ __forceinline__ int godunov_case(int ss, int sm, int sp) {
+  const int a = ss * sm, b = ss * sp;
+  return a > 0 && b > 0 ? 0 : a < 0 && b < 0 ? 1 : a < 0 && b > 0 ? 2 : 3;
+}
+
+// The exact FP64 sweep, bound by the FP64 and integer pipes: a node's update uses one
+// of its two one-sided derivatives per direction (or neither, in a rarefaction), and
+// which one follows from their signs.  FP32 evaluations of the candidate stencils
+// settle the signs almost everywhere; a thread evaluates the chosen side of one
+// direction of its node exactly, and the few that need both values (shocks, flat
+// directions) put the second evaluation on the block's list, which the block works
+// off densely.  The update has the bits of evaluating all four derivatives.  ring: the
+// grid's last block row copies src's ghost ring (needed until both buffers of the
+// sweeps hold it).
+// One level-set TVD-RK3 with its 75 sweeps at 512^2: 22.6 ms with four derivatives per
+// node in FP64 divisions and products (578 FP64 instructions per node), 6.4 ms with the
+// chosen sides, the differences shared and the divisions on the integer pipes (160), 3.5
+// ms with every product there too (74).  The FP64 pipe is half busy then and the wait for
+// dependent results shows: 5 blocks of 48 registers per SM 3.44 ms, 4 of 64 3.62, 3 of 79
+// 3.97.  Tiles of 32 x 8 nodes are 3% slower, and 1.3 times as slow on small grids, where
+// they leave SMs idle; 32 x 2 ones are no faster there.
+__global__ void __launch_bounds__(2 * kExX * kExY, 5) k_reinit_sweep_exact(const double* __restrict__ src_a, double* __restrict__ dst_a,
+                                                                     const double* __restrict__ S, LSArgs a, double dtau, int ring) {
+  pdl_enter();
+  constexpr int NN = kExX * kExY, NT = 2 * NN;  // nodes and threads: thread dir NN + node
+  __shared__ ExactTile t;
+  __shared__ double plus[NT], dy_own[NN];
+  __shared__ unsigned short list[NT];
+  __shared__ signed char dy_pick[NN];
+  __shared__ int count;
+  const DField src = dfield((double*)src_a, 2, a.ni, a.nj), dst = dfield(dst_a, 2, a.ni, a.nj);
+  if (ring && blockIdx.y == gridDim.y - 1) {
+    copy_ring(src, dst, blockIdx.x * NT + threadIdx.x, gridDim.x * NT);
+    return;
+  }
+  const int tid = threadIdx.x, i0 = (int)blockIdx.x * kExX, j0 = (int)blockIdx.y * kExY;
+  if (tid == 0) count = 0;
+  const bool fast = stage_exact(t, src, a, i0, j0);
+  const int node = tid & (NN - 1), dir = tid / NN, c = node & (kExX - 1), r = node / kExX, i = i0 + c, j = j0 + r;
+  const bool in = i < a.ni && j < a.nj;
+  const double s = in ? __ldg(&S[i + (size_t)j * a.ni]) : 0.0;
+  const long long sb = __double_as_longlong(s);
+  const bool sfast = (sb & kAbsBits) >= ((1023LL - 100) << 52) && (sb & kAbsBits) <= kInfBits;  // |s| >= 2^-100
+  int pick = in ? 3 : 2;
+  if (in && fast && sfast) {
+    float d[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) d[k] = narrow(ex_diff(t, dir, c, r, k));
+    pick = godunov_case(sb < 0 ? -1 : 1, weno5_sign(d[0], d[1], d[2], d[3], d[4]), weno5_sign(d[5], d[4], d[3], d[2], d[1]));
+  }
+  if (in && fast && pick == 3) list[atomicAdd(&count, 1)] = (unsigned short)tid;
+  __syncthreads();
+  double own = 0;
+  if (fast) {
+    const int n = count, rounds = 1 + (n + NT - 1) / NT;
+#pragma unroll 1
+    for (int k = 0; k < rounds; ++k) {
+      const int m = (k - 1) * NT + tid;
+      const int item = k == 0 ? tid : m < n ? (int)list[m] : 0;
+      if (k == 0 ? pick == 2 : m >= n) continue;
+      const int nd = item & (NN - 1), side = k == 0 ? pick == 1 : 1;
+      const double f = ex_side<true>(t, item / NN, nd & (kExX - 1), nd / kExX, side, a.eps);
+      if (k == 0) own = f;
+      else plus[item] = f;
+    }
+    __syncthreads();
+  } else if (in) {
+    own = ex_side_general(t, dir, c, r, 0, a.eps);
+    plus[tid] = ex_side_general(t, dir, c, r, 1, a.eps);
+  }
+  if (in && pick == 3) {
+    const double p = plus[tid];
+    pick = godunov_pick(s, own, p, dir == 0);
+    if (pick == 1) own = p;
+  }
+  if (dir == 1) {
+    dy_own[node] = own;
+    dy_pick[node] = (signed char)pick;
+  }
+  __syncthreads();
+  if (!in || dir == 1) return;
+  const double old = t.ph[r + 3][c + 3], gy = dy_own[node];
+  const int ypick = dy_pick[node];
+  if (pick < 0 || ypick < 0) {
+    GB_AT(dst, i, j) = old;
+    return;
+  }
+  double h = -1.0;
+  if (fast && sfast) {  // the same values: |g| < 2^-400 changes neither the sum's root nor h
+    const double g2 = (pick != 2 ? sqr_flush(own) : 0.0) + (ypick != 2 ? sqr_flush(gy) : 0.0);
+    if (pick != 2 || ypick != 2) h = sqrt_rn(g2) - 1.0;
+    GB_AT(dst, i, j) = old - mul_rn(mul_rn(s, dtau), h);
+    return;
+  }
+  if (pick != 2 && ypick != 2)
+    h = sqrt(own * own + gy * gy) - 1.0;
+  else if (pick != 2)
+    h = sqrt(own * own) - 1.0;
+  else if (ypick != 2)
+    h = sqrt(gy * gy) - 1.0;
+  GB_AT(dst, i, j) = old - dtau * s * h;
 }
 
 // The mixed reinit sweep, tiled: the WENO first differences of a node and of its
@@ -187,10 +394,11 @@ __global__ void k_reinit_sweep(const double* __restrict__ src_a, double* __restr
 // as the ghost-filled copy maps them) and forms every FP64 difference once (2.8 per node
 // instead of 12; FP64 issue is this kernel's bound), narrowed to FP32 in shared memory.
 // Each node then reads its 6 + 6 differences: the same values as the per-node gathers,
-// so the results equal k_reinit_sweep<true>'s bit for bit.
+// so the results equal k_reinit_sweep_mixed's bit for bit.
 constexpr int kRtX = 32, kRtY = 8;
 __global__ void __launch_bounds__(kRtX* kRtY) k_reinit_sweep_tiled(const double* __restrict__ src_a, double* __restrict__ dst_a,
                                                                     const double* __restrict__ S, LSArgs a, double dtau) {
+  pdl_enter();
   __shared__ double ph[kRtY + 6][kRtX + 6];
   __shared__ float dxs[kRtY][kRtX + 5];
   __shared__ float dys[kRtY + 5][kRtX];
@@ -238,6 +446,7 @@ __global__ void __launch_bounds__(kRtX* kRtY) k_reinit_sweep_tiled(const double*
 
 // Shu-Osher blend of the TVD-RK3 stages (EULERIAN_FLUID_SOLVER_2D.h:1706-1741): interior only.
 __global__ void k_blend(const double* __restrict__ keep_a, double* phi_a, int ni, int nj, double c0, double c1) {
+  pdl_enter();
   DField keep = dfield((double*)keep_a, 2, ni, nj), phi = dfield(phi_a, 2, ni, nj);
   GB_FOR_IJ(i, j, ni, nj) {
     GB_AT(phi, i, j) = c0 * GB_AT(keep, i, j) + c1 * GB_AT(phi, i, j);
@@ -260,6 +469,7 @@ struct EnoArgs {
 template <bool MIXED>
 __global__ void k_eno3(double* __restrict__ u_a, double* __restrict__ v_a, const double* __restrict__ ua_a, const double* __restrict__ va_a,
                        EnoArgs a, DtArg dt_arg) {
+  pdl_enter();
   int ni = a.ni, nj = a.nj;
   const double dt = dt_arg.get();
   DField ua = dfield((double*)ua_a, 3, ni + 1, nj), va = dfield((double*)va_a, 3, ni, nj + 1);
@@ -590,7 +800,9 @@ inline dim3 grid2d(int W, int H, dim3 blk) { return dim3((W + blk.x - 1) / blk.x
 
 LSArgs ls_args(const gb2d_ctx* c) {
   return LSArgs{c->grid.ni, c->grid.nj, c->base.odx, c->base.ody, c->prm.weno_epsilon,
-                (float)c->base.odx, (float)c->base.ody, (float)c->prm.weno_epsilon};
+                (float)c->base.odx, (float)c->base.ody, (float)c->prm.weno_epsilon,
+                c->prm.weno_epsilon >= 0x1p-100 && c->prm.weno_epsilon <= 0x1p100 &&
+                    c->base.dx >= 0x1p-300 && c->base.dx <= 0x1p300};
 }
 
 AsmArgs asm_args(const gb2d_ctx* c, double dt) {
@@ -612,8 +824,8 @@ AsmArgs asm_args(const gb2d_ctx* c, double dt) {
   return a;
 }
 
-// Self-check of div_by<3> / div_by<6> against the IEEE division: n pseudo-random
-// 64-bit patterns (every exponent, sign, NaN and infinity included) and n more
+// Self-check of div_by<3> / div_by<6> (and, on normal operands, of the functions of
+// gb2d_exact_math.cuh) against the IEEE operations: n pseudo-random 64-bit patterns (every exponent, sign, NaN and infinity included) and n more
 // with exponents in the range the schemes meet; counts results whose bits differ
 // (NaN == NaN).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
@@ -634,6 +846,18 @@ __global__ void k_check_div_by(unsigned long long n, unsigned long long seed, un
     const bool ok3 = __double_as_longlong(q3) == __double_as_longlong(r3) || (isnan(q3) && isnan(r3));
     const bool ok6 = __double_as_longlong(q6) == __double_as_longlong(r6) || (isnan(q6) && isnan(r6));
     local += (ok3 ? 0 : 1) + (ok6 ? 0 : 1);
+    // exponents in [-300, 300); every eighth significand has a long run of zeros or ones
+    auto normal = [](unsigned long long x) {
+      if ((x >> 60) == 1) x &= ~0x3ffffffffull;
+      if ((x >> 60) == 2) x |= 0xfffffffffull;
+      return __longlong_as_double((long long)((x & 0x800fffffffffffffull) | ((1023ull - 300 + (x >> 40) % 600) << 52)));
+    };
+    const double x = normal(mix64(b + 1)), y = normal(mix64(b + 2)), ax = fabs(x), ay = fabs(y);
+    auto differs = [](double u, double v) { return __double_as_longlong(u) != __double_as_longlong(v) ? 1 : 0; };
+    local += differs(div_pos(ax, ay), ax / ay) + differs(div_pos(0.3, ay), 0.3 / ay) + differs(mul_rn(x, y), x * y) +
+             differs(mul_rn(x, x), x * x) + differs(mul_rn(x, 7.0), x * 7.0) + differs(mul_rn(x, 13.0 / 12.0), x * (13.0 / 12.0)) +
+             differs(third_rn<0>(x), x / 3.0) + differs(third_rn<1>(y), y / 6.0) + differs(sqrt_rn(ax), sqrt(ax)) +
+             differs(sqrt_rn(ay * ay), sqrt(ay * ay));
   }
   if (local) atomicAdd(bad, local);
 }
@@ -662,45 +886,51 @@ void launch_fill_ghost_copy(cudaStream_t s, double* dst, int gd, const double* s
 
 void launch_extrapolate_ghosts(cudaStream_t s, double* f, int g, int nI, int nJ) {
   int n = nI > nJ ? nI : nJ;
-  k_extrapolate<<<blocks_for(n, 128), 128, 0, s>>>(f, g, nI, nJ);
+  pdl_launch(s, blocks_for(n, 128), 128, 0, k_extrapolate, f, g, nI, nJ);
   GB_LAUNCHED(1);
 }
 
 void launch_weno5_advect(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, double dt, int mixed) {
-  dim3 blk(32, 8);
-  dim3 grd = grid2d(c->grid.ni + 4, c->grid.nj + 4, blk);
-  if (mixed)
-    k_weno5_advect<true><<<grd, blk, 0, s>>>(src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
-  else
-    k_weno5_advect<false><<<grd, blk, 0, s>>>(src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
+  const int ni = c->grid.ni, nj = c->grid.nj;
+  if (mixed) {
+    dim3 blk(32, 8);
+    pdl_launch(s, grid2d(ni + 4, nj + 4, blk), blk, 0, k_weno5_advect_mixed, src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
+  } else {
+    const dim3 grd((ni + kExX - 1) / kExX, (nj + kExY - 1) / kExY + 1);
+    pdl_launch(s, grd, 2 * kExX * kExY, 0, k_weno5_advect_exact, src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
+  }
   GB_LAUNCHED(1);
 }
 
 void launch_reinit_sign(cudaStream_t s, const gb2d_ctx* c, const double* phi, double* S) {
-  k_reinit_sign<<<grid_ij(c->grid.ni, c->grid.nj), kThreads, 0, s>>>(phi, S, c->grid.ni, c->grid.nj, c->base.dx);
+  pdl_launch(s, grid_ij(c->grid.ni, c->grid.nj), kThreads, 0, k_reinit_sign, phi, S, c->grid.ni, c->grid.nj, c->base.dx);
   GB_LAUNCHED(1);
 }
 
-void launch_reinit_sweep(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, const double* S, double dtau, int mixed) {
-  dim3 blk(32, 8);
-  dim3 grd = grid2d(c->grid.ni + 4, c->grid.nj + 4, blk);
+void launch_reinit_sweep(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, const double* S, double dtau, int mixed,
+                         int ring) {
+  const int ni = c->grid.ni, nj = c->grid.nj;
   // GB2D_REINIT_UNTILED=1 (read once) selects the per-node mixed kernel, which the tiled one
   // must equal bit for bit.
   static const bool untiled = [] {
     const char* e = getenv("GB2D_REINIT_UNTILED");
     return e && e[0] == '1';
   }();
-  if (mixed && !untiled)
-    k_reinit_sweep_tiled<<<grd, blk, 0, s>>>(src, dst, S, ls_args(c), dtau);
-  else if (mixed)
-    k_reinit_sweep<true><<<grd, blk, 0, s>>>(src, dst, S, ls_args(c), dtau);
-  else
-    k_reinit_sweep<false><<<grd, blk, 0, s>>>(src, dst, S, ls_args(c), dtau);
+  dim3 blk(32, 8);
+  dim3 grd = grid2d(ni + 4, nj + 4, blk);
+  if (mixed && !untiled) {
+    pdl_launch(s, grd, blk, 0, k_reinit_sweep_tiled, src, dst, S, ls_args(c), dtau);
+  } else if (mixed) {
+    pdl_launch(s, grd, blk, 0, k_reinit_sweep_mixed, src, dst, S, ls_args(c), dtau);
+  } else {
+    const dim3 g((ni + kExX - 1) / kExX, (nj + kExY - 1) / kExY + (ring ? 1 : 0));
+    pdl_launch(s, g, 2 * kExX * kExY, 0, k_reinit_sweep_exact, src, dst, S, ls_args(c), dtau, ring);
+  }
   GB_LAUNCHED(1);
 }
 
 void launch_blend(cudaStream_t s, const gb2d_ctx* c, const double* keep, double* phi, double c0, double c1) {
-  k_blend<<<grid_ij(c->grid.ni, c->grid.nj), kThreads, 0, s>>>(keep, phi, c->grid.ni, c->grid.nj, c0, c1);
+  pdl_launch(s, grid_ij(c->grid.ni, c->grid.nj), kThreads, 0, k_blend, keep, phi, c->grid.ni, c->grid.nj, c0, c1);
   GB_LAUNCHED(1);
 }
 

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <utility>
 
 #include "gb2d.h"
 
@@ -63,6 +64,32 @@ __device__ __forceinline__ float narrow(double d) {
   else
     bits = s | ((unsigned)e << 23) | (unsigned)((b >> 29) & 0x7fffffull);
   return __uint_as_float(bits);
+}
+
+// Programmatic dependent launch inside chains of kernels on one stream: wait until
+// the previous kernel in the stream has completed (its writes visible), then let the
+// next kernel start launching, so launch latency and block scheduling overlap
+// this kernel's tail instead of following it.  Both are no-ops for kernels
+// launched without the programmatic-serialization attribute.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launch with programmatic stream serialization (see pdl_enter).
+template <typename... P, typename... A>
+void pdl_launch(cudaStream_t s, dim3 grid, dim3 block, size_t smem, void (*k)(P...), A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
 // ---- level construction -----------------------------------------------------
@@ -208,7 +235,9 @@ unsigned long long check_div_by(unsigned long long n, unsigned long long seed, i
 void launch_extrapolate_ghosts(cudaStream_t s, double* f, int g, int nI, int nJ);
 void launch_weno5_advect(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, double dt, int mixed);
 void launch_reinit_sign(cudaStream_t s, const gb2d_ctx* c, const double* phi, double* S);
-void launch_reinit_sweep(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, const double* S, double dtau, int mixed);
+// ring: copy src's ghost ring to dst (the mixed sweeps always do).
+void launch_reinit_sweep(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, const double* S, double dtau, int mixed,
+                         int ring);
 void launch_blend(cudaStream_t s, const gb2d_ctx* c, const double* keep, double* phi, double c0, double c1);
 void launch_eno3(cudaStream_t s, const gb2d_ctx* c, double dt);
 void launch_curvature(cudaStream_t s, const gb2d_ctx* c, const double* phi, double* kappa, int* flag);

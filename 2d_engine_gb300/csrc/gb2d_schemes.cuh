@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include "gb2d_exact_math.cuh"
 #include "gb2d_internal.cuh"
 
 namespace gb2d {
@@ -131,13 +132,53 @@ __device__ __forceinline__ R weno5_side(R a1, R a2, R a3, R a4, R a5, R eps) {
          w3 * (cdiv3(a3) + cdiv6(a4 * R(5)) - cdiv6(a5));
 }
 
-// Exact FP64 pair: q[0..6] are values at offsets -3..+3 (ADVECTION_METHOD_2D.h:521-543).
-__device__ __forceinline__ void weno5_pair(const double q[7], double o, double eps, double& dm, double& dp) {
-  double d[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) d[k] = o * (q[k + 1] - q[k]);
-  dm = weno5_side<double>(d[0], d[1], d[2], d[3], d[4], eps);
-  dp = weno5_side<double>(d[5], d[4], d[3], d[2], d[1], eps);
+// Range of the differences (and of epsilon) in which weno5_side_fast equals
+// weno5_side<double> bit for bit: zero, or a magnitude in [2^-300, 2^100);
+// epsilon in [2^-100, 2^100].
+__device__ __forceinline__ bool weno5_in_range(double d) {
+  const unsigned h = (unsigned)(__double_as_longlong(d) >> 32) & 0x7fffffffu;
+  return h - ((1023u - 300u) << 20) < (400u << 20) || (__double_as_longlong(d) & kAbsBits) == 0;
+}
+
+// weno5_side<double> with the same bits and a fifth of its FP64 operations (27
+// against 140 and more), for differences and epsilon in the range above: no
+// intermediate result overflows, and none but an exact zero is below 2^-1022.
+//   * Every product, the six divisions and the constant thirds and sixths run on the
+//     integer and FP32 pipes (gb2d_exact_math.cuh), correctly rounded; only the sums
+//     are left to the FP64 pipe.
+//   * Doubling and quadrupling are exact: RN(a1 - RN(2 a2)) is one FMA, and
+//     0.25 B B = RN(B B) / 4 joins its sum as an FMA.
+__device__ __forceinline__ double weno5_side_fast(double a1, double a2, double a3, double a4, double a5, double eps) {
+  const double c13 = 13.0 / 12.0, cm16 = (-1.0) / 6.0;
+  const double t3 = mul_rn(a3, 3.0);
+  const double A1 = __fma_rn(-2.0, a2, a1) + a3, B1 = __fma_rn(-4.0, a2, a1) + t3;
+  const double A2 = __fma_rn(-2.0, a3, a2) + a4, B2 = a2 - a4;
+  const double A3 = __fma_rn(-2.0, a4, a3) + a5, B3 = __fma_rn(-4.0, a4, t3) + a5;
+  const double e1 = eps + __fma_rn(0.25, mul_rn(B1, B1), mul_rn(mul_rn(A1, c13), A1));
+  const double e2 = eps + __fma_rn(0.25, mul_rn(B2, B2), mul_rn(mul_rn(A2, c13), A2));
+  const double e3 = eps + __fma_rn(0.25, mul_rn(B3, B3), mul_rn(mul_rn(A3, c13), A3));
+  const double al1 = div_pos(1.0 / 10.0, mul_rn(e1, e1)), al2 = div_pos(6.0 / 10.0, mul_rn(e2, e2)),
+               al3 = div_pos(3.0 / 10.0, mul_rn(e3, e3));
+  const double sum = al1 + al2 + al3;
+  const double p1 = third_rn<0>(a1) - third_rn<1>(mul_rn(a2, 7.0)) + third_rn<1>(mul_rn(a3, 11.0));
+  const double p2 = mul_rn(a2, cm16) + third_rn<1>(mul_rn(a3, 5.0)) + third_rn<0>(a4);
+  const double p3 = third_rn<0>(a3) + third_rn<1>(mul_rn(a4, 5.0)) - third_rn<1>(a5);
+  return mul_rn(div_pos(al1, sum), p1) + mul_rn(div_pos(al2, sum), p2) + mul_rn(div_pos(al3, sum), p3);
+}
+
+// Sign of a WENO5 one-sided derivative from FP32 copies of its differences, or 0
+// where that is not certain.  The derivative is a convex combination of three
+// candidate stencils, so it has their sign when they agree; the margin 2^-13 max|a|
+// on six times a candidate is 16 times the error of the truncated inputs and the
+// FP32 sums (20 max|a| 2^-21.6).
+__device__ __forceinline__ int weno5_sign(float a1, float a2, float a3, float a4, float a5) {
+  const float p1 = fmaf(11.0f, a3, fmaf(-7.0f, a2, 2.0f * a1));
+  const float p2 = fmaf(2.0f, a4, fmaf(5.0f, a3, -a2));
+  const float p3 = fmaf(5.0f, a4, fmaf(2.0f, a3, -a5));
+  const float m = fmaxf(fmaxf(fmaxf(fabsf(a1), fabsf(a2)), fmaxf(fabsf(a3), fabsf(a4))), fabsf(a5));
+  const float thr = m * 1.220703125e-4f;
+  if (!(m > 1e-25f)) return 0;
+  return fminf(fminf(p1, p2), p3) > thr ? 1 : fmaxf(fmaxf(p1, p2), p3) < -thr ? -1 : 0;
 }
 
 // Mixed pair: differences of the FP64 state formed in FP64, everything after in
@@ -153,37 +194,27 @@ __device__ __forceinline__ void weno5_pair_f32(const double q[7], float o, float
 // Godunov selection of WENO5thReinitialization (ADVECTION_METHOD_2D.h:1505-1655).
 // Returns false where the reference leaves phi unchanged (tie sss == 0 or NaN);
 // otherwise h = |grad phi| - 1 over the selected one-sided derivatives.
+// godunov_pick: one direction's choice from its one-sided derivatives m, p: 0 m, 1 p, 2 neither,
+// -1 unchanged.  along_x: only there a tie of the shock rule leaves phi unchanged.
+template <typename R>
+__device__ __forceinline__ int godunov_pick(R s, R m, R p, bool along_x) {
+  const R sm = s * m, sp = s * p;
+  if (gez(sp) && gez(sm)) return 0;
+  if (lez(sp) && lez(sm)) return 1;
+  if (gtz(sp) && ltz(sm)) return 2;
+  if (ltz(sp) && gtz(sm)) {
+    const R sss = s * (fabs(p) - fabs(m)) / (p - m);
+    if (gtz(sss)) return 0;
+    return along_x && !ltz(sss) ? -1 : 1;
+  }
+  return -1;
+}
 template <typename R>
 __device__ __forceinline__ bool godunov_h(R s, R mx, R px, R my, R py, R& h) {
-  R smx = s * mx, spx = s * px, smy = s * my, spy = s * py;
-  int xs, ys;
-  if (gez(spx) && gez(smx))
-    xs = 0;
-  else if (lez(spx) && lez(smx))
-    xs = 1;
-  else if (gtz(spx) && ltz(smx))
-    xs = 2;
-  else if (ltz(spx) && gtz(smx)) {
-    R sss = s * (fabs(px) - fabs(mx)) / (px - mx);
-    if (gtz(sss))
-      xs = 0;
-    else if (ltz(sss))
-      xs = 1;
-    else
-      return false;
-  } else
-    return false;
-  if (gez(spy) && gez(smy))
-    ys = 0;
-  else if (lez(spy) && lez(smy))
-    ys = 1;
-  else if (gtz(spy) && ltz(smy))
-    ys = 2;
-  else if (ltz(spy) && gtz(smy)) {
-    R ss = s * (fabs(py) - fabs(my)) / (py - my);
-    ys = gtz(ss) ? 0 : 1;
-  } else
-    return false;
+  const int xs = godunov_pick(s, mx, px, true);
+  if (xs < 0) return false;
+  const int ys = godunov_pick(s, my, py, false);
+  if (ys < 0) return false;
   R gx = xs == 0 ? mx : px, gy = ys == 0 ? my : py;
   if (xs != 2 && ys != 2)
     h = sqrt(gx * gx + gy * gy) - R(1);

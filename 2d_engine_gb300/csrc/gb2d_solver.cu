@@ -137,16 +137,6 @@ __device__ double sum_partials(const double* part, int n) {
 
 __device__ __forceinline__ unsigned block_linear() { return blockIdx.x + blockIdx.y * gridDim.x; }
 
-// Programmatic dependent launch inside the solver's launch chains: wait until the
-// previous kernel in the stream has completed (its writes visible), then let the
-// next kernel start launching, so launch latency and block scheduling overlap
-// this kernel's tail instead of following it.  Both are no-ops for kernels
-// launched without the programmatic-serialization attribute.
-__device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // The FP64 inputs in the hierarchy's precision: FP32 levels are built in FP32
 // arithmetic from truncated inputs (preconditioner data; FP64 divides and
 // conversions would take the scarce FP64 issue slots).
@@ -1499,22 +1489,6 @@ void build_level0_f64(cudaStream_t s, Hierarchy<double>& H, const gb2d_ctx* c, d
 template <typename T>
 double smooth_bytes(const Level<T>& L, bool pre) {
   return sizeof(T) * (double)L.nI * L.nJ * (pre ? 5.25 : 6.25);
-}
-
-// Launch with programmatic stream serialization (see pdl_enter).
-template <typename... P, typename... A>
-void pdl_launch(cudaStream_t s, dim3 grid, dim3 block, size_t smem, void (*k)(P...), A&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
 template <typename T, int NS, int SH>

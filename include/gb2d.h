@@ -155,10 +155,11 @@ int gb2d_kernel_launches(unsigned long long* count);
  * GB2D_ERR_CUDA if a launch fails, GB2D_ERR_NO_DEVICE without a device. */
 int gb2d_alu_peaks(double* fp64_tflops, double* fp32_tflops);
 
-/* Self-check of the exact FP64 division by 3 and 6 used in the WENO5 kernels
- * (three FP64 operations instead of a division): compares it bit for bit with
- * the IEEE division on 2 n pseudo-random inputs (every exponent, NaN and
- * infinity included) and stores the number of differing results.  No
+/* Self-check of the exact FP64 arithmetic of the WENO5 kernels that avoids the FP64
+ * division and the FP64 pipe: the division by 3 and 6 in three FP64 operations, compared
+ * bit for bit with the IEEE division on 2 n pseudo-random inputs (every exponent, NaN
+ * and infinity included), and the integer-pipe division, product, thirds and square root
+ * on 2 n pairs of normal operands.  Stores the number of differing results.  No
  * counterpart in the reference (diagnostics). */
 int gb2d_check_exact_division(unsigned long long n, unsigned long long seed, unsigned long long* mismatches);
 
