@@ -1177,8 +1177,8 @@ struct Hierarchy {
   size_t tail_smem = 0;
   int ctail = -1;          // levels [ctail, nlev) run in the cluster tail (-1: not used)
   int ct_P = 0;            // CTAs in that cluster
-  size_t ct_smem = 0;
-  CtArgs<T> ct;
+  size_t ct_smem[3] = {};  // per red-black sweeps a side (1, 2, 3), as ct
+  CtArgs<T> ct[3];
   Level<T> L[kMaxLevels];
   int shape[kMaxLevels] = {};  // tile shape of each tiled level's smoothing launches
   T* r = nullptr;  // the preconditioner's input (padded fine layout, = L[0].b); z = L[0].x
@@ -1285,10 +1285,48 @@ cudaError_t alloc_hierarchy(Hierarchy<T>& H, int ni, int nj) {
   return cudaSuccess;
 }
 
-inline int ceil_log2(int v) {
-  int l = 0;
-  while ((1 << l) < v) ++l;
-  return l;
+// Windows and shared memory of the cluster tail for nu sweeps a side.  A side's 2 nu
+// half sweeps cost one halo row each; below the top level x after post-smoothing must
+// also hold on the rows that the finer level's halo is prolonged from.
+template <typename T>
+bool layout_ctail(const CtArgs<T>& base, const int* stripe, int nu, CtArgs<T>* out, size_t* bytes) {
+  CtArgs<T> a = base;
+  const int nl = a.nlev;
+  int off = 0, items = 0, own = 0;
+  for (int l = 0; l < nl; ++l) {
+    CtLevel<T>& L = a.L[l];
+    L.H = l >= a.ndist ? 0 : l == 0 ? 2 * nu : 2 * nu + (a.L[l - 1].H + 1) / 2;
+    const int R = stripe[l] + 2 * L.H < L.nJ ? stripe[l] + 2 * L.H : L.nJ;
+    L.plane = R * L.pairs;
+    L.xplane = (R + 2) * (L.pairs + 2);
+    L.x = off;
+    off += 2 * L.xplane;
+    L.b = -1;
+    if (l > 0 && l < nl - 1) {
+      L.b = off;
+      off += 2 * L.plane;
+    }
+    if (l < nl - 1) {
+      items = L.plane > items ? L.plane : items;
+      own = stripe[l] * L.pairs > own ? stripe[l] * L.pairs : own;
+    }
+  }
+  a.zero_n = off;
+  for (int l = 0; l < a.ndist; ++l) {
+    a.L[l].xi = off;
+    off += 2 * a.L[l].plane;
+  }
+  a.res = off;
+  off += own;
+  a.rg = off;
+  off += a.L[a.ndist - 1].nJ * a.L[a.ndist - 1].pairs;
+  a.bc = off;
+  off += a.L[nl - 1].nI * a.L[nl - 1].nJ;
+  a.kpairs = (items + kCtThreads - 1) / kCtThreads;
+  if ((size_t)off * sizeof(T) > kCtSmemCap || a.kpairs > kCtPairsMax) return false;
+  *out = a;
+  *bytes = (size_t)off * sizeof(T);
+  return true;
 }
 
 // Lay out the cluster tail: the finest top level whose levels fit in one CTA's
@@ -1319,50 +1357,40 @@ bool plan_ctail(Hierarchy<T>& H, int P) {
       for (int c = 0; c < P; ++c) a.J0[l][c] = (short)(2 * a.J0[l + 1][c]);
       a.J0[l][P] = (short)H.L[top + l].nJ;
     }
-    size_t off = 0;
     bool ok = true;
+    size_t cells = 0;  // six padded stripes per level must fit in one CTA's shared memory
+    int stripe[kCtMaxLevels];
     for (int l = 0; l < a.nlev; ++l) {
       const Level<T>& L = H.L[top + l];
       CtLevel<T>& C = a.L[l];
       C.nI = L.nI;
       C.nJ = L.nJ;
       C.ld = L.ld;
-      int rc = L.nJ;
-      if (l < a.ndist) {
-        rc = 0;
-        for (int c = 0; c < P; ++c) {
-          int r = a.J0[l][c + 1] - a.J0[l][c];
-          if (r < 1) ok = false;
-          rc = r > rc ? r : rc;
-        }
-      }
-      C.rows_cap = rc;
-      C.off = (int)off;
-      off += 6 * (size_t)(rc + 2) * L.ld;
-      int hw = (L.nI + 1) / 2;
-      C.half_log2 = ceil_log2(hw < kCtThreads ? hw : kCtThreads);
-      C.full_log2 = ceil_log2(L.nI < kCtThreads ? L.nI : kCtThreads);
+      C.pairs = (L.nI + 1) / 2;
+      C.rpairs = C.pairs > 1 ? (unsigned)(((1ull << 32) + C.pairs - 1) / C.pairs) : 0u;
       C.cx = L.cx;
       C.cy = L.cy;
       C.idg = L.idg;
       C.dg = L.dg;
-      C.b = L.b;
-      C.x = L.x;
+      C.bg = L.b;
+      C.xg = L.x;
+      stripe[l] = L.nJ;
+      if (l < a.ndist) {
+        stripe[l] = 0;
+        for (int c = 0; c < P; ++c) {
+          const int r = a.J0[l][c + 1] - a.J0[l][c];
+          if (r < 1) ok = false;
+          stripe[l] = r > stripe[l] ? r : stripe[l];
+        }
+      }
+      cells += (l == a.ndist - 1 ? 7 : 6) * (size_t)(stripe[l] + 2) * L.ld;
     }
+    const size_t nc = (size_t)H.L[nl - 1].nI * H.L[nl - 1].nJ;
+    if (!ok || (cells + nc * nc + nc) * sizeof(T) > kCtSmemCap) continue;
+    for (int nu = 1; nu <= 3 && ok; ++nu) ok = layout_ctail(a, stripe, nu, &H.ct[nu - 1], &H.ct_smem[nu - 1]);
     if (!ok) continue;
-    a.res_off = (int)off;
-    off += (size_t)(a.L[a.ndist - 1].rows_cap + 2) * a.L[a.ndist - 1].ld;
-    a.ainv_off = (int)off;
-    const int nc = H.L[nl - 1].nI * H.L[nl - 1].nJ;
-    off += (size_t)nc * nc;
-    a.bc_off = (int)off;
-    off += (size_t)nc;
-    const size_t bytes = off * sizeof(T);
-    if (bytes > kCtSmemCap) continue;
     H.ctail = top;
-    H.ct = a;
     H.ct_P = P;
-    H.ct_smem = bytes;
     return true;
   }
   return false;
@@ -1377,10 +1405,12 @@ int ctail_cluster_size() {
   static int cached = -1;
   if (cached >= 0) return cached;
   cached = 0;
-  bool attr_ok = cudaFuncSetAttribute(k_ctail<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                 cudaFuncSetAttribute(k_ctail<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                 cudaFuncSetAttribute(k_ctail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtSmemCap) == cudaSuccess &&
-                 cudaFuncSetAttribute(k_ctail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtSmemCap) == cudaSuccess;
+  const void* kernels[4] = {(const void*)k_ctail<float, kCtPairs>, (const void*)k_ctail<double, kCtPairs>,
+                            (const void*)k_ctail<float, kCtPairsMax>, (const void*)k_ctail<double, kCtPairsMax>};
+  bool attr_ok = true;
+  for (const void* k : kernels)
+    attr_ok = attr_ok && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+              cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtSmemCap) == cudaSuccess;
   if (!attr_ok) {
     cudaGetLastError();
     return cached;
@@ -1400,14 +1430,13 @@ int ctail_cluster_size() {
     cfg.dynamicSmemBytes = kCtSmemCap;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int n32 = 0, n64 = 0;
-    bool ok = cudaOccupancyMaxActiveClusters(&n32, k_ctail<float>, &cfg) == cudaSuccess &&
-              cudaOccupancyMaxActiveClusters(&n64, k_ctail<double>, &cfg) == cudaSuccess;
-    if (!ok) {
-      cudaGetLastError();
-      continue;
+    bool ok = true;
+    for (const void* k : kernels) {
+      int n = 0;
+      ok = ok && cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n >= 1;
     }
-    if (n32 >= 1 && n64 >= 1) {
+    cudaGetLastError();
+    if (ok) {
       cached = P;
       break;
     }
@@ -1417,7 +1446,7 @@ int ctail_cluster_size() {
 
 template <typename T>
 void launch_ctail(cudaStream_t s, const Hierarchy<T>& H, const double* ainv, int nu, const int* done, Scalars* sc) {
-  CtArgs<T> a = H.ct;
+  CtArgs<T> a = H.ct[nu - 1];
   a.sc = H.ctail == 0 ? sc : nullptr;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
@@ -1429,11 +1458,11 @@ void launch_ctail(cudaStream_t s, const Hierarchy<T>& H, const double* ainv, int
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(H.ct_P);
   cfg.blockDim = dim3(kCtThreads);
-  cfg.dynamicSmemBytes = H.ct_smem;
+  cfg.dynamicSmemBytes = H.ct_smem[nu - 1];
   cfg.stream = s;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, k_ctail<T>, a, ainv, nu, done);
+  cudaLaunchKernelEx(&cfg, a.kpairs <= kCtPairs ? k_ctail<T, kCtPairs> : k_ctail<T, kCtPairsMax>, a, ainv, nu, done);
 }
 
 template <typename T>
