@@ -23,10 +23,10 @@ inline unsigned blocks_for(size_t n, int threads = kThreads) { return (unsigned)
 // zeros, subnormals, infinities, NaN and products that may round to zero take
 // the FP64 multiply.
 __device__ __forceinline__ bool prod_ge0(double x, double y) {
-  const long long bx = __double_as_longlong(x), by = __double_as_longlong(y);
-  const int ex = (int)((bx >> 52) & 0x7ff), ey = (int)((by >> 52) & 0x7ff);
-  if (ex != 0 && ey != 0 && ex != 0x7ff && ey != 0x7ff && ex + ey >= 972) return (bx ^ by) >= 0;
-  return x * y >= 0;
+  const unsigned bx = words(x).hi, by = words(y).hi;
+  const int ex = (int)((bx >> 20) & 0x7ff), ey = (int)((by >> 20) & 0x7ff);
+  if (ex != 0 && ey != 0 && ex != 0x7ff && ey != 0x7ff && ex + ey >= 972) return (int)(bx ^ by) >= 0;
+  return plain_mul(x, y) >= 0;
 }
 
 
@@ -93,6 +93,7 @@ struct LSArgs {
   int ni, nj;
   double odx, ody, eps;
   float odx_f, ody_f, eps_f;  // the same in FP32 for the FP32 flux path
+  int fast_f;                 // FP32 epsilon is in mx_sign's range
   int fast;                   // epsilon is in weno5_side_fast's range (and dx in [2^-300, 2^300], for dtau s h)
 };
 
@@ -151,7 +152,7 @@ __device__ __forceinline__ double ex_side(const ExactTile& t, int dir, int c, in
 }
 // g g, or 0 for |g| < 2^-400; |g| < 2^500.
 __device__ __forceinline__ double sqr_flush(double g) {
-  return ((unsigned)(__double_as_longlong(g) >> 52) & 0x7ffu) < 1023u - 400u ? 0.0 : mul_rn(g, g);
+  return ((words(g).hi >> 20) & 0x7ffu) < 1023u - 400u ? 0.0 : mul_rn(g, g);
 }
 // Out of line: the general forms serve differences outside the fast range only.
 __device__ __noinline__ double ex_side_general(const ExactTile& t, int dir, int c, int r, int side, double eps) {
@@ -180,35 +181,6 @@ __device__ __forceinline__ void copy_ring(const DField& src, const DField& dst, 
 // WENO5th (ADVECTION_METHOD_2D.h:508-663) for the node-grid level set: writes
 // dst's interior from src, copies src's ghost ring (the sweep leaves phi's own
 // ghosts to the caller's extrapolation).
-__global__ void k_weno5_advect_mixed(const double* __restrict__ src_a, double* __restrict__ dst_a, const double* __restrict__ ua_a,
-                                     const double* __restrict__ va_a, LSArgs a, DtArg dt_arg) {
-  pdl_enter();
-  int ni = a.ni, nj = a.nj;
-  const double dt = dt_arg.get();
-  int W = ni + 4, H = nj + 4;
-  int ix = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y * blockDim.y + threadIdx.y;
-  if (ix >= W || jy >= H) return;
-  int i = ix - 2, j = jy - 2;
-  DField src = dfield((double*)src_a, 2, ni, nj), dst = dfield(dst_a, 2, ni, nj);
-  if (i < 0 || j < 0 || i >= ni || j >= nj) {
-    GB_AT(dst, i, j) = GB_AT(src, i, j);
-    return;
-  }
-  DField ua = dfield((double*)ua_a, 3, ni + 1, nj), va = dfield((double*)va_a, 3, ni, nj + 1);
-  double q[7];
-  double u = (__ldg(&GB_AT(ua, i + 1, j)) + __ldg(&GB_AT(ua, i, j))) * 0.5;
-  double v = (__ldg(&GB_AT(va, i, j + 1)) + __ldg(&GB_AT(va, i, j))) * 0.5;
-  double fx, fy;
-  float m, p;
-  gather_x(src, i, j, q);
-  weno5_pair_f32(q, a.odx_f, a.eps_f, m, p);
-  fx = gtz(u) ? widen(m) : widen(p);
-  gather_y(src, i, j, q);
-  weno5_pair_f32(q, a.ody_f, a.eps_f, m, p);
-  fy = gtz(v) ? widen(m) : widen(p);
-  GB_AT(dst, i, j) = GB_AT(src, i, j) - dt * (u * fx + v * fy);
-}
-
 // The exact FP64 sweep, bound by the FP64 pipe: each node evaluates the upwind side
 // only (one WENO derivative per direction instead of two), from differences formed
 // once per tile, the x and y directions on two threads.  The grid's last block row
@@ -243,14 +215,31 @@ __global__ void __launch_bounds__(2 * kExX* kExY) k_weno5_advect_exact(const dou
   if (in && dir == 0) GB_AT(dst, i, j) = t.ph[r + 3][c + 3] - dt_arg.get() * (wf + vfy[node]);
 }
 
-// Sign function of Reinitialization (EULERIAN_FLUID_SOLVER_2D.h:2431-2435).
-__global__ void k_reinit_sign(const double* __restrict__ phi_a, double* __restrict__ S, int ni, int nj, double dx) {
+// The plain FP64 forms of the assembly's expressions, for operands outside the fast forms'
+// ranges (out of line, as plain_mul).
+__device__ __noinline__ double plain_mul4(double a, double b, double c, double d) { return a * b * c * d; }
+__device__ __noinline__ double plain_sign(double p, double dx2) { return p / sqrt(p * p + dx2); }
+__device__ __noinline__ double plain_div(double odx, double du, double ody, double dv, double one_over_dt) {
+  return (odx * du + ody * dv) * one_over_dt;
+}
+__device__ __noinline__ double plain_beta(double vc, double vn, double ac, double an) {
+  return vc * vn * (an + ac) / (vc * an + vn * ac);
+}
+
+// Sign function of Reinitialization (EULERIAN_FLUID_SOLVER_2D.h:2431-2435).  dx2 = dx dx.
+__global__ void k_reinit_sign(const double* __restrict__ phi_a, double* __restrict__ S, int ni, int nj, double dx2) {
   pdl_enter();
   DField phi = dfield((double*)phi_a, 2, ni, nj);
+  const bool fast = mid_range<400>(dx2) && !is_zero(dx2);
   GB_FOR_IJ(i, j, ni, nj) {
     const size_t t = (size_t)j * ni + i;
-    double p = GB_AT(phi, i, j);
-    S[t] = p / sqrt(p * p + dx * dx);
+    const double p = GB_AT(phi, i, j);
+    if (fast && mid_range<200>(p)) {  // the same value: one FP64 addition, the rest on the integer pipes
+      const Words w = words(div_pos(absd(p), sqrt_rn(mul_rn(p, p) + dx2)));
+      S[t] = is_zero(p) ? p : from_words(w.lo, w.hi | (words(p).hi & 0x80000000u));
+    } else {
+      S[t] = plain_sign(p, dx2);
+    }
   }
 }
 
@@ -327,14 +316,14 @@ __global__ void __launch_bounds__(2 * kExX * kExY, 5) k_reinit_sweep_exact(const
   const int node = tid & (NN - 1), dir = tid / NN, c = node & (kExX - 1), r = node / kExX, i = i0 + c, j = j0 + r;
   const bool in = i < a.ni && j < a.nj;
   const double s = in ? __ldg(&S[i + (size_t)j * a.ni]) : 0.0;
-  const long long sb = __double_as_longlong(s);
-  const bool sfast = (sb & kAbsBits) >= ((1023LL - 100) << 52) && (sb & kAbsBits) <= kInfBits;  // |s| >= 2^-100
+  const long long smag = mag_bits(s);
+  const bool sfast = smag >= ((1023LL - 100) << 52) && smag <= kInfBits;  // |s| >= 2^-100
   int pick = in ? 3 : 2;
   if (in && fast && sfast) {
     float d[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) d[k] = narrow(ex_diff(t, dir, c, r, k));
-    pick = godunov_case(sb < 0 ? -1 : 1, weno5_sign(d[0], d[1], d[2], d[3], d[4]), weno5_sign(d[5], d[4], d[3], d[2], d[1]));
+    pick = godunov_case((int)words(s).hi < 0 ? -1 : 1, weno5_sign(d[0], d[1], d[2], d[3], d[4]), weno5_sign(d[5], d[4], d[3], d[2], d[1]));
   }
   if (in && fast && pick == 3) list[atomicAdd(&count, 1)] = (unsigned short)tid;
   __syncthreads();
@@ -389,58 +378,152 @@ __global__ void __launch_bounds__(2 * kExX * kExY, 5) k_reinit_sweep_exact(const
   GB_AT(dst, i, j) = old - dtau * s * h;
 }
 
-// The mixed reinit sweep, tiled: the WENO first differences of a node and of its
-// neighbours overlap, so one 32 x 8 tile stages phi with a 3-node halo (positions mapped
-// as the ghost-filled copy maps them) and forms every FP64 difference once (2.8 per node
-// instead of 12; FP64 issue is this kernel's bound), narrowed to FP32 in shared memory.
-// Each node then reads its 6 + 6 differences: the same values as the per-node gathers,
-// so the results equal k_reinit_sweep_mixed's bit for bit.
-constexpr int kRtX = 32, kRtY = 8;
-__global__ void __launch_bounds__(kRtX* kRtY) k_reinit_sweep_tiled(const double* __restrict__ src_a, double* __restrict__ dst_a,
-                                                                    const double* __restrict__ S, LSArgs a, double dtau) {
+// One tile of the mixed sweeps: kMxX x kMxY nodes with every WENO first difference formed
+// once in FP64 (2.8 per node instead of 12; FP64 issue is scarce), narrowed to FP32 and
+// scaled; the same values as the per-node gathers.  dxs[r][c + k] is difference k of node
+// (c, r) along x, dys[r + k][c] along y.  Threads (kMxX, kMxY).
+constexpr int kMxX = 32, kMxY = 8;
+struct MixedTile {
+  double ph[kMxY + 6][kMxX + 6];
+  float dxs[kMxY][kMxX + 5], dys[kMxY + 5][kMxX];
+};
+__device__ __forceinline__ void stage_mixed(MixedTile& t, const DField& src, const LSArgs& a, int i0, int j0) {
+  const int tx = threadIdx.x, ty = threadIdx.y;
+#pragma unroll
+  for (int y = ty; y < kMxY + 6; y += kMxY) {
+    int j = j0 - 3 + y;
+    j = j < 0 ? 1 : (j >= src.nJ ? src.nJ - 2 : j);
+    const double* row = &GB_AT(src, 0, j);
+    auto col = [&](int i) { return i < 0 ? 1 : (i >= src.nI ? src.nI - 2 : i); };
+    t.ph[y][tx] = __ldg(row + col(i0 - 3 + tx));
+    if (tx < 6) t.ph[y][kMxX + tx] = __ldg(row + col(i0 - 3 + kMxX + tx));
+  }
+  __syncthreads();
+  t.dxs[ty][tx] = narrow(t.ph[ty + 3][tx + 1] - t.ph[ty + 3][tx]) * a.odx_f;
+  if (tx < 5) t.dxs[ty][kMxX + tx] = narrow(t.ph[ty + 3][kMxX + tx + 1] - t.ph[ty + 3][kMxX + tx]) * a.odx_f;
+#pragma unroll
+  for (int r = ty; r < kMxY + 5; r += kMxY) t.dys[r][tx] = narrow(t.ph[r + 1][tx + 3] - t.ph[r][tx + 3]) * a.ody_f;
+  __syncthreads();
+}
+// One-sided derivative of node (c, r) along dir (0: x, 1: y): side 0 the minus, side 1 the plus one.
+__device__ __forceinline__ float mx_side(const MixedTile& t, int dir, int c, int r, int side, float eps) {
+  const float* d = dir == 0 ? &t.dxs[r][c] : &t.dys[r][c];
+  const int st = dir == 0 ? 1 : kMxX, first = side ? 5 * st : 0, step = side ? -st : st;
+  return weno5_side<float>(d[first], d[first + step], d[first + 2 * step], d[first + 3 * step], d[first + 4 * step], eps);
+}
+// The common sign of both one-sided derivatives of node (c, r) along dir, or 0 where it is
+// not certain: with all six differences between lo and hi, six times each candidate
+// stencil lies above 13 lo - 7 hi (lo > 0), and a derivative is a convex combination of
+// its candidates.  The bounds keep the FP32 evaluation's rounding (relative 1e-6) and its
+// range out of question: 1e-15 < |d| < 1e8 with epsilon in [1e-15, 1e8] neither overflows
+// a weight nor underflows a derivative times |s| >= 1e-12.
+__device__ __forceinline__ int mx_sign(const MixedTile& t, int dir, int c, int r) {
+  const float* d = dir == 0 ? &t.dxs[r][c] : &t.dys[r][c];
+  const int st = dir == 0 ? 1 : kMxX;
+  const float d0 = d[0], d1 = d[st], d2 = d[2 * st], d3 = d[3 * st], d4 = d[4 * st], d5 = d[5 * st];
+  const float lo = fminf(fminf(fminf(d0, d1), fminf(d2, d3)), fminf(d4, d5));
+  const float hi = fmaxf(fmaxf(fmaxf(d0, d1), fmaxf(d2, d3)), fmaxf(d4, d5));
+  const bool nan = !(d0 + d1 + d2 + d3 + d4 + d5 < 1e9f);  // fminf and fmaxf pass over NaN
+  if (lo > 1e-15f && hi < 1e8f && 13.0f * lo > 7.01f * hi && !nan) return 1;
+  if (hi < -1e-15f && lo > -1e8f && 13.0f * hi < 7.01f * lo && !nan) return -1;
+  return 0;
+}
+
+// WENO5th (ADVECTION_METHOD_2D.h:508-663), the mixed form: the upwind side only, from the
+// tile's differences.  The grid's last block row copies the ghost ring.
+__global__ void __launch_bounds__(kMxX* kMxY) k_weno5_advect_mixed(const double* __restrict__ src_a, double* __restrict__ dst_a,
+                                                                   const double* __restrict__ ua_a, const double* __restrict__ va_a,
+                                                                   LSArgs a, DtArg dt_arg) {
+  constexpr int NT = kMxX * kMxY;
   pdl_enter();
-  __shared__ double ph[kRtY + 6][kRtX + 6];
-  __shared__ float dxs[kRtY][kRtX + 5];
-  __shared__ float dys[kRtY + 5][kRtX];
-  const int ni = a.ni, nj = a.nj, tx = threadIdx.x, ty = threadIdx.y;
-  const int i0 = (int)blockIdx.x * kRtX - 2, j0 = (int)blockIdx.y * kRtY - 2;  // tile origin in node coordinates
-  const DField src = dfield((double*)src_a, 2, ni, nj), dst = dfield(dst_a, 2, ni, nj);
-  for (int k = ty * kRtX + tx; k < (kRtX + 6) * (kRtY + 6); k += kRtX * kRtY) {
-    const int x = k % (kRtX + 6), y = k / (kRtX + 6);
-    int ii = i0 - 3 + x, jj = j0 - 3 + y;
-    ii = ii < 0 ? 1 : (ii >= ni ? ni - 2 : ii);
-    jj = jj < 0 ? 1 : (jj >= nj ? nj - 2 : jj);
-    ph[y][x] = __ldg(&GB_AT(src, ii, jj));
-  }
-  __syncthreads();
-  for (int k = ty * kRtX + tx; k < kRtY * (kRtX + 5); k += kRtX * kRtY) {
-    const int p = k % (kRtX + 5), r = k / (kRtX + 5);
-    dxs[r][p] = narrow(ph[r + 3][p + 1] - ph[r + 3][p]);
-  }
-  for (int k = ty * kRtX + tx; k < (kRtY + 5) * kRtX; k += kRtX * kRtY) {
-    const int c = k % kRtX, p = k / kRtX;
-    dys[p][c] = narrow(ph[p + 1][c + 3] - ph[p][c + 3]);
-  }
-  __syncthreads();
-  const int i = i0 + tx, j = j0 + ty;
-  if (i > ni + 1 || j > nj + 1) return;
-  if (i < 0 || j < 0 || i >= ni || j >= nj) {  // the ghost ring is copied
-    GB_AT(dst, i, j) = GB_AT(src, i, j);
+  __shared__ MixedTile t;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const DField src = dfield((double*)src_a, 2, a.ni, a.nj), dst = dfield(dst_a, 2, a.ni, a.nj);
+  if (blockIdx.y == gridDim.y - 1) {
+    copy_ring(src, dst, blockIdx.x * NT + ty * kMxX + tx, gridDim.x * NT);
     return;
   }
-  const double old = ph[ty + 3][tx + 3];
+  const int i0 = (int)blockIdx.x * kMxX, j0 = (int)blockIdx.y * kMxY, i = i0 + tx, j = j0 + ty;
+  stage_mixed(t, src, a, i0, j0);
+  if (i >= a.ni || j >= a.nj) return;
+  const DField ua = dfield((double*)ua_a, 3, a.ni + 1, a.nj), va = dfield((double*)va_a, 3, a.ni, a.nj + 1);
+  const double u = (__ldg(&GB_AT(ua, i + 1, j)) + __ldg(&GB_AT(ua, i, j))) * 0.5;
+  const double v = (__ldg(&GB_AT(va, i, j + 1)) + __ldg(&GB_AT(va, i, j))) * 0.5;
+  const double fx = widen(mx_side(t, 0, tx, ty, gtz(u) ? 0 : 1, a.eps_f)), fy = widen(mx_side(t, 1, tx, ty, gtz(v) ? 0 : 1, a.eps_f));
+  GB_AT(dst, i, j) = t.ph[ty + 3][tx + 3] - dt_arg.get() * (u * fx + v * fy);
+}
+
+// The mixed reinit sweep, bound by instruction issue.  Where the sign of a direction's
+// derivatives is certain (almost everywhere) the update uses one of the two, and only that
+// one is evaluated; the other nodes put the second evaluation on the block's list, which
+// the block works off densely.  The results equal k_reinit_sweep_mixed's bit for bit.
+// ring: as k_reinit_sweep_exact.
+__global__ void __launch_bounds__(kMxX* kMxY) k_reinit_sweep_tiled(const double* __restrict__ src_a, double* __restrict__ dst_a,
+                                                                   const double* __restrict__ S, LSArgs a, double dtau, int ring) {
+  constexpr int NT = kMxX * kMxY;
+  pdl_enter();
+  __shared__ MixedTile t;
+  __shared__ float plus[2 * NT];
+  __shared__ unsigned short list[2 * NT];
+  __shared__ int count;
+  const int ni = a.ni, nj = a.nj, tx = threadIdx.x, ty = threadIdx.y, tid = ty * kMxX + tx;
+  const DField src = dfield((double*)src_a, 2, ni, nj), dst = dfield(dst_a, 2, ni, nj);
+  if (ring && blockIdx.y == gridDim.y - 1) {
+    copy_ring(src, dst, blockIdx.x * NT + tid, gridDim.x * NT);
+    return;
+  }
+  if (tid == 0) count = 0;
+  const int i0 = (int)blockIdx.x * kMxX, j0 = (int)blockIdx.y * kMxY, i = i0 + tx, j = j0 + ty;
+  stage_mixed(t, src, a, i0, j0);
+  const bool in = i < ni && j < nj;
+  const double sv = in ? __ldg(&S[i + (size_t)j * ni]) : 0.0;
+  const float s = narrow(sv);
+  const int ss = !a.fast_f ? 0 : s >= 1e-12f ? 1 : s <= -1e-12f ? -1 : 0;
+  int xs = 0, ys = 0;  // 0: the minus side, 1: the plus side, 3: both are needed
+  if (in) {
+    const int sx = ss * mx_sign(t, 0, tx, ty), sy = ss * mx_sign(t, 1, tx, ty);
+    xs = sx > 0 ? 0 : sx < 0 ? 1 : 3;
+    ys = sy > 0 ? 0 : sy < 0 ? 1 : 3;
+    if (xs == 3) list[atomicAdd(&count, 1)] = (unsigned short)tid;
+    if (ys == 3) list[atomicAdd(&count, 1)] = (unsigned short)(NT + tid);
+  }
+  __syncthreads();
+  const int n = count;
+  for (int k = tid; k < n; k += NT) {
+    const int item = list[k], nd = item & (NT - 1);
+    plus[item] = mx_side(t, item / NT, nd & (kMxX - 1), nd / kMxX, 1, a.eps_f);
+  }
+  float gx = 0, gy = 0;
+  if (in) {
+    gx = mx_side(t, 0, tx, ty, xs == 1, a.eps_f);
+    gy = mx_side(t, 1, tx, ty, ys == 1, a.eps_f);
+  }
+  if (n > 0) __syncthreads();
+  if (!in) return;
+  const double old = t.ph[ty + 3][tx + 3];
+  if (xs == 3) {
+    const float p = plus[tid];
+    xs = godunov_pick(s, gx, p, true);
+    gx = xs == 0 ? gx : p;
+  }
+  if (ys == 3) {
+    const float p = plus[NT + tid];
+    ys = godunov_pick(s, gy, p, false);
+    gy = ys == 0 ? gy : p;
+  }
   double out = old;
-  float d[6], mx, px, my, py, h;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) d[k] = dxs[ty][tx + k] * a.odx_f;
-  mx = weno5_side<float>(d[0], d[1], d[2], d[3], d[4], a.eps_f);
-  px = weno5_side<float>(d[5], d[4], d[3], d[2], d[1], a.eps_f);
-#pragma unroll
-  for (int k = 0; k < 6; ++k) d[k] = dys[ty + k][tx] * a.ody_f;
-  my = weno5_side<float>(d[0], d[1], d[2], d[3], d[4], a.eps_f);
-  py = weno5_side<float>(d[5], d[4], d[3], d[2], d[1], a.eps_f);
-  const double sv = __ldg(&S[i + (size_t)j * ni]);
-  if (godunov_h<float>(narrow(sv), mx, px, my, py, h)) out = old - dtau * sv * widen(h);
+  if (xs >= 0 && ys >= 0) {
+    float h;
+    if (xs != 2 && ys != 2)
+      h = sqrtf(gx * gx + gy * gy) - 1.0f;
+    else if (xs != 2)
+      h = sqrtf(gx * gx) - 1.0f;
+    else if (ys != 2)
+      h = sqrtf(gy * gy) - 1.0f;
+    else
+      h = -1.0f;
+    out = old - dtau * sv * widen(h);
+  }
   GB_AT(dst, i, j) = out;
 }
 
@@ -449,7 +532,7 @@ __global__ void k_blend(const double* __restrict__ keep_a, double* phi_a, int ni
   pdl_enter();
   DField keep = dfield((double*)keep_a, 2, ni, nj), phi = dfield(phi_a, 2, ni, nj);
   GB_FOR_IJ(i, j, ni, nj) {
-    GB_AT(phi, i, j) = c0 * GB_AT(keep, i, j) + c1 * GB_AT(phi, i, j);
+    GB_AT(phi, i, j) = mul_wide(GB_AT(keep, i, j), c0) + c1 * GB_AT(phi, i, j);
   }
 }
 
@@ -513,44 +596,69 @@ __global__ void k_eno3(double* __restrict__ u_a, double* __restrict__ v_a, const
   GB_FOR_IJ(i, j, ni, nj + 1) face(false, i, j);
 }
 
+// A node's curvature in the plain FP64 forms (LEVELSET_2D.h:898-990); `zero` where the
+// denominator vanishes with the central and with the one-sided differences.
+struct Curv {
+  double k;
+  bool zero;
+};
+__device__ __noinline__ Curv plain_curvature(double c, double l, double r, double b, double tp, double dxy, const Space& s) {
+  double px = (r - l) * s.o2dx;
+  double py = (tp - b) * s.o2dy;
+  const double pxx = (r - 2 * c + l) * s.odx2;
+  const double pyy = (tp - 2 * c + b) * s.ody2;
+  const double pxy = dxy * s.o2dx * s.o2dy;
+  for (int k = 0; k < 2; ++k) {
+    const double mag = sqrt(px * px + py * py);
+    const double deno = mag * mag * mag;
+    if ((__double_as_longlong(deno) & kAbsBits) != 0) {  // deno != 0 (NaN included)
+      const double od = 1.0 / deno;
+      return Curv{-(px * px * pyy - 2.0 * px * py * pxy + py * py * pxx) * od, false};
+    }
+    px = (r - c) * s.odx;
+    py = (tp - c) * s.ody;
+  }
+  return Curv{0.0, true};
+}
+
 // ComputeCurvaturesThread with curvature_by_levelset (LEVELSET_2D.h:898-990);
 // phi's ghosts must already be extrapolated.
 __global__ void k_curvature(const double* __restrict__ phi_a, double* __restrict__ kappa, int ni, int nj, Space s, int* flag) {
   DField phi = dfield((double*)phi_a, 2, ni, nj);
   const double tol = s.dx < s.dy ? s.odx : s.ody;  // 1 / min(dx, dy), taken on the host
+  const bool fast = mid_range<30>(s.odx) && mid_range<30>(s.ody);
   GB_FOR_IJ(i, j, ni, nj) {
     const size_t t = (size_t)j * ni + i;
-    double c = GB_AT(phi, i, j);
-    double l = GB_AT(phi, i - 1, j), r = GB_AT(phi, i + 1, j), b = GB_AT(phi, i, j - 1), tp = GB_AT(phi, i, j + 1);
-    double px = (r - l) * s.o2dx;
-    double py = (tp - b) * s.o2dy;
-    double pxx = (r - 2 * c + l) * s.odx2;
-    double pyy = (tp - 2 * c + b) * s.ody2;
-    double pxy = (GB_AT(phi, i + 1, j + 1) - GB_AT(phi, i + 1, j - 1) - GB_AT(phi, i - 1, j + 1) + GB_AT(phi, i - 1, j - 1)) * s.o2dx * s.o2dy;
-    double mag = sqrt(px * px + py * py);
-    double deno = mag * mag * mag;
-    double curv;
-    if ((__double_as_longlong(deno) & kAbsBits) != 0) {  // deno != 0 (NaN included)
-      double od = 1.0 / deno;
-      curv = -(px * px * pyy - 2.0 * px * py * pxy + py * py * pxx) * od;
+    const double c = GB_AT(phi, i, j), l = GB_AT(phi, i - 1, j), r = GB_AT(phi, i + 1, j), b = GB_AT(phi, i, j - 1), tp = GB_AT(phi, i, j + 1);
+    // r - 2 c as one FMA: doubling is exact (where 2 c overflows, the plain form is taken)
+    const double dx = r - l, dy = tp - b, dxx = __fma_rn(-2.0, c, r) + l, dyy = __fma_rn(-2.0, c, tp) + b;
+    const double dxy = GB_AT(phi, i + 1, j + 1) - GB_AT(phi, i + 1, j - 1) - GB_AT(phi, i - 1, j + 1) + GB_AT(phi, i - 1, j - 1);
+    double curv = 0;
+    if (fast && mid_range<100>(dx) && mid_range<100>(dy) && mid_range<100>(dxx) && mid_range<100>(dyy) && mid_range<100>(dxy) &&
+        !(is_zero(dx) && is_zero(dy))) {
+      // The same value: products, root and quotient on the integer pipes but for the six
+      // scalings, which balance the two pipes.
+      const double px = dx * s.o2dx, py = dy * s.o2dy, pxx = dxx * s.odx2, pyy = dyy * s.ody2, pxy = dxy * s.o2dx * s.o2dy;
+      const double x2 = mul_rn(px, px), y2 = mul_rn(py, py);
+      const double mag = sqrt_rn(x2 + y2);
+      const double od = div_pos(1.0, mul_rn(mul_rn(mag, mag), mag));
+      // 2 px py pxy is twice the rounded px py pxy
+      const double n = __fma_rn(-2.0, mul_rn(mul_rn(px, py), pxy), mul_rn(x2, pyy)) + mul_rn(y2, pxx);
+      curv = negd(mul_rn(n, od));
     } else {
-      px = (r - c) * s.odx;
-      py = (tp - c) * s.ody;
-      mag = sqrt(px * px + py * py);
-      deno = mag * mag * mag;
-      if ((__double_as_longlong(deno) & kAbsBits) == 0) {  // deno == 0
+      const Curv g = plain_curvature(c, l, r, b, tp, dxy, s);
+      if (g.zero) {
         atomicOr(flag, 2);
         continue;
       }
-      double od = 1.0 / deno;
-      curv = -(px * px * pyy - 2.0 * px * py * pxy + py * py * pxx) * od;
+      curv = g.k;
     }
     // Clamp to [-tol, tol] with IEEE comparisons (tol > 0 finite; a NaN stores nothing)
-    const long long cb = __double_as_longlong(curv), cm = cb & kAbsBits, tb = __double_as_longlong(tol);
-    if (cm <= tb)
+    const long long cm = mag_bits(curv);
+    if (cm <= mag_bits(tol))
       kappa[t] = curv;
     else if (cm <= kInfBits)
-      kappa[t] = cb > 0 ? tol : -tol;
+      kappa[t] = (int)words(curv).hi >= 0 ? tol : negd(tol);
   }
 }
 
@@ -561,6 +669,7 @@ struct AsmArgs {
   double inv_water, inv_air;  // 1/water, 1/air: IEEE quotients taken once on the host
   const double* dtp;          // non-null: the time step is read here (one_over_dt = 1 / *dtp, IEEE)
   double oeh, oev;            // 1 / (1.5 dx), 1 / (1.5 dy): smeared-Heaviside scales
+  int fast;                   // densities and cell sizes are in the fast forms' range (mid_range<100>)
 };
 
 // 1/rho of a node.  The density takes two values, so the quotient is a select of
@@ -579,8 +688,15 @@ __device__ __forceinline__ double vnode(const DField& phi, int i, int j, const A
   return inv_density(GB_AT(phi, i, j), a);
 }
 
-__device__ __forceinline__ double face_beta(double vc, double vn, double pc, double pn) {
-  return vc * vn * (fabs(pn) + fabs(pc)) / (vc * fabs(pn) + vn * fabs(pc));
+// vc vn (|pn| + |pc|) / (vc |pn| + vn |pc|); with 1/rho and |phi| in the fast range the
+// quotient and half of the products on the integer pipes (the same value).
+__device__ __forceinline__ double face_beta(double vc, double vn, double pc, double pn, const AsmArgs& a) {
+  const double ac = absd(pc), an = absd(pn);
+  if (a.fast && mid_range<300>(pc) && mid_range<300>(pn)) {
+    const double sum = an + ac;
+    if (!is_zero(sum)) return div_pos(mul_rn(mul_rn(vc, vn), sum), vc * an + vn * ac);
+  }
+  return plain_beta(vc, vn, ac, an);
 }
 
 // Face weights of BuildLinearSystemNodeJumpConditionVaribleCoefficient
@@ -589,10 +705,10 @@ __global__ void k_faces(const double* __restrict__ phi_a, double* __restrict__ b
   int ni = a.ni, nj = a.nj;
   DField phi = dfield((double*)phi_a, 2, ni, nj);
   GB_FOR_IJ(i, j, ni + 1, nj) {
-    bx[(size_t)j * (ni + 1) + i] = face_beta(vnode(phi, i, j, a), vnode(phi, i - 1, j, a), GB_AT(phi, i, j), GB_AT(phi, i - 1, j));
+    bx[(size_t)j * (ni + 1) + i] = face_beta(vnode(phi, i, j, a), vnode(phi, i - 1, j, a), GB_AT(phi, i, j), GB_AT(phi, i - 1, j), a);
   }
   GB_FOR_IJ(i, j, ni, nj + 1) {
-    by[(size_t)j * ni + i] = face_beta(vnode(phi, i, j, a), vnode(phi, i, j - 1, a), GB_AT(phi, i, j), GB_AT(phi, i, j - 1));
+    by[(size_t)j * ni + i] = face_beta(vnode(phi, i, j, a), vnode(phi, i, j - 1, a), GB_AT(phi, i, j), GB_AT(phi, i, j - 1), a);
   }
 }
 
@@ -629,44 +745,75 @@ __global__ void k_diag(const double* __restrict__ bx, const double* __restrict__
     const size_t t = (size_t)j * ni + i;
     double bl = bx[i + (size_t)j * (ni + 1)], br = bx[i + 1 + (size_t)j * (ni + 1)];
     double bb = by[i + (size_t)j * ni], bt = by[i + (size_t)(j + 1) * ni];
-    double coef = 0;
-    if (i > 0) coef += bl;
-    if (i < ni - 1) coef += br;
-    if (j > 0) coef += bb;
-    if (j < nj - 1) coef += bt;
-    if (i == 0 && j == 0) {  // Neumann arms of the first cell (POISSON_SOLVER.cpp:789-806)
-      if (i - 1 < 0) coef += bl;
-      if (i + 1 > ni - 1) coef += br;
-      if (j - 1 < 0) coef += bb;
-      if (j + 1 > nj - 1) coef += bt;
+    double coef;
+    if (i > 0 && i < ni - 1 && j > 0 && j < nj - 1) {
+      coef = bl + br + bb + bt;
+    } else {
+      coef = 0;
+      if (i > 0) coef += bl;
+      if (i < ni - 1) coef += br;
+      if (j > 0) coef += bb;
+      if (j < nj - 1) coef += bt;
+      if (i == 0 && j == 0) {  // Neumann arms of the first cell (POISSON_SOLVER.cpp:789-806)
+        if (i - 1 < 0) coef += bl;
+        if (i + 1 > ni - 1) coef += br;
+        if (j - 1 < 0) coef += bb;
+        if (j + 1 > nj - 1) coef += bt;
+      }
     }
-    if ((__double_as_longlong(coef) & kAbsBits) == 0) coef = 1;  // coef == 0
+    if (is_zero(coef)) coef = 1;
     diag[t] = a.inv_dxdx * coef;
   }
 }
 
-// Right-hand side -div - F_X - F_Y (POISSON_SOLVER.cpp:878-948).
+// An arm of k_rhs crosses the interface (arm_flux is not zero for it).
+__device__ __forceinline__ bool arm_crosses(double pc, double pn) {
+  const bool cneg = lez(pc), nneg = lez(pn);
+  return cneg ? !nneg && gtz(pn) : nneg && gtz(pc);
+}
+
+// k_rhs's value at a node with an arm that crosses the interface (out of line, as plain_mul).
+__device__ __noinline__ double rhs_interface(double div, double pc, double pl, double pr, double pb, double pt, const double* kappa,
+                                             const double* bx, const double* by, int i, int j, const AsmArgs& a) {
+  const int ni = a.ni;
+  const double bl = bx[i + (size_t)j * (ni + 1)], br = bx[i + 1 + (size_t)j * (ni + 1)];
+  const double bb = by[i + (size_t)j * ni], bt = by[i + (size_t)(j + 1) * ni];
+  const double jcc = jc_at(kappa, i, j, a);
+  const double FL = arm_flux(pc, pl, jcc, kappa, i - 1, j, bl, a.s.odx2, a);
+  const double FR = arm_flux(pc, pr, jcc, kappa, i + 1, j, br, a.s.odx2, a);
+  const double FB = arm_flux(pc, pb, jcc, kappa, i, j - 1, bb, a.s.ody2, a);
+  const double FT = arm_flux(pc, pt, jcc, kappa, i, j + 1, bt, a.s.ody2, a);
+  const double FX = FL + FR, FY = FB + FT;
+  return -div - FX - FY;
+}
+
+// Right-hand side -div - F_X - F_Y (POISSON_SOLVER.cpp:878-948).  Away from the interface
+// the four fluxes are zero and drop out: three FP64 additions and two products a node, the
+// third product on the integer pipes.
 __global__ void k_rhs(const double* __restrict__ phi_a, const double* __restrict__ kappa, const double* __restrict__ u_a,
                       const double* __restrict__ v_a, const double* __restrict__ bx, const double* __restrict__ by, double* __restrict__ rhs,
                       AsmArgs a) {
   int ni = a.ni, nj = a.nj;
-  const double one_over_dt = a.dtp ? 1.0 / *a.dtp : a.one_over_dt;
+  double one_over_dt = a.one_over_dt;
+  if (a.dtp) one_over_dt = mid_range<100>(*a.dtp) && gtz(*a.dtp) ? div_pos(1.0, *a.dtp) : 1.0 / *a.dtp;
+  const bool fast = a.fast && mid_range<100>(one_over_dt);
   DField phi = dfield((double*)phi_a, 2, ni, nj);
   DField u = dfield((double*)u_a, 2, ni + 1, nj), v = dfield((double*)v_a, 2, ni, nj + 1);
   GB_FOR_IJ(i, j, ni, nj) {
     const size_t t = (size_t)j * ni + i;
-    double bl = bx[i + (size_t)j * (ni + 1)], br = bx[i + 1 + (size_t)j * (ni + 1)];
-    double bb = by[i + (size_t)j * ni], bt = by[i + (size_t)(j + 1) * ni];
-    double pc = GB_AT(phi, i, j);
-    double jcc = jc_at(kappa, i, j, a);
-    double FL = arm_flux(pc, GB_AT(phi, i - 1, j), jcc, kappa, i - 1, j, bl, a.s.odx2, a);
-    double FR = arm_flux(pc, GB_AT(phi, i + 1, j), jcc, kappa, i + 1, j, br, a.s.odx2, a);
-    double FB = arm_flux(pc, GB_AT(phi, i, j - 1), jcc, kappa, i, j - 1, bb, a.s.ody2, a);
-    double FT = arm_flux(pc, GB_AT(phi, i, j + 1), jcc, kappa, i, j + 1, bt, a.s.ody2, a);
-    double div = a.s.odx * (GB_AT(u, i + 1, j) - GB_AT(u, i, j)) + a.s.ody * (GB_AT(v, i, j + 1) - GB_AT(v, i, j));
-    div *= one_over_dt;
-    double FX = FL + FR, FY = FB + FT;
-    rhs[t] = -div - FX - FY;
+    const double pc = GB_AT(phi, i, j);
+    const double pl = GB_AT(phi, i - 1, j), pr = GB_AT(phi, i + 1, j), pb = GB_AT(phi, i, j - 1), pt = GB_AT(phi, i, j + 1);
+    const double du = GB_AT(u, i + 1, j) - GB_AT(u, i, j), dv = GB_AT(v, i, j + 1) - GB_AT(v, i, j);
+    double div;
+    if (fast && mid_range<300>(dv))
+      div = (a.s.odx * du + mul_rn(a.s.ody, dv)) * one_over_dt;
+    else
+      div = plain_div(a.s.odx, du, a.s.ody, dv, one_over_dt);
+    if (!(arm_crosses(pc, pl) || arm_crosses(pc, pr) || arm_crosses(pc, pb) || arm_crosses(pc, pt))) {
+      rhs[t] = negd(div);
+      continue;
+    }
+    rhs[t] = rhs_interface(div, pc, pl, pr, pb, pt, kappa, bx, by, i, j, a);
   }
 }
 
@@ -685,6 +832,17 @@ __global__ void k_apply_exact(const double* __restrict__ bx, const double* __res
   }
 }
 
+// An interface face's updated velocity (out of line, as plain_mul).
+__device__ __noinline__ double velocity_interface(double w, double dp, double dt, double od, double l0, double ln, double jcc, double jcn,
+                                                  bool xc, const AsmArgs& a) {
+  const double gam = (jcn * fabs(l0) + jcc * fabs(ln)) / (fabs(l0) + fabs(ln));
+  const double dh = a.air + (a.water - a.air) * heaviside(0.5 * (l0 + ln), 1.5 * (xc ? a.s.dx : a.s.dy), xc ? a.oeh : a.oev);
+  const double odh = 1 / dh;
+  if (ltz(l0)) return w - dt * (dp + gam) * odh * od;
+  if (gtz(l0)) return w - dt * (dp - gam) * odh * od;
+  return w;
+}
+
 // UpdateVelocityByPressureGradientVariableDensity (PROJECTION_2D.h:1297-1416):
 // same-sign faces use the node density on the + side, interface faces the
 // smeared-Heaviside density of the face-averaged phi (eps = 1.5 dx) and the
@@ -696,33 +854,27 @@ __global__ void k_velocity_update(const double* __restrict__ phi_a, const double
   DField phi = dfield((double*)phi_a, 2, ni, nj), p = dfield((double*)p_a, 1, ni, nj);
   DField u = dfield(u_a, 2, ni + 1, nj), v = dfield(v_a, 2, ni, nj + 1);
   const double odx = a.s.odx, ody = a.s.ody;  // 1 / dx, 1 / dy, taken on the host
-  double eh = 1.5 * a.s.dx, ev = 1.5 * a.s.dy;
+  const bool fast = a.fast && mid_range<100>(dt);
   unsigned long long mx = 0, my = 0;  // bits of max |u|, |v| (non-negative doubles order as integers)
-  auto face = [&](bool xc, int i, int j) {
-    int in = xc ? i - 1 : i, jn = xc ? j : j - 1;
-    double l0 = GB_AT(phi, i, j), ln = GB_AT(phi, in, jn);
-    double oor = lez(l0) ? a.inv_air : a.inv_water;  // 1 / rho_ij
-    double dp = GB_AT(p, i, j) - GB_AT(p, in, jn);
-    double od = xc ? odx : ody;
-    double* w = xc ? &GB_AT(u, i, j) : &GB_AT(v, i, j);
-    if (prod_ge0(l0, ln)) {
-      *w -= dt * dp * oor * od;
-    } else {
-      double jcc = jc_at(kappa, i, j, a), jcn = jc_at(kappa, in, jn, a);
-      double gam = (jcn * fabs(l0) + jcc * fabs(ln)) / (fabs(l0) + fabs(ln));
-      double dh = a.air + (a.water - a.air) * heaviside(0.5 * (l0 + ln), xc ? eh : ev, xc ? a.oeh : a.oev);
-      double odh = 1 / dh;
-      if (ltz(l0))
-        *w -= dt * (dp + gam) * odh * od;
-      else if (gtz(l0))
-        *w -= dt * (dp - gam) * odh * od;
-    }
-    unsigned long long& m = xc ? mx : my;
-    m = abs_max_bits(*w, m);
-  };
   GB_FOR_IJ(i, j, ni, nj) {
-    face(true, i, j);
-    face(false, i, j);
+    const double l0 = GB_AT(phi, i, j), lw = GB_AT(phi, i - 1, j), ls = GB_AT(phi, i, j - 1);
+    const double p0 = GB_AT(p, i, j), dpx = p0 - GB_AT(p, i - 1, j), dpy = p0 - GB_AT(p, i, j - 1);
+    double wu = GB_AT(u, i, j), wv = GB_AT(v, i, j);
+    const double oor = lez(l0) ? a.inv_air : a.inv_water;  // 1 / rho_ij
+    // The x-face's products on the FP64 pipe, the y-face's on the integer pipes (where none
+    // can leave the normal range).
+    if (prod_ge0(l0, lw))
+      wu -= dt * dpx * oor * odx;
+    else
+      wu = velocity_interface(wu, dpx, dt, odx, l0, lw, jc_at(kappa, i, j, a), jc_at(kappa, i - 1, j, a), true, a);
+    if (prod_ge0(l0, ls))
+      wv -= fast && mid_range<300>(dpy) ? mul_rn(mul_rn(mul_rn(dt, dpy), oor), ody) : plain_mul4(dt, dpy, oor, ody);
+    else
+      wv = velocity_interface(wv, dpy, dt, ody, l0, ls, jc_at(kappa, i, j, a), jc_at(kappa, i, j - 1, a), false, a);
+    GB_AT(u, i, j) = wu;
+    GB_AT(v, i, j) = wv;
+    mx = abs_max_bits(wu, mx);
+    my = abs_max_bits(wv, my);
   }
   block_max_bits(mx, &sc->maxu_bits);
   block_max_bits(my, &sc->maxv_bits);
@@ -801,6 +953,7 @@ inline dim3 grid2d(int W, int H, dim3 blk) { return dim3((W + blk.x - 1) / blk.x
 LSArgs ls_args(const gb2d_ctx* c) {
   return LSArgs{c->grid.ni, c->grid.nj, c->base.odx, c->base.ody, c->prm.weno_epsilon,
                 (float)c->base.odx, (float)c->base.ody, (float)c->prm.weno_epsilon,
+                c->prm.weno_epsilon >= 1e-15 && c->prm.weno_epsilon <= 1e8,
                 c->prm.weno_epsilon >= 0x1p-100 && c->prm.weno_epsilon <= 0x1p100 &&
                     c->base.dx >= 0x1p-300 && c->base.dx <= 0x1p300};
 }
@@ -821,6 +974,8 @@ AsmArgs asm_args(const gb2d_ctx* c, double dt) {
   a.inv_air = 1.0 / a.air;
   a.oeh = 1.0 / (1.5 * c->base.dx);
   a.oev = 1.0 / (1.5 * c->base.dy);
+  auto mid = [](double x) { return x >= 0x1p-100 && x < 0x1p100; };
+  a.fast = mid(a.inv_water) && mid(a.inv_air) && mid(a.s.odx) && mid(a.s.ody);
   return a;
 }
 
@@ -893,8 +1048,8 @@ void launch_extrapolate_ghosts(cudaStream_t s, double* f, int g, int nI, int nJ)
 void launch_weno5_advect(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, double dt, int mixed) {
   const int ni = c->grid.ni, nj = c->grid.nj;
   if (mixed) {
-    dim3 blk(32, 8);
-    pdl_launch(s, grid2d(ni + 4, nj + 4, blk), blk, 0, k_weno5_advect_mixed, src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
+    const dim3 grd((ni + kMxX - 1) / kMxX, (nj + kMxY - 1) / kMxY + 1);
+    pdl_launch(s, grd, dim3(kMxX, kMxY), 0, k_weno5_advect_mixed, src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
   } else {
     const dim3 grd((ni + kExX - 1) / kExX, (nj + kExY - 1) / kExY + 1);
     pdl_launch(s, grd, 2 * kExX * kExY, 0, k_weno5_advect_exact, src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
@@ -903,7 +1058,7 @@ void launch_weno5_advect(cudaStream_t s, const gb2d_ctx* c, const double* src, d
 }
 
 void launch_reinit_sign(cudaStream_t s, const gb2d_ctx* c, const double* phi, double* S) {
-  pdl_launch(s, grid_ij(c->grid.ni, c->grid.nj), kThreads, 0, k_reinit_sign, phi, S, c->grid.ni, c->grid.nj, c->base.dx);
+  pdl_launch(s, grid_ij(c->grid.ni, c->grid.nj), kThreads, 0, k_reinit_sign, phi, S, c->grid.ni, c->grid.nj, c->base.dx * c->base.dx);
   GB_LAUNCHED(1);
 }
 
@@ -916,12 +1071,12 @@ void launch_reinit_sweep(cudaStream_t s, const gb2d_ctx* c, const double* src, d
     const char* e = getenv("GB2D_REINIT_UNTILED");
     return e && e[0] == '1';
   }();
-  dim3 blk(32, 8);
-  dim3 grd = grid2d(ni + 4, nj + 4, blk);
   if (mixed && !untiled) {
-    pdl_launch(s, grd, blk, 0, k_reinit_sweep_tiled, src, dst, S, ls_args(c), dtau);
+    const dim3 g((ni + kMxX - 1) / kMxX, (nj + kMxY - 1) / kMxY + (ring ? 1 : 0));
+    pdl_launch(s, g, dim3(kMxX, kMxY), 0, k_reinit_sweep_tiled, src, dst, S, ls_args(c), dtau, ring);
   } else if (mixed) {
-    pdl_launch(s, grd, blk, 0, k_reinit_sweep_mixed, src, dst, S, ls_args(c), dtau);
+    const dim3 blk(32, 8);
+    pdl_launch(s, grid2d(ni + 4, nj + 4, blk), blk, 0, k_reinit_sweep_mixed, src, dst, S, ls_args(c), dtau);
   } else {
     const dim3 g((ni + kExX - 1) / kExX, (nj + kExY - 1) / kExY + (ring ? 1 : 0));
     pdl_launch(s, g, 2 * kExX * kExY, 0, k_reinit_sweep_exact, src, dst, S, ls_args(c), dtau, ring);

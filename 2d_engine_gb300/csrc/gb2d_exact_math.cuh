@@ -24,8 +24,16 @@ namespace gb2d {
 
 // Bit casts and FP32 steps, on the device and (for the CPU checks) on the host.
 #ifdef __CUDA_ARCH__
-GB_HD uint64_t dbits(double x) { return (uint64_t)__double_as_longlong(x); }
-GB_HD double bitsd(uint64_t b) { return __longlong_as_double((long long)b); }
+GB_HD uint64_t dbits(double x) {  // opaque: the compiler must not recognise FP64 operations in what follows
+  uint64_t b;
+  asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+  return b;
+}
+GB_HD double bitsd(uint64_t b) {
+  double x;
+  asm("mov.b64 %0, %1;" : "=d"(x) : "l"(b));
+  return x;
+}
 GB_HD uint32_t fbits(float x) { return __float_as_uint(x); }
 GB_HD float bitsf(uint32_t b) { return __uint_as_float(b); }
 GB_HD float fma32(float a, float b, float c) { return __fmaf_rn(a, b, c); }

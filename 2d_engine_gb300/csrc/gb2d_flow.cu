@@ -221,8 +221,8 @@ __global__ void k_face_blend(const double* __restrict__ ku_a, double* __restrict
   const DField ku = dfield((double*)ku_a, 2, ni + 1, nj), u = dfield(u_a, 2, ni + 1, nj);
   const DField kv = dfield((double*)kv_a, 2, ni, nj + 1), v = dfield(v_a, 2, ni, nj + 1);
   GB_FOR_IJ(i, j, ni + 1, nj + 1) {
-    if (j < nj) GB_AT(u, i, j) = c0 * GB_AT(ku, i, j) + c1 * GB_AT(u, i, j);
-    if (i < ni) GB_AT(v, i, j) = c0 * GB_AT(kv, i, j) + c1 * GB_AT(v, i, j);
+    if (j < nj) GB_AT(u, i, j) = mul_wide(GB_AT(ku, i, j), c0) + c1 * GB_AT(u, i, j);
+    if (i < ni) GB_AT(v, i, j) = mul_wide(GB_AT(kv, i, j), c0) + c1 * GB_AT(v, i, j);
   }
 }
 

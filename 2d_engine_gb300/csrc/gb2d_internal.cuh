@@ -31,18 +31,20 @@ __host__ __device__ inline DField dfield(double* a, int g, int nI, int nJ) { ret
 #define GB_AT(f, i, j) ((f).a[((i) + (f).g) + (size_t)((j) + (f).g) * (f).ld])
 
 // FP32 <-> FP64 moves as bit manipulations on the integer pipes (FP64 issue
-// slots, which conversions use, are scarce on this part).
+// slots, which conversions use, are scarce on this part), a handful of 32-bit
+// operations for normal values.
 // Exact FP32 -> FP64 (every FP32 value is an FP64 value); FP32 subnormals, below
 // 1.2e-38, become signed zero.
 __device__ __forceinline__ double widen(float f) {
-  const unsigned u = __float_as_uint(f);
-  const unsigned e = (u >> 23) & 0xffu;
-  unsigned long long bits = (unsigned long long)(u >> 31) << 63;
-  if (e != 0u) {
-    const unsigned long long E = e == 0xffu ? 0x7ffull : (unsigned long long)(e + 896u);
-    bits |= (E << 52) | ((unsigned long long)(u & 0x7fffffu) << 29);
+  const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu, s = u & 0x80000000u;
+  unsigned hi = ((m >> 3) + 0x38000000u) | s, lo = u << 29;  // the exponent gains 896
+  if (m - 0x00800000u >= 0x7f000000u) {                       // zero, subnormal; infinity, NaN
+    hi = m < 0x00800000u ? s : s | 0x7ff00000u | ((m & 0x7fffffu) >> 3);
+    lo = m < 0x00800000u ? 0u : lo;
   }
-  return __longlong_as_double((long long)bits);
+  double d;
+  asm("mov.b64 %0, {%1, %2};" : "=d"(d) : "r"(lo), "r"(hi));
+  return d;
 }
 __device__ __forceinline__ double widen(double d) { return d; }
 
@@ -50,19 +52,18 @@ __device__ __forceinline__ double widen(double d) { return d; }
 // only); magnitudes below the FP32 normal range become signed zero, above it
 // infinity.
 __device__ __forceinline__ float narrow(double d) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-  const unsigned s = (unsigned)(b >> 63) << 31;
-  const int E = (int)((b >> 52) & 0x7ffull);
-  const int e = E - 896;
-  unsigned bits;
-  if (E == 0x7ff)
-    bits = s | 0x7f800000u | (unsigned)((b >> 29) & 0x7fffffull) | ((b & 0xfffffffffffffull) ? 0x400000u : 0u);
-  else if (e <= 0)
+  unsigned lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(d));
+  const unsigned h = hi & 0x7fffffffu, s = hi & 0x80000000u;
+  const unsigned t = __funnelshift_l(lo, hi, 3);  // exponent (low bits) and the leading 23 bits of the significand
+  unsigned bits = ((t - 0xc0000000u) & 0x7fffffffu) | s;  // the exponent loses 896
+  if (h - (897u << 20) >= (254u << 20)) {
     bits = s;
-  else if (e >= 255)
-    bits = s | 0x7f800000u;
-  else
-    bits = s | ((unsigned)e << 23) | (unsigned)((b >> 29) & 0x7fffffull);
+    if (h >= (1151u << 20)) {
+      bits |= 0x7f800000u;
+      if (h > 0x7ff00000u || (h == 0x7ff00000u && lo != 0u)) bits |= (t & 0x7fffffu) | 0x400000u;
+    }
+  }
   return __uint_as_float(bits);
 }
 
@@ -235,7 +236,7 @@ unsigned long long check_div_by(unsigned long long n, unsigned long long seed, i
 void launch_extrapolate_ghosts(cudaStream_t s, double* f, int g, int nI, int nJ);
 void launch_weno5_advect(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, double dt, int mixed);
 void launch_reinit_sign(cudaStream_t s, const gb2d_ctx* c, const double* phi, double* S);
-// ring: copy src's ghost ring to dst (the mixed sweeps always do).
+// ring: copy src's ghost ring to dst.
 void launch_reinit_sweep(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, const double* S, double dtau, int mixed,
                          int ring);
 void launch_blend(cudaStream_t s, const gb2d_ctx* c, const double* keep, double* phi, double c0, double c1);

@@ -11,39 +11,78 @@
 
 namespace gb2d {
 
+// The two words of a double, and back.  The moves are opaque to the compiler, which
+// otherwise recognises integer tests and masks of a double's bits and turns them into FP64
+// comparisons and additions (a fabs or a negation is an FP64 addition on this part: the
+// right-hand side kernel issued 15 FP64 instructions a node, 3 of them its sums).
+struct Words {
+  unsigned lo, hi;
+};
+__device__ __forceinline__ Words words(double x) {
+  Words w;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(w.lo), "=r"(w.hi) : "d"(x));
+  return w;
+}
+__device__ __forceinline__ double from_words(unsigned lo, unsigned hi) {
+  double x;
+  asm("mov.b64 %0, {%1, %2};" : "=d"(x) : "r"(lo), "r"(hi));
+  return x;
+}
+__device__ __forceinline__ double absd(double x) {
+  const Words w = words(x);
+  return from_words(w.lo, w.hi & 0x7fffffffu);
+}
+__device__ __forceinline__ double negd(double x) {
+  const Words w = words(x);
+  return from_words(w.lo, w.hi ^ 0x80000000u);
+}
+__device__ __forceinline__ bool is_zero(double x) {
+  const Words w = words(x);
+  return ((w.hi << 1) | w.lo) == 0u;
+}
+// |x| as an integer (ordered as the magnitudes are; above kInfBits: NaN).
+constexpr long long kAbsBits = 0x7fffffffffffffffLL, kInfBits = 0x7ff0000000000000LL;
+__device__ __forceinline__ long long mag_bits(double x) {
+  const Words w = words(x);
+  return (long long)((unsigned long long)(w.hi & 0x7fffffffu) << 32 | w.lo);
+}
+
 // IEEE comparisons with zero.  FP64: on the integer pipes (an FP64 compare takes
 // one of the part's few FP64 issue slots), exact for every input, NaN and
 // infinities included.  FP32: the native compare.
-constexpr long long kAbsBits = 0x7fffffffffffffffLL, kInfBits = 0x7ff0000000000000LL;
+__device__ __forceinline__ bool nan_words(Words w) {
+  const unsigned h = w.hi & 0x7fffffffu;
+  return h > 0x7ff00000u || (h == 0x7ff00000u && w.lo != 0u);
+}
 __device__ __forceinline__ bool gtz(double x) {  // x > 0
-  const long long b = __double_as_longlong(x);
-  return b > 0 && b <= kInfBits;
+  const Words w = words(x);
+  return (int)w.hi >= 0 && (w.hi | w.lo) != 0u && !nan_words(w);
 }
 __device__ __forceinline__ bool gez(double x) {  // x >= 0
-  const long long b = __double_as_longlong(x);
-  return (b >= 0 && b <= kInfBits) || b == (long long)0x8000000000000000ull;
+  const Words w = words(x);
+  return ((int)w.hi >= 0 || ((w.hi << 1) | w.lo) == 0u) && !nan_words(w);
 }
 __device__ __forceinline__ bool lez(double x) {  // x <= 0
-  const long long b = __double_as_longlong(x);
-  return b == 0 || (b < 0 && (b & kAbsBits) <= kInfBits);
+  const Words w = words(x);
+  return ((int)w.hi < 0 || (w.hi | w.lo) == 0u) && !nan_words(w);
 }
 __device__ __forceinline__ bool ltz(double x) {  // x < 0
-  const long long b = __double_as_longlong(x), m = b & kAbsBits;
-  return b < 0 && m != 0 && m <= kInfBits;
+  const Words w = words(x);
+  return (int)w.hi < 0 && ((w.hi << 1) | w.lo) != 0u && !nan_words(w);
 }
 // |a| <= |b| (false when either is NaN), on the integer pipes.
 __device__ __forceinline__ bool abs_le(double a, double b) {
-  const long long ma = __double_as_longlong(a) & kAbsBits, mb = __double_as_longlong(b) & kAbsBits;
+  const long long ma = mag_bits(a), mb = mag_bits(b);
   return ma <= mb && mb <= kInfBits;
 }
 // x < -e and x > e for a finite e > 0, on the integer pipes (false for NaN).
 __device__ __forceinline__ bool lt_neg(double x, double e) {
-  const long long b = __double_as_longlong(x), m = b & kAbsBits;
-  return b < 0 && m > __double_as_longlong(e) && m <= kInfBits;
+  const long long m = mag_bits(x);
+  return (int)words(x).hi < 0 && m > mag_bits(e) && m <= kInfBits;
 }
 __device__ __forceinline__ bool gt_pos(double x, double e) {
-  const long long b = __double_as_longlong(x);
-  return b > __double_as_longlong(e) && b <= kInfBits;
+  const long long m = mag_bits(x);
+  return (int)words(x).hi >= 0 && m > mag_bits(e) && m <= kInfBits;
 }
 
 // Smeared Heaviside inside its band |phi| <= eps (HeavisideFunction,
@@ -70,7 +109,7 @@ __device__ __forceinline__ void block_max_bits(unsigned long long b, unsigned lo
 }
 // max(|x|, m) as the reference's `if (m <= |x|) m = |x|`: NaN never replaces m.
 __device__ __forceinline__ unsigned long long abs_max_bits(double x, unsigned long long m) {
-  const unsigned long long ab = (unsigned long long)(__double_as_longlong(x) & kAbsBits);
+  const unsigned long long ab = (unsigned long long)mag_bits(x);
   return (ab > m && ab <= (unsigned long long)kInfBits) ? ab : m;
 }
 
@@ -132,12 +171,29 @@ __device__ __forceinline__ R weno5_side(R a1, R a2, R a3, R a4, R a5, R eps) {
          w3 * (cdiv3(a3) + cdiv6(a4 * R(5)) - cdiv6(a5));
 }
 
+// Zero, or a magnitude in [2^-E, 2^E): operands in this range keep every product and
+// quotient of the fast forms below normal (each caller states its E).
+template <int E>
+__device__ __forceinline__ bool mid_range(double d) {
+  const Words w = words(d);
+  return (w.hi & 0x7fffffffu) - ((1023u - E) << 20) < ((2u * E) << 20) || ((w.hi << 1) | w.lo) == 0u;
+}
+
+// The plain FP64 product, for operands outside a fast form's range.  Out of line:
+// inlined, the compiler evaluates both forms and selects.
+static __device__ __noinline__ double plain_mul(double a, double b) { return a * b; }
+// a b for b in [2^-100, 2^100] on the integer pipes; where the product may leave the
+// normal range the FP64 multiply.  An FP64 instruction takes an SM's FP64 pipe 16 cycles a
+// warp and mul_rn its integer pipes about 14, so a kernel is fastest with its products
+// shared out between the two.
+__device__ __forceinline__ double mul_wide(double a, double b) { return mid_range<900>(a) ? mul_rn(a, b) : plain_mul(a, b); }
+
 // Range of the differences (and of epsilon) in which weno5_side_fast equals
 // weno5_side<double> bit for bit: zero, or a magnitude in [2^-300, 2^100);
 // epsilon in [2^-100, 2^100].
 __device__ __forceinline__ bool weno5_in_range(double d) {
-  const unsigned h = (unsigned)(__double_as_longlong(d) >> 32) & 0x7fffffffu;
-  return h - ((1023u - 300u) << 20) < (400u << 20) || (__double_as_longlong(d) & kAbsBits) == 0;
+  const Words w = words(d);
+  return (w.hi & 0x7fffffffu) - ((1023u - 300u) << 20) < (400u << 20) || ((w.hi << 1) | w.lo) == 0u;
 }
 
 // weno5_side<double> with the same bits and a fifth of its FP64 operations (27

@@ -145,10 +145,13 @@ __device__ __forceinline__ double in_prec(double v, double) { return v; }
 
 // Level 0 from the assembled FP64 system: conductances beta/dx^2 on interior
 // faces, zero on walls; diagonal as assembled; shift = pin + (dx != dy) terms.
+// lean: without 1/diagonal and shift, which only smoothing and coarsening this level
+// need (the mixed path's FP64 level serves the CG alone; the FP64 quotient took most of
+// the launch: 96 us at 2048^2).
 template <typename T>
 __global__ void k_build_level0(const double* __restrict__ bx, const double* __restrict__ by, const double* __restrict__ diag,
                                const double* __restrict__ rhs, const double* __restrict__ shift, Level<T> L, double* __restrict__ b64,
-                               double idx2_, double idy2_) {
+                               double idx2_, double idy2_, int lean) {
   int ni = L.nI, nj = L.nJ;
   const T idx2 = in_prec(idx2_, T()), idy2 = in_prec(idy2_, T()), zero = 0;
   GB_FOR_IJ(i, j, ni, nj) {
@@ -162,6 +165,8 @@ __global__ void k_build_level0(const double* __restrict__ bx, const double* __re
     if (j == nj - 1) L.cy[k + L.ld] = zero;
     const T d = in_prec(diag[t], T());
     L.dg[k] = d;
+    if (b64) b64[k] = rhs[t];
+    if (lean) continue;
     L.idg[k] = (T)1 / d;
     if (shift) {  // a system that states its diagonal beyond the face conductances itself
       L.sh[k] = in_prec(shift[t], T());
@@ -170,7 +175,6 @@ __global__ void k_build_level0(const double* __restrict__ bx, const double* __re
       const T pin = (i == 0 && j == 0) ? (bl + bb) : zero;
       L.sh[k] = pin * idx2 + ybeta * (idx2 - idy2);
     }
-    if (b64) b64[k] = rhs[t];
   }
 }
 
@@ -1497,17 +1501,17 @@ template <typename T>
 void build_hierarchy(cudaStream_t s, Hierarchy<T>& H, const gb2d_ctx* c, double* b64, double* ainv) {
   double idx2 = 1.0 / (c->base.dx * c->base.dx), idy2 = 1.0 / (c->base.dy * c->base.dy);
   Level<T>& L0 = H.L[0];
-  k_build_level0<T><<<grid_ij(L0.nI, L0.nJ), kThreads, 0, s>>>(c->bx, c->by, c->diag, c->rhs, c->sys_shift, L0, b64, idx2, idy2);
+  k_build_level0<T><<<grid_ij(L0.nI, L0.nJ), kThreads, 0, s>>>(c->bx, c->by, c->diag, c->rhs, c->sys_shift, L0, b64, idx2, idy2, 0);
   GB_LAUNCHED(1);
   build_coarse<T>(s, H, ainv);
 }
 
 // Only the finest FP64 level (the refinement residual's operator) and b.
-void build_level0_f64(cudaStream_t s, Hierarchy<double>& H, const gb2d_ctx* c, double* b64) {
+void build_level0_f64(cudaStream_t s, Hierarchy<double>& H, const gb2d_ctx* c, double* b64, int lean) {
   double idx2 = 1.0 / (c->base.dx * c->base.dx), idy2 = 1.0 / (c->base.dy * c->base.dy);
   Level<double>& L0 = H.L[0];
   k_build_level0<double><<<grid_ij(L0.nI, L0.nJ), kThreads, 0, s>>>(c->bx, c->by, c->diag, c->rhs, c->sys_shift, L0, b64, idx2,
-                                                                     idy2);
+                                                                     idy2, lean);
   GB_LAUNCHED(1);
 }
 
@@ -2144,7 +2148,7 @@ void solver_prebuild(gb2d_ctx* c, const gb2d_solve_opts* o) {
   } else {
     // The FP64 finest level first (the residual waits for it; solver_solve copies its
     // right-hand side once that exists), then the coarse levels and dense inverse.
-    build_level0_f64(c->side2, S->h64, c, nullptr);
+    build_level0_f64(c->side2, S->h64, c, nullptr, 0);
     cudaEventRecord(c->ev_pre0, c->side2);
     build_coarse<double>(c->side2, S->h64, S->ainv64);
   }
@@ -2282,7 +2286,7 @@ int solver_solve(gb2d_ctx* c, const double* /*rhs*/, double* x, const gb2d_solve
   } else if (use_mg && S->prebuilt) {
     // Started by solver_prebuild during the assembly; joined before the first V-cycle.
     if (prec) {
-      build_level0_f64(s, S->h64, c, S->b64);
+      build_level0_f64(s, S->h64, c, S->b64, 1);
     } else {  // b here, the finest FP64 level before the residual
       launch_copy_interior(s, c->rhs, 0, S->b64, 1, c->grid.ni, c->grid.nj);
       cudaStreamWaitEvent(s, c->ev_pre0, 0);
@@ -2299,7 +2303,7 @@ int solver_solve(gb2d_ctx* c, const double* /*rhs*/, double* x, const gb2d_solve
       cudaEventRecord(c->ev_join, c->side);
     }
     if (prec || !use_mg)
-      build_level0_f64(s, S->h64, c, S->b64);
+      build_level0_f64(s, S->h64, c, S->b64, prec);
     else
       build_hierarchy<double>(s, S->h64, c, S->b64, S->ainv64);
   }
@@ -2307,7 +2311,7 @@ int solver_solve(gb2d_ctx* c, const double* /*rhs*/, double* x, const gb2d_solve
   if (prec && !use_mg && !keep) {
     double idx2 = 1.0 / (c->base.dx * c->base.dx), idy2 = 1.0 / (c->base.dy * c->base.dy);
     k_build_level0<float><<<grid_ij(c->grid.ni, c->grid.nj), kThreads, 0, s>>>(c->bx, c->by, c->diag, c->rhs, c->sys_shift,
-                                                                                                S->h32.L[0], nullptr, idx2, idy2);
+                                                                                                S->h32.L[0], nullptr, idx2, idy2, 0);
     GB_LAUNCHED(1);
   }
   if (c->graph_mode) {
