@@ -6,6 +6,8 @@
 // Built with --fmad=false, in the reference's association order, like
 // gb2d_exact.cu: the results are the reference's FP64 results bit for bit, except
 // where the smeared Heaviside's sine (the only libm call) differs in the last ulp.
+#include <cmath>
+
 #include "gb2d_internal.cuh"
 #include "gb2d_schemes.cuh"
 
@@ -47,21 +49,8 @@ struct FlowArgs {
   // FP32 viscous-flux path
   float odx_f, ody_f, eps_f, oe_f, dt_f, coef0_f, coef1_f;
   SmearF rho_f, mu_f;
+  int fast;            // densities, viscosities and cell sizes are in the fast products' range
 };
-
-__device__ __forceinline__ double smear(double l, const Smear& s, const FlowArgs& a) {
-  if (lt_neg(l, a.eps)) return s.at0;
-  if (gt_pos(l, a.eps)) return s.at1;
-  return s.lo + s.d * heaviside_band(l, a.oe);
-}
-
-// dt / rho of a face: rho takes two values outside the band, whose quotients the
-// host formed (FP64 divisions are scarce on this part).
-__device__ __forceinline__ double face_coef(double l, const FlowArgs& a) {
-  if (lt_neg(l, a.eps)) return a.coef0;
-  if (gt_pos(l, a.eps)) return a.coef1;
-  return a.dt * (1 / (a.rho.lo + a.rho.d * heaviside_band(l, a.oe)));
-}
 
 // FP32 forms for the viscous flux of the mixed path.
 __device__ __forceinline__ float heaviside_band_f(float phi, float oe) {
@@ -72,11 +61,6 @@ __device__ __forceinline__ float smear_f(float l, const SmearF& s, const FlowArg
   if (l < -a.eps_f) return s.at0;
   if (l > a.eps_f) return s.at1;
   return s.lo + s.d * heaviside_band_f(l, a.oe_f);
-}
-__device__ __forceinline__ float face_coef_f(float l, const FlowArgs& a) {
-  if (l < -a.eps_f) return a.coef0_f;
-  if (l > a.eps_f) return a.coef1_f;
-  return __fdividef(a.dt_f, a.rho_f.lo + a.rho_f.d * heaviside_band_f(l, a.oe_f));
 }
 
 // The dt-dependent fields of FlowArgs, as launch_flow forms them on the host.
@@ -91,127 +75,232 @@ __host__ __device__ __forceinline__ void with_time_step(FlowArgs& a, double dt) 
   a.coef1_f = (float)a.coef1;
 }
 
-// One pass over the (ni+1) x (nj+1) face index space: x-face (i, j), i <= ni,
-// j < nj; y-face (i, j), i < ni, j <= nj; node (i, j) for the density.
-//   VISC = false: gravity and wall conditions in place (u_out may equal u_in).
-//   VISC = true:  ApplyViscosity from the copies temp_x / temp_y of the faces after
-//                 gravity, whose values off the face grids are zero (the reference's
-//                 freshly initialised temporaries), written to u_out / v_out.
-//   MIXED (with VISC): the viscous flux in FP32 from FP64 velocity differences (the
-//                 face values and the update stay FP64).
+// Gravity and wall conditions over the (ni+1) x (nj+1) face index space, in place: x-face
+// (i, j), i <= ni, j < nj; y-face (i, j), i < ni, j <= nj; node (i, j) for the density.
 // density (ghost 2, may be null) receives DetermineDensity (:2162-2180): air where
 // phi <= 0, water where phi > 0, unchanged for NaN.
-template <bool VISC, bool MIXED>
-__global__ void k_flow(const double* __restrict__ phi_a, const double* u_in_a, const double* v_in_a, double* u_out_a,
-                       double* v_out_a, double* __restrict__ dens_a, FlowArgs a) {
+__device__ __forceinline__ void put_density(double* dens_a, const FlowArgs& a, int i, int j, double l) {
+  const DField dn = dfield(dens_a, 2, a.ni, a.nj);
+  if (lez(l))
+    GB_AT(dn, i, j) = a.air;
+  else if (gtz(l))
+    GB_AT(dn, i, j) = a.water;
+}
+__global__ void k_flow(const double* __restrict__ phi_a, double* u_a, double* v_a, double* __restrict__ dens_a, FlowArgs a) {
+  pdl_enter();
   if (a.dtp) with_time_step(a, *a.dtp);
   const int ni = a.ni, nj = a.nj;
-  const DField phi = dfield((double*)phi_a, 2, ni, nj);
-  const DField ui = dfield((double*)u_in_a, 2, ni + 1, nj), vi = dfield((double*)v_in_a, 2, ni, nj + 1);
-  const DField uo = dfield(u_out_a, 2, ni + 1, nj), vo = dfield(v_out_a, 2, ni, nj + 1);
-  auto tu = [&](int i, int j) -> double {
-    if (i < 0 || i > ni || j < 0 || j >= nj) return 0.0;
-    const double w = GB_AT(ui, i, j);
-    return a.grav ? w + a.gx : w;
-  };
-  auto tv = [&](int i, int j) -> double {
-    if (i < 0 || i >= ni || j < 0 || j > nj) return 0.0;
-    const double w = GB_AT(vi, i, j);
-    return a.grav ? w + a.gy : w;
-  };
-  auto P = [&](int i, int j) -> double { return __ldg(&GB_AT(phi, i, j)); };
-  // Face values without gravity: off the grids -gravity, so that differences of
-  // these equal differences of the temporaries.
-  auto ru = [&](int i, int j) -> double {
-    if (i < 0 || i > ni || j < 0 || j >= nj) return a.grav ? -a.gx : 0.0;
-    return GB_AT(ui, i, j);
-  };
-  auto rv = [&](int i, int j) -> double {
-    if (i < 0 || i >= ni || j < 0 || j > nj) return a.grav ? -a.gy : 0.0;
-    return GB_AT(vi, i, j);
-  };
-  auto Pf = [&](int i, int j) -> float { return narrow(__ldg(&GB_AT(phi, i, j))); };
+  const DField phi = dfield((double*)phi_a, 2, ni, nj), u = dfield(u_a, 2, ni + 1, nj), v = dfield(v_a, 2, ni, nj + 1);
   GB_FOR_IJ(i, j, ni + 1, nj + 1) {
-    if (dens_a && i < ni && j < nj) {
-      const double l = P(i, j);
-      DField dn = dfield(dens_a, 2, ni, nj);
-      if (lez(l))
-        GB_AT(dn, i, j) = a.air;
-      else if (gtz(l))
-        GB_AT(dn, i, j) = a.water;
-    }
-    if (j < nj) {  // x-face between nodes (i-1, j) and (i, j)
-      double w;
-      if (VISC && MIXED) {
-        const float pl = Pf(i - 1, j), pc = Pf(i, j);
-        const float cu = 0.25f * (pl + pc + Pf(i - 1, j + 1) + Pf(i, j + 1));
-        const float cd = 0.25f * (Pf(i - 1, j - 1) + Pf(i, j - 1) + pl + pc);
-        const float mu_cu = smear_f(cu, a.mu_f, a), mu_cd = smear_f(cd, a.mu_f, a);
-        const float mu_r = smear_f(pc, a.mu_f, a), mu_c = smear_f(pl, a.mu_f, a);
-        const float coef = face_coef_f(0.5f * (pl + pc), a);
-        const double u0 = ru(i, j);
-        const float dxp = narrow(ru(i + 1, j) - u0), dxm = narrow(u0 - ru(i - 1, j));
-        const float dyp = narrow(ru(i, j + 1) - u0), dym = narrow(u0 - ru(i, j - 1));
-        const float dvu = narrow(rv(i, j + 1) - rv(i - 1, j + 1)), dvd = narrow(rv(i, j) - rv(i - 1, j));
-        const float first = 2.0f * coef * a.odx_f * (mu_r * a.odx_f * dxp - mu_c * a.odx_f * dxm);
-        const float second = coef * a.ody_f * (mu_cu * (a.ody_f * dyp + a.odx_f * dvu) - mu_cd * (a.ody_f * dym + a.odx_f * dvd));
-        w = (a.grav ? u0 + a.gx : u0) + widen(first + second);
-      } else if (VISC) {
-        const double pl = P(i - 1, j), pc = P(i, j);
-        const double half = 0.5 * (pl + pc);
-        const double cu = 0.25 * (pl + pc + P(i - 1, j + 1) + P(i, j + 1));
-        const double cd = 0.25 * (P(i - 1, j - 1) + P(i, j - 1) + pl + pc);
-        const double mu_cu = smear(cu, a.mu, a), mu_cd = smear(cd, a.mu, a);
-        const double mu_r = smear(pc, a.mu, a), mu_c = smear(pl, a.mu, a);
-        const double coef = face_coef(half, a);
-        const double t0 = tu(i, j);
-        const double first = 2.0 * coef * a.odx * (mu_r * a.odx * (tu(i + 1, j) - t0) - mu_c * a.odx * (t0 - tu(i - 1, j)));
-        const double second = coef * a.ody *
-                               (mu_cu * (a.ody * (tu(i, j + 1) - t0) + a.odx * (tv(i, j + 1) - tv(i - 1, j + 1))) -
-                                mu_cd * (a.ody * (t0 - tu(i, j - 1)) + a.odx * (tv(i, j) - tv(i - 1, j))));
-        w = t0 + (first + second);
-      } else {
-        w = tu(i, j);
-      }
+    if (dens_a && i < ni && j < nj) put_density(dens_a, a, i, j, GB_AT(phi, i, j));
+    if (j < nj) {
+      double w = GB_AT(u, i, j);
+      if (a.grav) w = w + a.gx;
       if (a.bc && (i == 0 || i == ni)) w = 0.0;
-      GB_AT(uo, i, j) = w;
+      GB_AT(u, i, j) = w;
     }
-    if (i < ni) {  // y-face between nodes (i, j-1) and (i, j)
-      double w;
-      if (VISC && MIXED) {
-        const float pb = Pf(i, j - 1), pc = Pf(i, j);
-        const float cu = 0.25f * (pb + Pf(i + 1, j - 1) + pc + Pf(i + 1, j));
-        const float cl = 0.25f * (Pf(i - 1, j - 1) + pb + Pf(i - 1, j) + pc);
-        const float mu_cu = smear_f(cu, a.mu_f, a), mu_cl = smear_f(cl, a.mu_f, a);
-        const float mu_u = smear_f(pc, a.mu_f, a), mu_c = smear_f(pb, a.mu_f, a);
-        const float coef = face_coef_f(0.5f * (pb + pc), a);
-        const double v0 = rv(i, j);
-        const float dyp = narrow(rv(i, j + 1) - v0), dym = narrow(v0 - rv(i, j - 1));
-        const float dur = narrow(ru(i + 1, j) - ru(i + 1, j - 1)), dul = narrow(ru(i, j) - ru(i, j - 1));
-        const float dxp = narrow(rv(i + 1, j) - v0), dxm = narrow(v0 - rv(i - 1, j));
-        const float first = 2.0f * coef * a.ody_f * (mu_u * a.ody_f * dyp - mu_c * a.ody_f * dym);
-        const float second = coef * a.odx_f * (mu_cu * (a.ody_f * dur + a.odx_f * dxp) - mu_cl * (a.ody_f * dul + a.odx_f * dxm));
-        w = (a.grav ? v0 + a.gy : v0) + widen(first + second);
-      } else if (VISC) {
-        const double pb = P(i, j - 1), pc = P(i, j);
-        const double half = 0.5 * (pb + pc);
-        const double cu = 0.25 * (pb + P(i + 1, j - 1) + pc + P(i + 1, j));
-        const double cl = 0.25 * (P(i - 1, j - 1) + pb + P(i - 1, j) + pc);
-        const double mu_cu = smear(cu, a.mu, a), mu_cl = smear(cl, a.mu, a);
-        const double mu_u = smear(pc, a.mu, a), mu_c = smear(pb, a.mu, a);
-        const double coef = face_coef(half, a);
-        const double t0 = tv(i, j);
-        const double first = 2.0 * coef * a.ody * (mu_u * a.ody * (tv(i, j + 1) - t0) - mu_c * a.ody * (t0 - tv(i, j - 1)));
-        const double second = coef * a.odx *
-                              (mu_cu * (a.ody * (tu(i + 1, j) - tu(i + 1, j - 1)) + a.odx * (tv(i + 1, j) - t0)) -
-                               mu_cl * (a.ody * (tu(i, j) - tu(i, j - 1)) + a.odx * (t0 - tv(i - 1, j))));
-        w = t0 + (first + second);
-      } else {
-        w = tv(i, j);
-      }
+    if (i < ni) {
+      double w = GB_AT(v, i, j);
+      if (a.grav) w = w + a.gy;
       if (a.bc && (j == 0 || j == nj)) w = 0.0;
-      GB_AT(vo, i, j) = w;
+      GB_AT(v, i, j) = w;
     }
+  }
+}
+
+// ---- the explicit viscosity (ApplyViscosity) with gravity and walls ----
+//
+// With T the faces after gravity (zero off the face grids, the reference's freshly
+// initialised temporaries), node terms and corner terms
+//   X(i, j) = mu(phi(i, j)) ox (Tu(i+1, j) - Tu(i, j)),   Y(i, j) = mu(phi(i, j)) oy (Tv(i, j+1) - Tv(i, j)),
+//   K(i, j) = mu(phi at the lower left corner) (oy (Tu(i, j) - Tu(i, j-1)) + ox (Tv(i, j) - Tv(i-1, j))),
+// the new faces are
+//   u = Tu + (2 c ox (X(i, j) - X(i-1, j)) + c oy (K(i, j+1) - K(i, j))),
+//   v = Tv + (2 c oy (Y(i, j) - Y(i, j-1)) + c ox (K(i+1, j) - K(i, j))),   c = dt / rho of the face,
+// every term with the operations, and their order, of the reference's expression: a term
+// that two or four faces share is the same number in each.  A tile forms each term once
+// (20 FP64 additions a node instead of 55 operations a face), products on the integer
+// pipes.  MIXED (R = float): the terms in FP32 from FP64 differences of the faces before
+// gravity (off the grids minus gravity, so that the differences are those of T), the face
+// values and the update FP64.
+constexpr int kFlX = 32, kFlY = 8;
+template <typename R>
+struct FlowTile {
+  double u[kFlY + 2][kFlX + 2], v[kFlY + 2][kFlX + 2];  // faces (i0 - 1 + x, j0 - 1 + y)
+  R p[kFlY + 2][kFlX + 2], mu[kFlY + 2][kFlX + 2];      // phi and mu(phi) at nodes (i0 - 1 + x, j0 - 1 + y)
+  R X[kFlY][kFlX + 1], Y[kFlY + 1][kFlX], K[kFlY + 1][kFlX + 1];
+};
+// dt-derived values, formed once per block.
+template <typename R>
+struct FlowStep {
+  double gx, gy;
+  R dt, c0, c1, c0x2, c1x2, c0y2, c1y2, c0x, c1x, c0y, c1y;  // c: outside the band; 2 c ox, 2 c oy, c ox, c oy
+  int ok;                                                    // they are in the fast products' range
+};
+__device__ __noinline__ double smear_band(double l, const Smear& s, double oe) { return s.lo + s.d * heaviside_band(l, oe); }
+__device__ __noinline__ double coef_band(double l, const Smear& s, double oe, double dt) { return dt * (1 / (s.lo + s.d * heaviside_band(l, oe))); }
+__device__ __forceinline__ double visc_mu(double l, const FlowArgs& a) {
+  if (lt_neg(l, a.eps)) return a.mu.at0;
+  if (gt_pos(l, a.eps)) return a.mu.at1;
+  return smear_band(l, a.mu, a.oe);
+}
+__device__ __forceinline__ float visc_mu(float l, const FlowArgs& a) { return smear_f(l, a.mu_f, a); }
+template <bool FAST>
+__device__ __forceinline__ double visc_mul(double x, double y) { return FAST ? mul_rn(x, y) : x * y; }
+template <bool FAST>
+__device__ __forceinline__ float visc_mul(float x, float y) { return x * y; }
+__device__ __forceinline__ double visc_quarter(double s) { return mul_wide(s, 0.25); }
+__device__ __forceinline__ float visc_quarter(float s) { return 0.25f * s; }
+__device__ __forceinline__ double visc_half(double s) { return mul_wide(s, 0.5); }
+__device__ __forceinline__ float visc_half(float s) { return 0.5f * s; }
+__device__ __forceinline__ double visc_diff(double x, double y, double) { return x - y; }
+__device__ __forceinline__ float visc_diff(double x, double y, float) { return narrow(x - y); }
+// 2 c o and c o of a face whose phi averages to l: o = ox (along = true) for 2 c o and the
+// other cell size for c o.
+__device__ __forceinline__ void visc_coef(double l, bool xface, const FlowArgs& a, const FlowStep<double>& t, double& c2, double& c1) {
+  if (lt_neg(l, a.eps)) {
+    c2 = xface ? t.c0x2 : t.c0y2;
+    c1 = xface ? t.c0y : t.c0x;
+  } else if (gt_pos(l, a.eps)) {
+    c2 = xface ? t.c1x2 : t.c1y2;
+    c1 = xface ? t.c1y : t.c1x;
+  } else {
+    const double c = coef_band(l, a.rho, a.oe, t.dt);
+    c2 = 2.0 * c * (xface ? a.odx : a.ody);
+    c1 = c * (xface ? a.ody : a.odx);
+  }
+}
+__device__ __forceinline__ void visc_coef(float l, bool xface, const FlowArgs& a, const FlowStep<float>& t, float& c2, float& c1) {
+  const float c = l < -a.eps_f ? t.c0 : l > a.eps_f ? t.c1 : __fdividef(t.dt, a.rho_f.lo + a.rho_f.d * heaviside_band_f(l, a.oe_f));
+  c2 = 2.0f * c * (xface ? a.odx_f : a.ody_f);
+  c1 = c * (xface ? a.ody_f : a.odx_f);
+}
+
+// The tile's terms and new faces, after its staging.  FAST: every product on the integer pipes.
+template <typename R, bool FAST>
+__device__ __forceinline__ void flow_tile(FlowTile<R>& t, const FlowStep<R>& st, const FlowArgs& a, int i0, int j0, DField uo, DField vo) {
+  constexpr int NT = kFlX * kFlY, W = kFlX + 1;
+  constexpr bool MIXED = sizeof(R) == 4;
+  const int tid = threadIdx.x, tx = tid & (kFlX - 1), ty = tid / kFlX, i = i0 + tx, j = j0 + ty;
+  R ox, oy;
+  if constexpr (MIXED) {
+    ox = a.odx_f;
+    oy = a.ody_f;
+  } else {
+    ox = a.odx;
+    oy = a.ody;
+  }
+  for (int k = tid; k < kFlY * W; k += NT) {  // X of nodes (i0 - 1 + x, j0 + y)
+    const int y = k / W, x = k - y * W;
+    t.X[y][x] = visc_mul<FAST>(visc_mul<FAST>(t.mu[y + 1][x], ox), visc_diff(t.u[y + 1][x + 1], t.u[y + 1][x], R()));
+  }
+  for (int k = tid; k < (kFlY + 1) * kFlX; k += NT) {  // Y of nodes (i0 + x, j0 - 1 + y)
+    const int y = k / kFlX, x = k - y * kFlX;
+    t.Y[y][x] = visc_mul<FAST>(visc_mul<FAST>(t.mu[y][x + 1], oy), visc_diff(t.v[y + 1][x + 1], t.v[y][x + 1], R()));
+  }
+  for (int k = tid; k < (kFlY + 1) * W; k += NT) {  // K of the lower left corners of nodes (i0 + x, j0 + y)
+    const int y = k / W, x = k - y * W;
+    const R mu = visc_mu(visc_quarter(t.p[y][x] + t.p[y][x + 1] + t.p[y + 1][x] + t.p[y + 1][x + 1]), a);
+    const R du = visc_mul<FAST>(oy, visc_diff(t.u[y + 1][x + 1], t.u[y][x + 1], R()));
+    const R dv = visc_mul<FAST>(ox, visc_diff(t.v[y + 1][x + 1], t.v[y + 1][x], R()));
+    t.K[y][x] = visc_mul<FAST>(mu, du + dv);
+  }
+  __syncthreads();
+  const R pc = t.p[ty + 1][tx + 1];
+  R c2, c1;
+  if (i <= a.ni && j < a.nj) {
+    visc_coef(visc_half(t.p[ty + 1][tx] + pc), true, a, st, c2, c1);
+    const R f = visc_mul<FAST>(c2, t.X[ty][tx + 1] - t.X[ty][tx]) + visc_mul<FAST>(c1, t.K[ty + 1][tx] - t.K[ty][tx]);
+    double w = t.u[ty + 1][tx + 1];
+    if (MIXED && a.grav) w = w + st.gx;
+    w = w + widen(f);
+    if (a.bc && (i == 0 || i == a.ni)) w = 0.0;
+    GB_AT(uo, i, j) = w;
+  }
+  if (i < a.ni && j <= a.nj) {
+    visc_coef(visc_half(t.p[ty][tx + 1] + pc), false, a, st, c2, c1);
+    const R f = visc_mul<FAST>(c2, t.Y[ty + 1][tx] - t.Y[ty][tx]) + visc_mul<FAST>(c1, t.K[ty][tx + 1] - t.K[ty][tx]);
+    double w = t.v[ty + 1][tx + 1];
+    if (MIXED && a.grav) w = w + st.gy;
+    w = w + widen(f);
+    if (a.bc && (j == 0 || j == a.nj)) w = 0.0;
+    GB_AT(vo, i, j) = w;
+  }
+}
+// Out of line: differences outside the fast products' range.
+__device__ __noinline__ void flow_tile_plain(FlowTile<double>& t, const FlowStep<double>& st, const FlowArgs& a, int i0, int j0, DField uo,
+                                             DField vo) {
+  flow_tile<double, false>(t, st, a, i0, j0, uo, vo);
+}
+
+// u_in / v_in to u_out / v_out (other buffers); density as k_flow.  225 -> 83 us at
+// 1000 x 750 (FP64), 183 -> 109 us at 2048^2 (mixed).
+template <typename R>
+__global__ void __launch_bounds__(kFlX* kFlY) k_flow_visc(const double* __restrict__ phi_a, const double* __restrict__ u_in,
+                                                          const double* __restrict__ v_in, double* __restrict__ u_out,
+                                                          double* __restrict__ v_out, double* __restrict__ dens_a, const FlowArgs a) {
+  constexpr int NT = kFlX * kFlY, W = kFlX + 2;
+  constexpr bool MIXED = sizeof(R) == 4;
+  pdl_enter();
+  __shared__ FlowTile<R> t;
+  __shared__ FlowStep<R> st;
+  const int ni = a.ni, nj = a.nj, tid = threadIdx.x;
+  const int i0 = (int)blockIdx.x * kFlX, j0 = (int)blockIdx.y * kFlY;
+  const DField phi = dfield((double*)phi_a, 2, ni, nj);
+  const DField ui = dfield((double*)u_in, 2, ni + 1, nj), vi = dfield((double*)v_in, 2, ni, nj + 1);
+  if (tid == 0) {
+    FlowArgs b = a;
+    if (a.dtp) with_time_step(b, *a.dtp);
+    st.gx = b.gx;
+    st.gy = b.gy;
+    if constexpr (MIXED) {
+      st.dt = b.dt_f;
+      st.c0 = b.coef0_f;
+      st.c1 = b.coef1_f;
+    } else {
+      st.dt = b.dt;
+      st.c0x2 = 2.0 * b.coef0 * a.odx, st.c1x2 = 2.0 * b.coef1 * a.odx;
+      st.c0y2 = 2.0 * b.coef0 * a.ody, st.c1y2 = 2.0 * b.coef1 * a.ody;
+      st.c0x = b.coef0 * a.odx, st.c1x = b.coef1 * a.odx, st.c0y = b.coef0 * a.ody, st.c1y = b.coef1 * a.ody;
+      st.ok = a.fast && mid_range<200>(b.dt) && mid_range<200>(b.coef0) && mid_range<200>(b.coef1);
+    }
+  }
+  __syncthreads();
+  bool ok = true;
+  for (int k = tid; k < (kFlY + 2) * W; k += NT) {
+    const int y = k / W, x = k - y * W, i = i0 - 1 + x, j = j0 - 1 + y;
+    const double l = __ldg(&GB_AT(phi, i < ni + 2 ? i : ni + 1, j < nj + 2 ? j : nj + 1));
+    R p;
+    if constexpr (MIXED)
+      p = narrow(l);
+    else
+      p = l;
+    t.p[y][x] = p;
+    t.mu[y][x] = visc_mu(p, a);
+    // Off the grids T is zero: FP64 tiles hold T, FP32 tiles the faces before gravity.
+    double u = MIXED && a.grav ? negd(st.gx) : 0.0, v = MIXED && a.grav ? negd(st.gy) : 0.0;
+    if (i >= 0 && i <= ni && j >= 0 && j < nj) {
+      u = GB_AT(ui, i, j);
+      if (!MIXED && a.grav) u = u + st.gx;
+    }
+    if (i >= 0 && i < ni && j >= 0 && j <= nj) {
+      v = GB_AT(vi, i, j);
+      if (!MIXED && a.grav) v = v + st.gy;
+    }
+    t.u[y][x] = u;
+    t.v[y][x] = v;
+    if (!MIXED) ok = ok && mid_range<200>(u) && mid_range<200>(v) && mid_range<200>(l);
+    if (dens_a && x >= 1 && x <= kFlX && y >= 1 && y <= kFlY && i < ni && j < nj) put_density(dens_a, a, i, j, l);
+  }
+  const bool fast = __syncthreads_and(MIXED || (ok && st.ok));
+  const DField uo = dfield(u_out, 2, ni + 1, nj), vo = dfield(v_out, 2, ni, nj + 1);
+  if constexpr (MIXED) {
+    flow_tile<R, true>(t, st, a, i0, j0, uo, vo);
+  } else {
+    if (fast)
+      flow_tile<R, true>(t, st, a, i0, j0, uo, vo);
+    else
+      flow_tile_plain(t, st, a, i0, j0, uo, vo);
   }
 }
 
@@ -337,10 +426,14 @@ void launch_flow(cudaStream_t s, gb2d_ctx* c, double dt, int grav, int visc, int
   const double* phi = c->phi_buf[c->phi_cur];
   const bool mixed = c->prm.advection_precision == GB2D_PRECISION_MIXED;
   if (visc) {
+    auto mid = [](double x) { return x == 0 || (std::fabs(x) >= 0x1p-60 && std::fabs(x) <= 0x1p60); };
+    a.fast = mid(a.mu.lo) && mid(a.mu.at0) && mid(a.mu.at1) && mid(a.rho.at0) && mid(a.rho.at1) && mid(a.odx) && mid(a.ody) && a.odx > 0 &&
+             a.ody > 0 && mid(c->prm.water_density) && mid(c->prm.air_density);
+    const dim3 grd((ni + kFlX) / kFlX, (nj + kFlY) / kFlY);  // covers ni + 1 and nj + 1 faces
     if (mixed)
-      k_flow<true, true><<<grid_ij(ni + 1, nj + 1), kThreads, 0, s>>>(phi, c->u, c->v, c->u_alt, c->v_alt, density, a);
+      pdl_launch(s, grd, kFlX * kFlY, 0, k_flow_visc<float>, phi, (const double*)c->u, (const double*)c->v, c->u_alt, c->v_alt, density, a);
     else
-      k_flow<true, false><<<grid_ij(ni + 1, nj + 1), kThreads, 0, s>>>(phi, c->u, c->v, c->u_alt, c->v_alt, density, a);
+      pdl_launch(s, grd, kFlX * kFlY, 0, k_flow_visc<double>, phi, (const double*)c->u, (const double*)c->v, c->u_alt, c->v_alt, density, a);
     double* t = c->u;
     c->u = c->u_alt;
     c->u_alt = t;
@@ -348,7 +441,8 @@ void launch_flow(cudaStream_t s, gb2d_ctx* c, double dt, int grav, int visc, int
     c->v = c->v_alt;
     c->v_alt = t;
   } else {
-    k_flow<false, false><<<grid_ij(ni + 1, nj + 1), kThreads, 0, s>>>(phi, c->u, c->v, c->u, c->v, density, a);
+    a.fast = 0;
+    pdl_launch(s, grid_ij(ni + 1, nj + 1), kThreads, 0, k_flow, phi, c->u, c->v, density, a);
   }
   GB_LAUNCHED(1);
 }

@@ -343,13 +343,4 @@ __device__ __forceinline__ void eno3_pair(const double q[7], double o, double o2
   eno3_select<double>(d, o2, o3, h, dm, dp);
 }
 
-// Mixed pair: differences of the FP64 state formed in FP64, the divided
-// differences and the selection in FP32.
-__device__ __forceinline__ void eno3_pair_f32(const double q[7], float o, float o2, float o3, float h, float& dm, float& dp) {
-  float d[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) d[k] = narrow(q[k + 1] - q[k]) * o;
-  eno3_select<float>(d, o2, o3, h, dm, dp);
-}
-
 }  // namespace gb2d
