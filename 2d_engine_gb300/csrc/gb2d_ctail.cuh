@@ -169,8 +169,9 @@ __device__ __forceinline__ void ct_load(const CtLevel<T>& L, const CtWin& w, con
 // One colour of a red-black Gauss-Seidel sweep over the window's pairs [lo, hi).  The
 // pair's cells are (2m, J), (2m + 1, J); the red one is 2m + (J & 1).  A cell's horizontal
 // neighbours are the pair's other cell and the neighbouring pair's cell of the other
-// colour; its vertical ones sit at the same pair of rows J -+ 1.
-template <int COLOR, typename T, int K>
+// colour; its vertical ones sit at the same pair of rows J -+ 1.  FIRST: x is zero, and
+// the update is b / dg.
+template <int COLOR, bool FIRST, typename T, int K>
 __device__ __forceinline__ void ct_half(T* xp, int xplane, int ps, CtRegs<T, K>& g, int lo, int hi) {
   const T* xo = xp + (COLOR == 0 ? xplane : 0);
   T* xw = xp + (COLOR == 0 ? 0 : xplane);
@@ -179,6 +180,10 @@ __device__ __forceinline__ void ct_half(T* xp, int xplane, int ps, CtRegs<T, K>&
     const int u = (int)threadIdx.x + k * kCtThreads;
     if (u < lo || u >= hi) continue;
     const int ad = g.ad[k];
+    if (FIRST) {
+      xw[ad] = g.x[COLOR][k] = mulr(g.b[COLOR][k], g.idg[COLOR][k]);
+      continue;
+    }
     const bool right = (g.od[k] != 0) == (COLOR == 0);  // the cell is the pair's right one
     const T own = g.x[1 - COLOR][k], side = xo[right ? ad + 1 : ad - 1], xb = xo[ad - ps], xt = xo[ad + ps];
     const T v = gs_update(g.b[COLOR][k], g.cl[COLOR][k], right ? own : side, g.cr[COLOR][k], right ? side : own, g.y0[COLOR][k], xb,
@@ -207,10 +212,13 @@ __device__ __forceinline__ void ct_smooth(const CtLevel<T>& L, const CtWin& w, T
   const int o0 = (w.J0 - w.w0) * L.pairs, o1 = (w.J1 - w.w0) * L.pairs;
   int e = (last + 2 * nu - 1) * L.pairs;
   for (int s = 0; s < nu; ++s) {
-    ct_half<C0>(xp, L.xplane, L.pairs + 2, g, o0 - e, o1 + e);
+    if (C0 == 0 && s == 0)  // pre-smoothing starts from x = 0
+      ct_half<C0, C0 == 0>(xp, L.xplane, L.pairs + 2, g, o0 - e, o1 + e);
+    else
+      ct_half<C0, false>(xp, L.xplane, L.pairs + 2, g, o0 - e, o1 + e);
     e -= L.pairs;
     ct_sync<FEW>();
-    ct_half<1 - C0>(xp, L.xplane, L.pairs + 2, g, o0 - e, o1 + e);
+    ct_half<1 - C0, false>(xp, L.xplane, L.pairs + 2, g, o0 - e, o1 + e);
     e -= L.pairs;
     ct_sync<FEW>();
   }

@@ -37,6 +37,7 @@
 #include <mutex>
 #include <utility>
 
+#include "gb2d_exact_math.cuh"
 #include "gb2d_internal.cuh"
 
 namespace gb2d {
@@ -218,17 +219,33 @@ __global__ void k_coarsen(Level<T> F, Level<T> C) {
   }
 }
 
+// Multiply-add and product with every rounding stated.
+__device__ __forceinline__ float fmad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fmad(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mulr(double a, double b) { return __dmul_rn(a, b); }
+
+// 1 / x as the IEEE quotient; an FP64 one on the integer pipes where the exponents allow.
+__device__ __forceinline__ float pivot_inverse(float x) { return 1.0f / x; }
+__device__ __noinline__ double plain_inverse(double x) { return 1.0 / x; }
+__device__ __forceinline__ double pivot_inverse(double x) {
+  const unsigned hi = (unsigned)(dbits(x) >> 32);
+  return hi - ((1023u - 900u) << 20) < (1800u << 20) ? div_pos(1.0, x) : plain_inverse(x);  // positive, 2^-900 <= x < 2^900
+}
+
 // Dense inverse of the coarsest operator (n <= 64), Gauss-Jordan without
-// pivoting (the operator is SPD), computed in the hierarchy's precision (one SM's
-// FP64 rate makes the FP64 elimination ~60 us; the FP32 one takes a few).  One
+// pivoting (the operator is SPD), computed in the hierarchy's precision.  One
 // block of 1024 threads, thread t owning row t/16 and columns t%16 + 16q
-// (q = 0..3) in registers; each pivot step publishes the pivot row, the pivot
-// column and the pivot's reciprocal through shared memory.
+// (q = 0..3) in registers.  A pivot step: the pivot row's half warp takes the pivot by
+// shuffle, forms its reciprocal and publishes the scaled row, the pivot column's owners
+// publish the column; one barrier (the two are double-buffered); everyone updates.
+// FP64 is bound by one SM's FP64 pipe, 64 x 64 FMAs a step (2048 cycles): the row is
+// scaled by its owners, once, and the reciprocal runs on the integer pipes (191 us with
+// every thread scaling and two barriers a step; FP32 39 us).
 template <typename T>
 __global__ void __launch_bounds__(1024) k_dense_inverse(Level<T> C, double* __restrict__ ainv) {
   static_assert(kCoarseMax == 64, "register blocking assumes 64 x 64");
-  __shared__ T prow[kCoarseMax], fcol[kCoarseMax];
-  __shared__ T s_inv;
+  __shared__ T prow[2][kCoarseMax], fcol[2][kCoarseMax], pinv[2];
   const int n = C.nI * C.nJ;
   if (n > kCoarseMax) return;  // prevented on the host (alloc_hierarchy)
   const int r = threadIdx.x >> 4, m0 = threadIdx.x & 15;
@@ -257,30 +274,34 @@ __global__ void __launch_bounds__(1024) k_dense_inverse(Level<T> C, double* __re
     }
   }
   for (int kk = 0; kk < n; ++kk) {
-    const int qk = kk >> 4;
+    const int qk = kk >> 4, mk = kk & 15, par = kk & 1;
     const T own_col = qk == 0 ? a[0] : qk == 1 ? a[1] : qk == 2 ? a[2] : a[3];
-    if (r == kk) {
+    if (r == kk) {  // sixteen threads of one warp
+      const unsigned half = 0xffffu << (threadIdx.x & 16);
+      const T inv = pivot_inverse(__shfl_sync(half, own_col, mk, 16));
 #pragma unroll
-      for (int q = 0; q < 4; ++q) prow[m0 + 16 * q] = a[q];
-      if (m0 == (kk & 15)) s_inv = (T)1 / own_col;
+      for (int q = 0; q < 4; ++q) {
+        const int m = m0 + 16 * q;
+        const T pm = m == kk ? inv : mulr(a[q], inv);
+        if (m < n) a[q] = pm;
+        prow[par][m] = pm;
+      }
+      if (m0 == 0) pinv[par] = inv;
+    } else if (rok && m0 == mk) {
+      fcol[par][r] = own_col;
     }
-    if (rok && m0 == (kk & 15)) fcol[r] = own_col;
     __syncthreads();
-    const T inv = s_inv;
-    const T fr = rok ? fcol[r] : (T)0;
+    if (!rok || r == kk) continue;
+    const T fr = fcol[par][r];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int m = m0 + 16 * q;
-      if (!rok || m >= n) continue;
-      const T pm = m == kk ? inv : prow[m] * inv;
-      if (r == kk)
-        a[q] = pm;
-      else if (m == kk)
-        a[q] = -fr * inv;
+      if (m >= n) continue;
+      if (m == kk)
+        a[q] = mulr(-fr, pinv[par]);
       else
-        a[q] -= fr * pm;
+        a[q] = fmad(-fr, prow[par][m], a[q]);
     }
-    __syncthreads();
   }
   if (rok) {
 #pragma unroll
@@ -377,7 +398,10 @@ __device__ __forceinline__ void cp_async_zfill(T* dst, const T* src, bool valid)
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"((int)sizeof(T)), "r"(n) : "memory");
 }
 
-// Stage the window.  LOAD_X: read x (else zero); PROLONG: add the coarse correction.
+// Stage the window.  LOAD_X: read x (else it starts from zero: the first half sweep writes
+// its colour without reading x, and each later one reads cells that the one before wrote;
+// the natural layout's sweeps leave out cells outside the domain, which are set to zero);
+// PROLONG: add the coarse correction.
 // The window is enumerated flat (division by compile-time constants only), so
 // every thread of the block has work in every pass.
 //   Natural layout: one cell per thread and pass, loaded through registers.
@@ -422,9 +446,6 @@ __device__ __forceinline__ void stage_window(const Level<T>& L, const Level<T>& 
         } else if (LOAD_X) {
           cp_async_zfill(xs + ea, L.x + ka, ina);
           cp_async_zfill(xs + eb, L.x + kb, inb);
-        } else {
-          xs[ea] = 0;
-          xs[eb] = 0;
         }
         if (inner) {
           cp_async(bs + ea, L.b + k);
@@ -471,8 +492,6 @@ __device__ __forceinline__ void stage_window(const Level<T>& L, const Level<T>& 
           xs[e] = x;
         } else if (LOAD_X) {
           cp_async_zfill(xs + e, L.x + kz, in);
-        } else {
-          xs[e] = 0;
         }
         if (inner) {
           cp_async(bs + e, L.b + k);
@@ -510,7 +529,7 @@ __device__ __forceinline__ void stage_window(const Level<T>& L, const Level<T>& 
         cy = L.cy[k];
         if (DG) dg = L.dg[k];
       }
-      xs[q] = x;
+      if (LOAD_X || !inner) xs[q] = x;  // from zero, every cell of an inner window that is read is written first
       bs[q] = b;
       is[q] = id;
       cxs[q] = cx;
@@ -527,10 +546,6 @@ __device__ __forceinline__ void stage_window(const Level<T>& L, const Level<T>& 
 // Written with the rounding intrinsics so that every kernel that smooths a level
 // (tiled or streaming) computes each value with the same operations, whatever
 // the compiler would contract.
-__device__ __forceinline__ float fmad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fmad(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mulr(double a, double b) { return __dmul_rn(a, b); }
 template <typename T>
 __device__ __forceinline__ T gs_update(T b, T cxl, T xl, T cxr, T xr, T cyb, T xb, T cyt, T xt, T idg) {
   return mulr(fmad(cyt, xt, fmad(cyb, xb, fmad(cxr, xr, fmad(cxl, xl, b)))), idg);
@@ -558,7 +573,9 @@ __device__ __forceinline__ T gs_residual(T b, T dg, T x, T cxl, T xl, T cxr, T x
 //   exact values, since half sweep k + 1 updates columns k+1 .. W-k-2 from
 //   neighbours in columns k .. W-k-1, and the tile with its one-cell ring lies
 //   in columns 2 NS .. W-2NS-1.
-template <typename T, int H, int R, int SH, int COLOR>
+//   FIRST: the pre-smoothing's first half sweep, where x is zero: the update is b / dg (the
+//   four products with zero add nothing), two reads instead of ten.
+template <typename T, int H, int R, int SH, int COLOR, bool FIRST>
 __device__ __forceinline__ void window_half(T* sm, int i0, int j0, int nI, int nJ) {
   using Wn = Win<T, H, SH>;
   constexpr int W = Wn::W, HH = Wn::HH, NA = Wn::NA;
@@ -573,6 +590,10 @@ __device__ __forceinline__ void window_half(T* sm, int i0, int j0, int nI, int n
     for (int u0 = 0; u0 < TOT; u0 += BXT * BYT) {
       const int e = E0 + u0 + tid;
       if (u0 + BXT * BYT > TOT && e >= E0 + TOT) continue;
+      if (FIRST) {
+        xp[e] = mulr(bp[e], ip[e]);
+        continue;
+      }
       const int o = (p + e / WH) & 1;
       xp[e] = gs_update(bp[e], cxp[e], xq[e - 1 + o], cxq[e + o], xq[e + o], cyp[e], xq[e - WH], cyq[e + WH], xq[e + WH], ip[e]);
     }
@@ -594,6 +615,10 @@ __device__ __forceinline__ void window_half(T* sm, int i0, int j0, int nI, int n
         if (gi < 0 || gi >= nI || gj < 0 || gj >= nJ) continue;
       }
       const int s = c + r * W;
+      if (FIRST) {
+        xs[s] = mulr(bs[s], is[s]);
+        continue;
+      }
       xs[s] = gs_update(bs[s], cxs[s], xs[s - 1], cxs[s + 1], xs[s + 1], cys[s], xs[s - W], cys[s + W], xs[s + W], is[s]);
     }
   }
@@ -656,12 +681,12 @@ __device__ __forceinline__ void publish_rz(Scalars* sc, double rz) {
 
 // Half sweeps R = R0..R1 (window shrunk by R), colour of the first = C0,
 // alternating, with a block barrier after each.
-template <typename T, int H, int R, int R1, int C0, int SH>
+template <typename T, int H, int R, int R1, int C0, int SH, bool FROM_ZERO>
 __device__ __forceinline__ void window_halves(T* sm, int i0, int j0, int nI, int nJ) {
   if constexpr (R <= R1) {
-    window_half<T, H, R, SH, (C0 + R - 1) & 1>(sm, i0, j0, nI, nJ);
+    window_half<T, H, R, SH, (C0 + R - 1) & 1, FROM_ZERO && R == 1>(sm, i0, j0, nI, nJ);
     __syncthreads();
-    window_halves<T, H, R + 1, R1, C0, SH>(sm, i0, j0, nI, nJ);
+    window_halves<T, H, R + 1, R1, C0, SH, FROM_ZERO>(sm, i0, j0, nI, nJ);
   }
 }
 
@@ -696,7 +721,7 @@ __global__ void __launch_bounds__(BXT* BYT) k_pre_smooth(Level<T> L, Level<T> C,
   const int i0 = blockIdx.x * Ts::X, j0 = blockIdx.y * Ts::Y;
   stage_window<T, H, false, false, false, SH>(L, C, sm, i0, j0);
   __syncthreads();
-  window_halves<T, H, 1, 2 * NS, 0, SH>(sm, i0, j0, L.nI, L.nJ);
+  window_halves<T, H, 1, 2 * NS, 0, SH, true>(sm, i0, j0, L.nI, L.nJ);
   const T *xs = sm, *bs = sm + NA, *is = sm + 2 * NA, *cxs = sm + 3 * NA, *cys = sm + 4 * NA;
   const int tid = threadIdx.x + threadIdx.y * BXT;
 #pragma unroll
@@ -741,7 +766,7 @@ __global__ void __launch_bounds__(BXT* BYT) k_post_smooth(Level<T> L, Level<T> C
   const int i0 = blockIdx.x * Ts::X, j0 = blockIdx.y * Ts::Y;
   stage_window<T, H, true, true, false, SH>(L, C, sm, i0, j0);
   __syncthreads();
-  window_halves<T, H, 1, 2 * NS, 1, SH>(sm, i0, j0, L.nI, L.nJ);
+  window_halves<T, H, 1, 2 * NS, 1, SH, false>(sm, i0, j0, L.nI, L.nJ);
   const T *xs = sm, *bs = sm + NA;
   Acc<T> acc;
   const int tid = threadIdx.x + threadIdx.y * BXT;
