@@ -235,22 +235,24 @@ __device__ __forceinline__ double pivot_inverse(double x) {
 
 // Dense inverse of the coarsest operator (n <= 64), Gauss-Jordan without
 // pivoting (the operator is SPD), computed in the hierarchy's precision.  One
-// block of 1024 threads, thread t owning row t/16 and columns t%16 + 16q
-// (q = 0..3) in registers.  A pivot step: the pivot row's half warp takes the pivot by
-// shuffle, forms its reciprocal and publishes the scaled row, the pivot column's owners
-// publish the column; one barrier (the two are double-buffered); everyone updates.
+// block of 256 threads, thread t owning row t/4 and columns 16 (t%4) .. + 15 in
+// registers (the pivot loop unrolled by 16, so that a register holds each step's column).
+// A pivot step: the pivot row's four threads take the pivot by shuffle, form its
+// reciprocal and publish the scaled row, the pivot column's owners publish the column; one
+// barrier (the two are double-buffered); everyone updates.
 // FP64 is bound by one SM's FP64 pipe, 64 x 64 FMAs a step (2048 cycles): the row is
-// scaled by its owners, once, and the reciprocal runs on the integer pipes (191 us with
-// every thread scaling and two barriers a step; FP32 39 us).
+// scaled by its owners, once, and the reciprocal runs on the integer pipes.
+constexpr int kInvThreads = 4 * kCoarseMax;
 template <typename T>
-__global__ void __launch_bounds__(1024) k_dense_inverse(Level<T> C, double* __restrict__ ainv) {
+__global__ void __launch_bounds__(kInvThreads) k_dense_inverse(Level<T> C, double* __restrict__ ainv) {
   static_assert(kCoarseMax == 64, "register blocking assumes 64 x 64");
-  __shared__ T prow[2][kCoarseMax], fcol[2][kCoarseMax], pinv[2];
+  __shared__ __align__(16) T prow[2][kCoarseMax];
+  __shared__ T fcol[2][kCoarseMax], pinv[2];
   const int n = C.nI * C.nJ;
   if (n > kCoarseMax) return;  // prevented on the host (alloc_hierarchy)
-  const int r = threadIdx.x >> 4, m0 = threadIdx.x & 15;
+  const int r = threadIdx.x >> 2, g = threadIdx.x & 3;
   const bool rok = r < n;
-  T a[4];
+  T a[16];
   {
     int ri = 0, rj = 0;
     size_t k = 0;
@@ -260,8 +262,8 @@ __global__ void __launch_bounds__(1024) k_dense_inverse(Level<T> C, double* __re
       k = (size_t)(ri + 1) + (size_t)(rj + 1) * C.ld;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int m = m0 + 16 * q;
+    for (int q = 0; q < 16; ++q) {
+      const int m = 16 * g + q;
       T v = 0;
       if (rok && m < n) {
         if (m == r) v = C.dg[k];
@@ -273,40 +275,35 @@ __global__ void __launch_bounds__(1024) k_dense_inverse(Level<T> C, double* __re
       a[q] = v;
     }
   }
-  for (int kk = 0; kk < n; ++kk) {
-    const int qk = kk >> 4, mk = kk & 15, par = kk & 1;
-    const T own_col = qk == 0 ? a[0] : qk == 1 ? a[1] : qk == 2 ? a[2] : a[3];
-    if (r == kk) {  // sixteen threads of one warp
-      const unsigned half = 0xffffu << (threadIdx.x & 16);
-      const T inv = pivot_inverse(__shfl_sync(half, own_col, mk, 16));
+  for (int gk = 0; 16 * gk < n; ++gk) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int m = m0 + 16 * q;
-        const T pm = m == kk ? inv : mulr(a[q], inv);
-        if (m < n) a[q] = pm;
-        prow[par][m] = pm;
+    for (int qk = 0; qk < 16; ++qk) {
+      const int kk = 16 * gk + qk, par = qk & 1;
+      if (kk >= n) break;
+      if (r == kk) {  // four threads of one warp
+        const unsigned quad = 0xfu << (threadIdx.x & 28);
+        const T inv = pivot_inverse(__shfl_sync(quad, a[qk], gk, 4));
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          a[q] = q == qk && g == gk ? inv : mulr(a[q], inv);
+          prow[par][16 * g + q] = a[q];
+        }
+        if (g == 0) pinv[par] = inv;
+      } else if (g == gk) {
+        fcol[par][r] = a[qk];
       }
-      if (m0 == 0) pinv[par] = inv;
-    } else if (rok && m0 == mk) {
-      fcol[par][r] = own_col;
-    }
-    __syncthreads();
-    if (!rok || r == kk) continue;
-    const T fr = fcol[par][r];
+      __syncthreads();
+      if (rok && r != kk) {
+        const T fr = -fcol[par][r];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int m = m0 + 16 * q;
-      if (m >= n) continue;
-      if (m == kk)
-        a[q] = mulr(-fr, pinv[par]);
-      else
-        a[q] = fmad(-fr, prow[par][m], a[q]);
+        for (int q = 0; q < 16; ++q) a[q] = q == qk && g == gk ? mulr(fr, pinv[par]) : fmad(fr, prow[par][16 * g + q], a[q]);
+      }
     }
   }
   if (rok) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int m = m0 + 16 * q;
+    for (int q = 0; q < 16; ++q) {
+      const int m = 16 * g + q;
       if (m < n) ainv[(size_t)r * n + m] = (double)a[q];
     }
   }
@@ -1518,7 +1515,7 @@ void build_coarse(cudaStream_t s, Hierarchy<T>& H, double* ainv) {
     k_coarsen<T><<<grid_ij(H.L[l].nI, H.L[l].nJ), kThreads, 0, s>>>(H.L[l - 1], H.L[l]);
     GB_LAUNCHED(1);
   }
-  k_dense_inverse<T><<<1, 1024, 0, s>>>(H.L[H.nlev - 1], ainv);
+  k_dense_inverse<T><<<1, kInvThreads, 0, s>>>(H.L[H.nlev - 1], ainv);
   GB_LAUNCHED(1);
 }
 
