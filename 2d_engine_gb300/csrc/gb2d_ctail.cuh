@@ -147,8 +147,8 @@ __device__ __forceinline__ void ct_load(const CtLevel<T>& L, const CtWin& w, con
       f = ct_coef(L, w, u);
       if (L.b < 0) {
         const int q = (w.w0 + lr + 1) * L.ld + 2 * m + 1;
-        g.b[0][k] = L.bg[q + o];
-        g.b[1][k] = L.bg[q + 1 - o];
+        g.b[0][k] = __ldcg(L.bg + q + o);  // through L2: the CG kernel's other CTAs write it
+        g.b[1][k] = __ldcg(L.bg + q + 1 - o);
       } else {
         g.b[0][k] = sm[L.b + u];
         g.b[1][k] = sm[L.b + L.plane + u];
@@ -414,9 +414,9 @@ __device__ __forceinline__ void ct_hand_down(const CtArgs<T>& a, int l, int c, i
 
 // r.z when the top level is the finest: a block sum over 1024 strided partials (two per
 // thread) in block_sum's order; a warp's sum over no elements is the zero it would add up.
+// Valid in the first warp's lane 0.
 template <typename T>
-__device__ __forceinline__ void ct_publish(const CtArgs<T>& a, int c, int P, const T* sm, double* rz_part) {
-  cgx::cluster_group cl = cgx::this_cluster();
+__device__ __forceinline__ double ct_rz(const CtArgs<T>& a, int c, const T* sm) {
   const CtLevel<T>& L = a.L[0];
   const CtWin w = ct_win(a, 0, c);
   double* scratch = reduce_scratch();
@@ -427,7 +427,7 @@ __device__ __forceinline__ void ct_publish(const CtArgs<T>& a, int c, int P, con
     if ((tid & ~31) + h * kCtThreads < n) {
       for (int u = tid + h * kCtThreads; u < n; u += 2 * kCtThreads) {
         const int lr = u / L.nI, i = u - lr * L.nI, J = w.J0 + lr;
-        const T bv = L.bg[(J + 1) * L.ld + i + 1];
+        const T bv = __ldcg(L.bg + (J + 1) * L.ld + i + 1);
         const T xv = sm[L.x + (((i + J) & 1) ? L.xplane : 0) + (J - w.w0 + 1) * (L.pairs + 2) + (i >> 1) + 1];
         acc = __fma_rn((double)bv, (double)xv, acc);
       }
@@ -436,43 +436,13 @@ __device__ __forceinline__ void ct_publish(const CtArgs<T>& a, int c, int P, con
     if ((tid & 31) == 0) scratch[(tid >> 5) + h * (kCtThreads / 32)] = acc;
   }
   __syncthreads();
-  if (tid < 32) {
-    const double v = warp_sum(scratch[tid]);
-    if (tid == 0) *cl.map_shared_rank(&rz_part[c], 0) = v;
-  }
-  cl.sync();
-  if (c == 0 && tid == 0) {
-    double rz = 0.0;
-    for (int o = 0; o < P; ++o) rz += rz_part[o];
-    publish_rz(a.sc, rz);
-  }
+  return tid < 32 ? warp_sum(scratch[tid]) : 0.0;
 }
 
-// The whole tail, up to K pairs per thread.
-// Against a cluster of 1024-thread CTAs that staged whole levels in shared memory (ten
-// reads and a cluster barrier per half sweep, about 50 barriers): the mixed projection to
-// 1e-8 from host arrays 0.88 -> 0.66 ms at 64^2 and 2.77 -> 2.57 ms at 1024^2, about 13 us
-// of an iteration's 118; FP64 tails are bound by the FP64 pipe and gain little.  Also
-// measured, not kept: the coefficients packed by pairs and staged in shared memory while
-// the previous kernel runs, each level's pairs held in registers from the way down to the
-// way up (124 registers): 2% faster at 64^2 but 5% slower at 1024^2, where the wider CTAs
-// find room only when the previous kernel's blocks have left; 64 and 80 registers a thread
-// are no faster than the 96 that it takes.
-template <typename T, int K>
-__global__ void __launch_bounds__(kCtThreads, 1) k_ctail(const __grid_constant__ CtArgs<T> a, const double* __restrict__ ainv, int nu,
-                                                         const int* __restrict__ done) {
-  cgx::cluster_group cl = cgx::this_cluster();
-  const int P = (int)cl.num_blocks(), c = (int)cl.block_rank(), tid = (int)threadIdx.x;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sm = reinterpret_cast<T*>(smem_raw);
-  __shared__ double rz_part[kClusterMax];
-  const int nl = a.nlev, nd = a.ndist;
-  // Before the previous kernel has finished: what it does not write.
-  const CtDense<T> dense = ct_dense_load(a.L[nl - 1], ainv);
-  for (int u = tid; u < a.zero_n; u += kCtThreads) sm[u] = (T)0;
-  cl.sync();  // every CTA's planes are clear before any remote write
-  pdl_enter();
-  if (*done) return;  // uniform over the cluster: no CTA writes remotely or reaches a cluster barrier
+// One V-cycle from the top level's right-hand side to its x, both in global memory.
+template <int K, typename T>
+__device__ __forceinline__ void ct_vcycle(const CtArgs<T>& a, int c, int P, const CtDense<T>& dense, T* sm, int nu) {
+  const int nl = a.nlev, nd = a.ndist, tid = (int)threadIdx.x;
   for (int l = 0; l < nl; ++l) {
     if (l >= nd) ct_restrict_local(a, l, sm);
     if (l == nl - 1) break;
@@ -497,5 +467,41 @@ __global__ void __launch_bounds__(kCtThreads, 1) k_ctail(const __grid_constant__
       ct_up<1, true>(a, l, c, sm, nu);
     __syncthreads();
   }
-  if (a.sc) ct_publish(a, c, P, sm, rz_part);
+}
+
+// The whole tail, up to K pairs per thread.
+// Against a cluster of 1024-thread CTAs that staged whole levels in shared memory (ten
+// reads and a cluster barrier per half sweep, about 50 barriers): the mixed projection to
+// 1e-8 from host arrays 0.88 -> 0.66 ms at 64^2 and 2.77 -> 2.57 ms at 1024^2, about 13 us
+// of an iteration's 118; FP64 tails are bound by the FP64 pipe and gain little.  Also
+// measured, not kept: the coefficients packed by pairs and staged in shared memory while
+// the previous kernel runs, each level's pairs held in registers from the way down to the
+// way up (124 registers): 2% faster at 64^2 but 5% slower at 1024^2, where the wider CTAs
+// find room only when the previous kernel's blocks have left; 64 and 80 registers a thread
+// are no faster than the 96 that it takes.
+template <typename T, int K>
+__global__ void __launch_bounds__(kCtThreads, 1) k_ctail(const __grid_constant__ CtArgs<T> a, const double* __restrict__ ainv, int nu,
+                                                         const int* __restrict__ done) {
+  cgx::cluster_group cl = cgx::this_cluster();
+  const int P = (int)cl.num_blocks(), c = (int)cl.block_rank(), tid = (int)threadIdx.x;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* sm = reinterpret_cast<T*>(smem_raw);
+  __shared__ double rz_part[kClusterMax];
+  // Before the previous kernel has finished: what it does not write.
+  const CtDense<T> dense = ct_dense_load(a.L[a.nlev - 1], ainv);
+  for (int u = tid; u < a.zero_n; u += kCtThreads) sm[u] = (T)0;
+  cl.sync();  // every CTA's planes are clear before any remote write
+  pdl_enter();
+  if (*done) return;  // uniform over the cluster: no CTA writes remotely or reaches a cluster barrier
+  ct_vcycle<K>(a, c, P, dense, sm, nu);
+  if (a.sc) {
+    const double v = ct_rz(a, c, sm);
+    if (tid == 0) *cl.map_shared_rank(&rz_part[c], 0) = v;
+    cl.sync();
+    if (c == 0 && tid == 0) {
+      double rz = 0.0;
+      for (int o = 0; o < P; ++o) rz += rz_part[o];
+      publish_rz(a.sc, rz);
+    }
+  }
 }

@@ -1016,10 +1016,20 @@ __global__ void k_direction(Level<double> L, const TZ* __restrict__ z, double* _
       st2(p, k, widen(zv.x), widen(zv.y));
     } else {
       const double2 pv = ld2(p, k);
-      st2(p, k, widen(zv.x) + bt * pv.x, widen(zv.y) + bt * pv.y);
+      st2(p, k, __fma_rn(bt, pv.x, widen(zv.x)), __fma_rn(bt, pv.y, widen(zv.y)));
     }
   }
 }
+
+// One row of A p and the two vector updates, every rounding stated (the cluster CG below
+// performs the same operations).
+__device__ __forceinline__ double ap_row(double dg, double pc, double cxl, double pl, double cxr, double pr, double cyb, double pb,
+                                         double cyt, double pt) {
+  return __fma_rn(-cyt, pt, __fma_rn(-cyb, pb, __fma_rn(-cxr, pr, __fma_rn(dg, pc, -__dmul_rn(cxl, pl)))));
+}
+// A thread's partial of ||r||^2: r r added to acc.
+__device__ __forceinline__ void add_square(Acc<float>& acc, float f) { acc.add(f * f); }
+__device__ __forceinline__ void add_square(Acc<double>& acc, double r) { acc.s = __fma_rn(r, r, acc.s); }
 
 // Ap = A p (reference entries) and p.Ap; the last block publishes
 // alpha = rz_new / p.Ap and rz_cur = rz_new.  With an even row length two
@@ -1040,18 +1050,18 @@ __global__ void k_apply_pap(Level<double> L, const double* __restrict__ p, doubl
       const double2 pc = ld2(p, k), pb = ld2(p, k - ld), pt = ld2(p, k + ld);
       const double2 dg = ld2(L.dg, k), cx = ld2(L.cx, k), cy = ld2(L.cy, k), cyt = ld2(L.cy, k + ld);
       const double pl = p[k - 1], pr = p[k + 2], cx2 = L.cx[k + 2];
-      const double y0 = dg.x * pc.x - cx.x * pl - cx.y * pc.y - cy.x * pb.x - cyt.x * pt.x;
-      const double y1 = dg.y * pc.y - cx.y * pc.x - cx2 * pr - cy.y * pb.y - cyt.y * pt.y;
+      const double y0 = ap_row(dg.x, pc.x, cx.x, pl, cx.y, pc.y, cy.x, pb.x, cyt.x, pt.x);
+      const double y1 = ap_row(dg.y, pc.y, cx.y, pc.x, cx2, pr, cy.y, pb.y, cyt.y, pt.y);
       st2(ap, k, y0, y1);
-      acc += pc.x * y0;
-      acc += pc.y * y1;
+      acc = __fma_rn(pc.x, y0, acc);
+      acc = __fma_rn(pc.y, y1, acc);
     }
   } else {
     GB_FLAT_FOR(L, k) {
       const double pc = p[k];
-      double y = L.dg[k] * pc - L.cx[k] * p[k - 1] - L.cx[k + 1] * p[k + 1] - L.cy[k] * p[k - L.ld] - L.cy[k + L.ld] * p[k + L.ld];
+      const double y = ap_row(L.dg[k], pc, L.cx[k], p[k - 1], L.cx[k + 1], p[k + 1], L.cy[k], p[k - L.ld], L.cy[k + L.ld], p[k + L.ld]);
       ap[k] = y;
-      acc += pc * y;
+      acc = __fma_rn(pc, y, acc);
     }
   }
   double pap, blk;
@@ -1082,17 +1092,17 @@ __global__ void k_update(Level<double> L, double* __restrict__ x, double* __rest
   Acc<T> acc;
   GB_FLAT_PAIRS(L, k) {
     const double2 pv = ld2(p, k), av = ld2(ap, k), xv = ld2(x, k), rv = ld2(r, k);
-    st2(x, k, xv.x + al * pv.x, xv.y + al * pv.y);
-    const double r0 = rv.x - al * av.x, r1 = rv.y - al * av.y;
+    st2(x, k, __fma_rn(al, pv.x, xv.x), __fma_rn(al, pv.y, xv.y));
+    const double r0 = __fma_rn(-al, av.x, rv.x), r1 = __fma_rn(-al, av.y, rv.y);
     st2(r, k, r0, r1);
     if constexpr (sizeof(T) == 4) {
       const float f0 = narrow(r0), f1 = narrow(r1);
       st2(rT, k, f0, f1);
-      acc.add(f0 * f0);
-      acc.add(f1 * f1);
+      add_square(acc, f0);
+      add_square(acc, f1);
     } else {
-      acc.add(r0 * r0);
-      acc.add(r1 * r1);
+      add_square(acc, r0);
+      add_square(acc, r1);
     }
   }
   double rr;
@@ -1156,8 +1166,8 @@ __global__ void k_loop_cond(cudaGraphConditionalHandle h, Scalars* sc, const int
 // done flag from the true residual and ||b||^2 in the frame scalars fs (g_rr, g_bb), as
 // solver_solve's host loop decides them (a non-finite norm marks fs->flag bit 4 and ends
 // the solve), the pass's iteration cap (what the solve's earlier passes left of max_it),
-// and the WHILE node's condition.  first: the solve's first pass.
-__global__ void k_begin_device(cudaGraphConditionalHandle h, Scalars* sc, int* done, Scalars* fs, double tol2, int max_it, int first) {
+// and (loop) the WHILE node's condition.  first: the solve's first pass.
+__global__ void k_begin_device(cudaGraphConditionalHandle h, int loop, Scalars* sc, int* done, Scalars* fs, double tol2, int max_it, int first) {
   const double rr = fs->g_rr, bb = fs->g_bb;
   if (first) fs->iters = 0;  // the frame scalars' iters count this solve's iterations
   const double thr2 = tol2 * bb;
@@ -1175,7 +1185,7 @@ __global__ void k_begin_device(cudaGraphConditionalHandle h, Scalars* sc, int* d
   sc->rz_cur = 1.0;
   sc->iters = 0;
   sc->max_it = cap;
-  cudaGraphSetConditional(h, d ? 0u : 1u);
+  if (loop) cudaGraphSetConditional(h, d ? 0u : 1u);
 }
 
 // End of a pass (after the true residual is in fs->g_rr / g_bb): the pass's iterations join
@@ -1191,6 +1201,237 @@ __global__ void k_end_device(const Scalars* sc, Scalars* fs, int last) {
   const double rel2 = bb > 0 ? rr / bb : 0.0;
   if (rel2 > fs->g_rel2_max) fs->g_rel2_max = rel2;
   if (!(rr <= sc->thr2) && bb != 0.0) fs->g_capped = 1;
+}
+
+// ---- the whole CG of a small grid in one cluster -----------------------------------
+//
+// Where the cluster tail holds the finest level (at most 128^2 cells), a CG iteration was
+// four launches of a few microseconds each around vectors of some 100 KB: launch and
+// reduction latency (64^2: 28 us of kernels and 6 of gaps). This kernel runs the whole
+// iteration loop in the tail's cluster: vectors in global memory (L2), five cluster
+// barriers an iteration (residual; the V-cycle's two and r.z; direction; p.Ap), no host.
+// Every number equals the launched kernels': their blocks of 256 threads become the
+// halves of a CTA, with the same elements, the same sums and the same order of partials.
+// Vectors that another CTA wrote are read through L2 (__ldcg). Every CTA computes the same
+// scalars from the same partials, so that all take the same branches; at most max_it
+// iterations.  Measured: the mixed projection at 64^2 0.60 -> 0.49 ms, an iteration 34 -> 19
+// us (the V-cycle 9 of them); a bubble frame at 128^2 (FP64) 3.70 -> 3.65 ms, whose
+// V-cycles are bound by 16 SMs' FP64 pipes.
+template <typename T>
+struct CgArgs {
+  CtArgs<T> a;
+  Level<double> L;
+  double *x, *r, *p, *ap;
+  T* rT;
+  const double* ainv;
+  double *part_rr, *part_pap;
+  int G, nu;      // virtual blocks
+  Scalars* sc;    // thr2, max_it in; iters, rr, flag out
+  int* done;      // nonzero: nothing to do
+  double* host;   // [0] ||r||^2, [1] iterations
+};
+
+// block_sum over each half of the block (256 threads); valid in the half's first warp.  A
+// warp of zeros (active false throughout it) adds the zero that it would sum up, and the
+// second stage's steps that only add zeros to the eight warps' sums drop out.
+__device__ __forceinline__ double half_sum(double v, bool active, double* scratch) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, base = w & ~7;
+  if (__any_sync(0xffffffffu, active)) v = warp_sum(v);
+  __syncthreads();
+  if (lane == 0) scratch[w] = v;
+  __syncthreads();
+  if (w != base) return 0.0;
+  double x = lane < 8 ? scratch[base + lane] : 0.0;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  return x;
+}
+__device__ __forceinline__ double half_sum_df(DF v, bool active, double* scratch) {
+  float* shi = reinterpret_cast<float*>(scratch);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, base = w & ~7;
+  if (__any_sync(0xffffffffu, active)) v = warp_sum_df(v);
+  __syncthreads();
+  if (lane == 0) {
+    shi[w] = v.hi;
+    shi[16 + w] = v.lo;
+  }
+  __syncthreads();
+  if (w != base) return 0.0;
+  DF x = lane < 8 ? DF{shi[base + lane], shi[16 + base + lane]} : DF{0.f, 0.f};
+  x = warp_sum_df(x);
+  return widen(x.hi) + widen(x.lo);
+}
+// sum_partials by a block of 256 threads; valid in the first warp.
+__device__ __forceinline__ double cluster_total(const double* part, int G, double* scratch) {
+  const int t = (int)threadIdx.x;
+  double v = 0.0;
+  if (G <= 32) {  // one warp's sum, to which the other warps' zeros add nothing
+    if (t < G) v = __ldcg(part + t);
+    return t < 32 ? warp_sum(v) : 0.0;
+  }
+  if (t < kThreads)
+    for (int k = t; k < G; k += kThreads) v += __ldcg(part + k);
+  return half_sum(v, t < G && t < kThreads, scratch);
+}
+
+template <typename T, int K>
+__global__ void __launch_bounds__(kCtThreads, 1) k_cg_cluster(const __grid_constant__ CgArgs<T> g) {
+  static_assert(kCtThreads == 2 * kThreads, "two virtual blocks per CTA");
+  cgx::cluster_group cl = cgx::this_cluster();
+  const int P = (int)cl.num_blocks(), c = (int)cl.block_rank(), tid = (int)threadIdx.x;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* sm = reinterpret_cast<T*>(smem_raw);
+  __shared__ double rz_part[kClusterMax], scratch[16], s_rz, s_scalar;
+  const CtArgs<T>& a = g.a;
+  const Level<double>& L = g.L;
+  if (*g.done) return;  // uniform over the cluster
+  const CtDense<T> dense = ct_dense_load(a.L[a.nlev - 1], g.ainv);
+  for (int u = tid; u < a.zero_n; u += kCtThreads) sm[u] = (T)0;
+  const double thr2 = g.sc->thr2;
+  const int max_it = g.sc->max_it, G = g.G;
+  const size_t ld = L.ld, end = ld * (L.nJ + 1), pair_end = (end + 1) & ~(size_t)1;
+  const int vt = tid & (kThreads - 1), vb0 = c + P * (tid / kThreads), rounds = (G + 2 * P - 1) / (2 * P);
+  cl.sync();
+  double rz_cur = 1.0, alpha = 0.0, rr = 0.0;
+  int it = 0;
+  bool bad = false, converged = false;
+  for (;;) {
+    if (it > 0) {
+      // x += alpha p, r -= alpha Ap, ||r||^2 (k_update)
+      for (int n = 0; n < rounds; ++n) {
+        const int vb = vb0 + 2 * P * n;
+        Acc<T> acc;
+        bool any = false;
+        if (vb < G)
+          for (size_t k = (ld & ~(size_t)1) + 2 * ((size_t)vb * kThreads + vt); k < pair_end; k += 2 * (size_t)G * kThreads) {
+            any = true;
+            const double2 pv = __ldcg(reinterpret_cast<const double2*>(g.p + k)), av = __ldcg(reinterpret_cast<const double2*>(g.ap + k));
+            const double2 xv = ld2(g.x, k), rv = ld2(g.r, k);
+            st2(g.x, k, __fma_rn(alpha, pv.x, xv.x), __fma_rn(alpha, pv.y, xv.y));
+            const double r0 = __fma_rn(-alpha, av.x, rv.x), r1 = __fma_rn(-alpha, av.y, rv.y);
+            st2(g.r, k, r0, r1);
+            if constexpr (sizeof(T) == 4) {
+              const float f0 = narrow(r0), f1 = narrow(r1);
+              st2(g.rT, k, f0, f1);
+              add_square(acc, f0);
+              add_square(acc, f1);
+            } else {
+              add_square(acc, r0);
+              add_square(acc, r1);
+            }
+          }
+        double blk;
+        if constexpr (sizeof(T) == 4)
+          blk = half_sum_df(DF{acc.s, -acc.c}, any, scratch);
+        else
+          blk = half_sum(acc.s, any, scratch);
+        if (vt == 0 && vb < G) g.part_rr[vb] = blk;
+      }
+      cl.sync();
+      {
+        const double total = cluster_total(g.part_rr, G, scratch);
+        if (tid == 0) s_scalar = total;
+        __syncthreads();
+        rr = s_scalar;
+      }
+      if (!(rr > thr2)) {
+        converged = true;
+        bad = !isfinite(rr);
+        break;
+      }
+      if (it >= max_it) break;
+    }
+    // z = M r and r.z
+    ct_vcycle<K>(a, c, P, dense, sm, g.nu);
+    const double part = ct_rz(a, c, sm);
+    if (tid < 32) {
+      const double v = __shfl_sync(0xffffffffu, part, 0);
+      if (tid < P) *cl.map_shared_rank(&rz_part[c], tid) = v;
+    }
+    cl.sync();
+    if (tid == 0) {
+      double rz = 0.0;
+      for (int o = 0; o < P; ++o) rz += rz_part[o];
+      s_rz = rz;
+      s_scalar = it == 0 ? 0.0 : rz / rz_cur;  // in one thread: 512 would hold up the FP64 pipe
+    }
+    __syncthreads();
+    const double rz = s_rz, bt = s_scalar;
+    // p = z + beta p (k_direction)
+    for (int n = 0; n < rounds; ++n) {
+      const int vb = vb0 + 2 * P * n;
+      if (vb >= G) break;
+      for (size_t k = (ld & ~(size_t)1) + 2 * ((size_t)vb * kThreads + vt); k < pair_end; k += 2 * (size_t)G * kThreads) {
+        const T* z = a.L[0].xg + k;
+        const double z0 = widen(__ldcg(z)), z1 = widen(__ldcg(z + 1));
+        if (it == 0) {
+          st2(g.p, k, z0, z1);
+        } else {
+          const double2 pv = ld2(g.p, k);
+          st2(g.p, k, __fma_rn(bt, pv.x, z0), __fma_rn(bt, pv.y, z1));
+        }
+      }
+    }
+    cl.sync();
+    // Ap, p.Ap and alpha (k_apply_pap)
+    for (int n = 0; n < rounds; ++n) {
+      const int vb = vb0 + 2 * P * n;
+      double acc = 0.0;
+      bool any = false;
+      if (vb < G) {
+        if ((ld & 1) == 0) {
+          for (size_t k = (ld & ~(size_t)1) + 2 * ((size_t)vb * kThreads + vt); k < pair_end; k += 2 * (size_t)G * kThreads) {
+            any = true;
+            auto at = [&](size_t e) { return __ldcg(reinterpret_cast<const double2*>(g.p + e)); };
+            const double2 pc = at(k), pb = at(k - ld), pt = at(k + ld);
+            const double2 dg = ld2(L.dg, k), cx = ld2(L.cx, k), cy = ld2(L.cy, k), cyt = ld2(L.cy, k + ld);
+            const double pl = __ldcg(g.p + k - 1), pr = __ldcg(g.p + k + 2), cx2 = L.cx[k + 2];
+            const double y0 = ap_row(dg.x, pc.x, cx.x, pl, cx.y, pc.y, cy.x, pb.x, cyt.x, pt.x);
+            const double y1 = ap_row(dg.y, pc.y, cx.y, pc.x, cx2, pr, cy.y, pb.y, cyt.y, pt.y);
+            st2(g.ap, k, y0, y1);
+            acc = __fma_rn(pc.x, y0, acc);
+            acc = __fma_rn(pc.y, y1, acc);
+          }
+        } else {
+          for (size_t k = ld + (size_t)vb * kThreads + vt; k < end; k += (size_t)G * kThreads) {
+            any = true;
+            const double* p = g.p + k;
+            const double pc = __ldcg(p);
+            const double y = ap_row(L.dg[k], pc, L.cx[k], __ldcg(p - 1), L.cx[k + 1], __ldcg(p + 1), L.cy[k], __ldcg(p - ld), L.cy[k + ld],
+                                    __ldcg(p + ld));
+            g.ap[k] = y;
+            acc = __fma_rn(pc, y, acc);
+          }
+        }
+      }
+      double blk;
+      if constexpr (sizeof(T) == 4) {
+        const float hi = narrow(acc);
+        blk = half_sum_df(DF{hi, narrow(acc - widen(hi))}, any, scratch);
+      } else {
+        blk = half_sum(acc, any, scratch);
+      }
+      if (vt == 0 && vb < G) g.part_pap[vb] = blk;
+    }
+    cl.sync();
+    {
+      const double total = cluster_total(g.part_pap, G, scratch);
+      if (tid == 0) s_scalar = rz / total;
+      __syncthreads();
+      alpha = s_scalar;
+    }
+    rz_cur = rz;
+    ++it;
+    if (it > max_it) break;
+  }
+  if (c == 0 && tid == 0) {
+    g.sc->iters = it;
+    g.sc->rr = rr;
+    if (converged) *g.done = 1;
+    if (bad) g.sc->flag |= 1;
+    g.host[0] = rr;
+    g.host[1] = (double)it;
+  }
 }
 
 }  // namespace
@@ -1377,15 +1618,29 @@ bool plan_ctail(Hierarchy<T>& H, int P) {
     CtArgs<T> a;
     memset(&a, 0, sizeof a);
     a.nlev = nl - top;
-    a.ndist = lb - top + 1;
-    for (int c = 0; c <= P; ++c) a.J0[a.ndist - 1][c] = (short)((long)c * H.L[lb].nJ / P);
-    for (int l = a.ndist - 2; l >= 0; --l) {
-      for (int c = 0; c < P; ++c) a.J0[l][c] = (short)(2 * a.J0[l + 1][c]);
-      a.J0[l][P] = (short)H.L[top + l].nJ;
-    }
-    bool ok = true;
+    int stripe[kCtMaxLevels];  // rows of each level's widest stripe
+    // Stripes of levels 0 .. ndist - 1: the bottom one's rows in equal parts, nested above.
+    auto distribute = [&](int ndist) {
+      a.ndist = ndist;
+      bool ok = true;
+      for (int c = 0; c <= P; ++c) a.J0[ndist - 1][c] = (short)((long)c * H.L[top + ndist - 1].nJ / P);
+      for (int l = ndist - 2; l >= 0; --l) {
+        for (int c = 0; c < P; ++c) a.J0[l][c] = (short)(2 * a.J0[l + 1][c]);
+        a.J0[l][P] = (short)H.L[top + l].nJ;
+      }
+      for (int l = 0; l < a.nlev; ++l) {
+        stripe[l] = l < ndist ? 0 : H.L[top + l].nJ;
+        for (int c = 0; l < ndist && c < P; ++c) {
+          const int r = a.J0[l][c + 1] - a.J0[l][c];
+          if (r < 1) ok = false;
+          stripe[l] = r > stripe[l] ? r : stripe[l];
+        }
+      }
+      return ok;
+    };
+    const int nd = lb - top + 1;
+    bool ok = distribute(nd);
     size_t cells = 0;  // six padded stripes per level must fit in one CTA's shared memory
-    int stripe[kCtMaxLevels];
     for (int l = 0; l < a.nlev; ++l) {
       const Level<T>& L = H.L[top + l];
       CtLevel<T>& C = a.L[l];
@@ -1400,21 +1655,25 @@ bool plan_ctail(Hierarchy<T>& H, int P) {
       C.dg = L.dg;
       C.bg = L.b;
       C.xg = L.x;
-      stripe[l] = L.nJ;
-      if (l < a.ndist) {
-        stripe[l] = 0;
-        for (int c = 0; c < P; ++c) {
-          const int r = a.J0[l][c + 1] - a.J0[l][c];
-          if (r < 1) ok = false;
-          stripe[l] = r > stripe[l] ? r : stripe[l];
-        }
-      }
-      cells += (l == a.ndist - 1 ? 7 : 6) * (size_t)(stripe[l] + 2) * L.ld;
+      cells += (l == nd - 1 ? 7 : 6) * (size_t)(stripe[l] + 2) * L.ld;
     }
     const size_t nc = (size_t)H.L[nl - 1].nI * H.L[nl - 1].nJ;
     if (!ok || (cells + nc * nc + nc) * sizeof(T) > kCtSmemCap) continue;
-    for (int nu = 1; nu <= 3 && ok; ++nu) ok = layout_ctail(a, stripe, nu, &H.ct[nu - 1], &H.ct_smem[nu - 1]);
-    if (!ok) continue;
+    // One level more, of at least two rows per CTA, where running it in every CTA takes
+    // more than one pair per thread, or is FP64 (each CTA's FP64 pipe is the bound): 16
+    // batched bubbles 9.1 -> 8.6 ms, the FP64 frame at 128^2 3.65 -> 3.50 ms; in FP32 with
+    // one pair per thread its cluster barrier costs more (64^2 projection 0.49 -> 0.50 ms).
+    // Not where that moves the finest level's stripes, whose sums of r.z they order.
+    short J0top[kClusterMax + 1];
+    memcpy(J0top, a.J0[0], sizeof J0top);
+    bool deeper = lb + 1 < nl - 1 && H.L[lb + 1].nJ >= 2 * P && (sizeof(T) == 8 || a.L[nd].pairs * a.L[nd].nJ > kCtThreads) &&
+                  distribute(nd + 1) && (top > 0 || memcmp(J0top, a.J0[0], (size_t)(P + 1) * sizeof(short)) == 0);
+    for (int nu = 1; nu <= 3 && deeper; ++nu) deeper = layout_ctail(a, stripe, nu, &H.ct[nu - 1], &H.ct_smem[nu - 1]);
+    if (!deeper) {
+      distribute(nd);
+      for (int nu = 1; nu <= 3 && ok; ++nu) ok = layout_ctail(a, stripe, nu, &H.ct[nu - 1], &H.ct_smem[nu - 1]);
+      if (!ok) continue;
+    }
     H.ctail = top;
     H.ct_P = P;
     return true;
@@ -1431,8 +1690,10 @@ int ctail_cluster_size() {
   static int cached = -1;
   if (cached >= 0) return cached;
   cached = 0;
-  const void* kernels[4] = {(const void*)k_ctail<float, kCtPairs>, (const void*)k_ctail<double, kCtPairs>,
-                            (const void*)k_ctail<float, kCtPairsMax>, (const void*)k_ctail<double, kCtPairsMax>};
+  const void* kernels[8] = {(const void*)k_ctail<float, kCtPairs>,         (const void*)k_ctail<double, kCtPairs>,
+                            (const void*)k_ctail<float, kCtPairsMax>,      (const void*)k_ctail<double, kCtPairsMax>,
+                            (const void*)k_cg_cluster<float, kCtPairs>,    (const void*)k_cg_cluster<double, kCtPairs>,
+                            (const void*)k_cg_cluster<float, kCtPairsMax>, (const void*)k_cg_cluster<double, kCtPairsMax>};
   bool attr_ok = true;
   for (const void* k : kernels)
     attr_ok = attr_ok && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
@@ -1489,6 +1750,51 @@ void launch_ctail(cudaStream_t s, const Hierarchy<T>& H, const double* ainv, int
   cfg.attrs = at;
   cfg.numAttrs = 2;
   cudaLaunchKernelEx(&cfg, a.kpairs <= kCtPairs ? k_ctail<T, kCtPairs> : k_ctail<T, kCtPairsMax>, a, ainv, nu, done);
+}
+
+// The cluster CG serves grids whose finest level the cluster tail holds.
+template <typename T>
+bool cluster_cg(const Hierarchy<T>& H, int use_mg) {
+  static const bool off = [] {  // GB2D_CLUSTER_CG=0: the launched kernels, for comparison
+    const char* e = getenv("GB2D_CLUSTER_CG");
+    return e && e[0] == '0';
+  }();
+  return use_mg && H.ctail == 0 && !off;
+}
+// Runs the CG from the state that k_begin_loop or k_begin_device set.
+template <typename T>
+void launch_cg_cluster(cudaStream_t s, Solver* S, const Hierarchy<T>& H, const double* ainv, double* x, int nu) {
+  CgArgs<T> g;
+  g.a = H.ct[nu - 1];
+  g.a.sc = nullptr;
+  g.L = S->h64.L[0];
+  g.x = x;
+  g.r = S->h64.r;
+  g.p = S->p;
+  g.ap = S->ap;
+  g.rT = sizeof(T) == 4 ? H.r : nullptr;
+  g.ainv = ainv;
+  g.part_rr = slot(S, kSlotRr);
+  g.part_pap = slot(S, kSlotPap);
+  g.G = S->G;
+  g.nu = nu;
+  g.sc = S->sc;
+  g.done = S->done;
+  g.host = S->host + 2;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = H.ct_P;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(H.ct_P);
+  cfg.blockDim = dim3(kCtThreads);
+  cfg.dynamicSmemBytes = H.ct_smem[nu - 1];
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, g.a.kpairs <= kCtPairs ? k_cg_cluster<T, kCtPairs> : k_cg_cluster<T, kCtPairsMax>, g);
+  GB_LAUNCHED(1);
 }
 
 template <typename T>
@@ -1897,6 +2203,14 @@ int inner_pcg(gb2d_ctx* c, Solver* S, Hierarchy<T>& H, const double* ainv, doubl
               double* last_rr) {
   cudaStream_t s = c->stream;
   Probe* pr = &c->probe;
+  if (!pr->on && cluster_cg(H, use_mg)) {
+    k_begin_loop<<<1, 1, 0, s>>>(S->sc, S->done, thr2, max_it);
+    GB_LAUNCHED(1);
+    launch_cg_cluster<T>(s, S, H, ainv, x64, nu);
+    cudaStreamSynchronize(s);
+    *last_rr = S->host[2];
+    return (int)S->host[3];
+  }
   GraphSet* gs = pr->on ? nullptr : graphs_for<T>(c, S, H, ainv, x64, prec, use_mg, nu);
   if (gs && gs->loop) {  // the whole run on the device: one launch, one wait
     k_begin_loop<<<1, 1, 0, s>>>(S->sc, S->done, thr2, max_it);
@@ -2246,7 +2560,17 @@ int solve_on_device(gb2d_ctx* c, Solver* S, Hierarchy<T>& H, const double* ainv,
   residual();
   if (!joined) cudaStreamWaitEvent(s, join_ev, 0);
   cudaMemsetAsync(&S->sc->flag, 0, sizeof(int), s);
+  const bool in_cluster = cluster_cg(H, use_mg);  // one kernel instead of the loop node
+  S->body_nodes = 0;
   for (int pass = 0; pass < 2; ++pass) {
+    if (in_cluster) {
+      k_begin_device<<<1, 1, 0, s>>>(cudaGraphConditionalHandle(), 0, S->sc, S->done, c->sc, tol * tol, max_it, pass == 0);
+      launch_cg_cluster<T>(s, S, H, ainv, x, nu);
+      residual();
+      k_end_device<<<1, 1, 0, s>>>(S->sc, c->sc, pass == 1);
+      GB_LAUNCHED(2);
+      continue;
+    }
     cudaStreamCaptureStatus st;
     cudaGraph_t g = nullptr;
     if (cudaStreamGetCaptureInfo(s, &st, nullptr, &g, nullptr, nullptr, nullptr) != cudaSuccess || st != cudaStreamCaptureStatusActive) {
@@ -2259,7 +2583,7 @@ int solve_on_device(gb2d_ctx* c, Solver* S, Hierarchy<T>& H, const double* ainv,
       snprintf(c->err, sizeof(c->err), "device-driven solve: conditional handle refused");
       return GB2D_ERR_CUDA;
     }
-    k_begin_device<<<1, 1, 0, s>>>(h, S->sc, S->done, c->sc, tol * tol, max_it, pass == 0);
+    k_begin_device<<<1, 1, 0, s>>>(h, 1, S->sc, S->done, c->sc, tol * tol, max_it, pass == 0);
     GB_LAUNCHED(1);
     enqueue_init<T>(s, S, H, ainv, use_mg, nu, nullptr);
     if (!append_cg_loop<T>(s, c->body_stream, h, S, H, ainv, x, use_mg, nu)) {
