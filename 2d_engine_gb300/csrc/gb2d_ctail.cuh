@@ -53,6 +53,7 @@ struct CtLevel {
   int pairs;         // (nI + 1) / 2
   unsigned rpairs;   // 2^32 / pairs, rounded up (pairs > 1): u / pairs as a high product
   int H;             // halo rows of the window (0 on local levels)
+  int rcp;           // the residual as the tiled launches form it: dg as 1 / (1/dg), their order
   int x, xplane;     // x: red plane, black plane (xplane elements each)
   int b, xi, plane;  // right-hand side and received halo x: red, black (plane elements each); b -1 on the top level
   const T *cx, *cy, *idg, *dg, *bg;
@@ -68,6 +69,8 @@ struct CtArgs {
   int rg;     // the bottom distributed level's red residuals, all rows
   int bc;     // the coarsest level's right-hand side in cell order
   int zero_n; // elements from 0 to clear: every x, b plane
+  int inv;    // dense inverse in shared memory, element (m, row) at m * cells + row (doubles), or -1:
+              // rows summed in order by one thread each, as the single-CTA tail does
   CtLevel<T> L[kCtMaxLevels];
   short J0[kCtMaxLevels][kClusterMax + 1];  // CTA c owns rows [J0[l][c], J0[l][c+1])
   Scalars* sc;  // set when the top level is the finest: publish r.z and beta
@@ -243,8 +246,13 @@ __device__ __forceinline__ void ct_smooth_down(const CtArgs<T>& a, int l, int c,
     if (u < o0 || u >= o1) continue;
     const bool right = g.od[k] != 0;
     const T own = g.x[1][k], side = xb[right ? ad + 1 : ad - 1];
-    sm[a.res + u - o0] = ct_residual(g.b[0][k], dg[k], g.x[0][k], g.cl[0][k], right ? own : side, g.cr[0][k], right ? side : own,
-                                     g.y0[0][k], xb[ad - ps], g.y1[0][k], xb[ad + ps]);
+    const T xl = right ? own : side, xr = right ? side : own;
+    // A pair at an odd row's end may lack its red cell: 1/dg is the padding's zero there.
+    const T d = !L.rcp ? dg[k] : g.idg[0][k] == (T)0 ? (T)0 : diag_of(g.idg[0][k]);
+    sm[a.res + u - o0] = L.rcp ? gs_residual(g.b[0][k], d, g.x[0][k], g.cl[0][k], xl, g.cr[0][k], xr, g.y0[0][k],
+                                             xb[ad - ps], g.y1[0][k], xb[ad + ps])
+                               : ct_residual(g.b[0][k], d, g.x[0][k], g.cl[0][k], xl, g.cr[0][k], xr, g.y0[0][k], xb[ad - ps],
+                                             g.y1[0][k], xb[ad + ps]);
     if (l < a.ndist) {
       const int J = w.w0 + ct_row(L, u);
       auto push = [&](int d) {
@@ -324,9 +332,17 @@ struct CtDense {
   int zx[2];
 };
 template <typename T>
-__device__ __forceinline__ CtDense<T> ct_dense_load(const CtLevel<T>& Z, const double* __restrict__ ainv) {
+__device__ __forceinline__ CtDense<T> ct_dense_load(const CtArgs<T>& a, const double* __restrict__ ainv, T* sm) {
   CtDense<T> d;
+  const CtLevel<T>& Z = a.L[a.nlev - 1];
   const int nz = Z.nI * Z.nJ, tid = (int)threadIdx.x;
+  if (a.inv >= 0) {
+    double* inv = reinterpret_cast<double*>(sm + a.inv);
+    for (int u = tid; u < nz * nz; u += kCtThreads) {
+      const int r = u / nz, m = u - r * nz;
+      inv[m * nz + r] = ainv[u];
+    }
+  }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int r = (tid >> 4) + 32 * h, J = r / Z.nI, I = r - J * Z.nI;
@@ -341,8 +357,20 @@ __device__ __forceinline__ CtDense<T> ct_dense_load(const CtLevel<T>& Z, const d
 }
 // Right-hand side at bc, fixed-order tree sum.
 template <typename T>
-__device__ __forceinline__ void ct_dense_solve(const CtLevel<T>& Z, int bc, const CtDense<T>& d, T* sm) {
-  const int nz = Z.nI * Z.nJ, tid = (int)threadIdx.x, part = tid & 15;
+__device__ __forceinline__ void ct_dense_solve(const CtArgs<T>& a, const CtDense<T>& d, T* sm) {
+  const CtLevel<T>& Z = a.L[a.nlev - 1];
+  const int nz = Z.nI * Z.nJ, tid = (int)threadIdx.x, part = tid & 15, bc = a.bc;
+  if (a.inv >= 0) {
+    if (tid < nz) {
+      const double* inv = reinterpret_cast<const double*>(sm + a.inv) + tid;
+      double acc = 0.0;
+      for (int m = 0; m < nz; ++m) acc = __fma_rn(inv[m * nz], (double)sm[bc + m], acc);
+      const int J = tid / Z.nI, I = tid - J * Z.nI;
+      sm[Z.x + (((I + J) & 1) ? Z.xplane : 0) + (J + 1) * (Z.pairs + 2) + (I >> 1) + 1] = (T)acc;
+    }
+    __syncthreads();
+    return;
+  }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int r = (tid >> 4) + 32 * h;
@@ -456,7 +484,7 @@ __device__ __forceinline__ void ct_vcycle(const CtArgs<T>& a, int c, int P, cons
     __syncthreads();
     if (l < nd) ct_hand_down(a, l, c, P, sm);
   }
-  ct_dense_solve(a.L[nl - 1], a.bc, dense, sm);
+  ct_dense_solve(a, dense, sm);
   for (int l = nl - 2; l >= 0; --l) {
     const int n = ct_win(a, l, c).R * a.L[l].pairs;
     if (K > 1 && n > kCtThreads)
@@ -488,7 +516,7 @@ __global__ void __launch_bounds__(kCtThreads, 1) k_ctail(const __grid_constant__
   T* sm = reinterpret_cast<T*>(smem_raw);
   __shared__ double rz_part[kClusterMax];
   // Before the previous kernel has finished: what it does not write.
-  const CtDense<T> dense = ct_dense_load(a.L[a.nlev - 1], ainv);
+  const CtDense<T> dense = ct_dense_load(a, ainv, sm);
   for (int u = tid; u < a.zero_n; u += kCtThreads) sm[u] = (T)0;
   cl.sync();  // every CTA's planes are clear before any remote write
   pdl_enter();

@@ -1285,7 +1285,7 @@ __global__ void __launch_bounds__(kCtThreads, 1) k_cg_cluster(const __grid_const
   const CtArgs<T>& a = g.a;
   const Level<double>& L = g.L;
   if (*g.done) return;  // uniform over the cluster
-  const CtDense<T> dense = ct_dense_load(a.L[a.nlev - 1], g.ainv);
+  const CtDense<T> dense = ct_dense_load(a, g.ainv, sm);
   for (int u = tid; u < a.zero_n; u += kCtThreads) sm[u] = (T)0;
   const double thr2 = g.sc->thr2;
   const int max_it = g.sc->max_it, G = g.G;
@@ -1589,6 +1589,12 @@ bool layout_ctail(const CtArgs<T>& base, const int* stripe, int nu, CtArgs<T>* o
   off += a.L[a.ndist - 1].nJ * a.L[a.ndist - 1].pairs;
   a.bc = off;
   off += a.L[nl - 1].nI * a.L[nl - 1].nJ;
+  if (a.inv >= 0) {  // rows summed in order: the inverse in shared memory, 16-byte aligned
+    off = (off + 3) & ~3;
+    a.inv = off;
+    const int nc = a.L[nl - 1].nI * a.L[nl - 1].nJ;
+    off += nc * nc * (int)(sizeof(double) / sizeof(T));
+  }
   a.kpairs = (items + kCtThreads - 1) / kCtThreads;
   if ((size_t)off * sizeof(T) > kCtSmemCap || a.kpairs > kCtPairsMax) return false;
   *out = a;
@@ -1601,9 +1607,7 @@ bool layout_ctail(const CtArgs<T>& base, const int* stripe, int nu, CtArgs<T>* o
 // coarsest level is always local.  Returns false (single-CTA tail instead) when
 // no top level qualifies.
 template <typename T>
-bool plan_ctail(Hierarchy<T>& H, int P) {
-  H.ctail = -1;
-  if (P < 2 || P > kClusterMax) return false;
+bool plan_ctail_from(Hierarchy<T>& H, int P, bool small) {
   const int nl = H.nlev;
   const char* env = getenv("GB2D_CTAIL_TOP_CELLS");  // tuning override of kCtMaxTopCells
   const long top_cells = env && atol(env) > 0 ? atol(env) : kCtMaxTopCells;
@@ -1611,12 +1615,14 @@ bool plan_ctail(Hierarchy<T>& H, int P) {
   const int min_rows = env_rows && atoi(env_rows) > 0 ? atoi(env_rows) : kCtMinRows;
   for (int top = 0; top < nl - 1; ++top) {
     if (nl - top > kCtMaxLevels) continue;
-    if ((long)H.L[top].nI * H.L[top].nJ > top_cells) continue;
+    if ((long)H.L[top].nI * H.L[top].nJ > (small ? (long)kTailCells : top_cells)) continue;
+    if (small && (top == 0 || top > H.tail)) continue;  // levels from the tail down have no tiled launches
     int lb = top - 1;
-    while (lb + 1 < nl - 1 && H.L[lb + 1].nJ >= P * min_rows) ++lb;
+    while (lb + 1 < nl - 1 && H.L[lb + 1].nJ >= P * (small ? 2 : min_rows)) ++lb;
     if (lb < top || H.L[lb].nJ > kCtOwnerRows) continue;
     CtArgs<T> a;
     memset(&a, 0, sizeof a);
+    a.inv = small ? 0 : -1;
     a.nlev = nl - top;
     int stripe[kCtMaxLevels];  // rows of each level's widest stripe
     // Stripes of levels 0 .. ndist - 1: the bottom one's rows in equal parts, nested above.
@@ -1655,10 +1661,11 @@ bool plan_ctail(Hierarchy<T>& H, int P) {
       C.dg = L.dg;
       C.bg = L.b;
       C.xg = L.x;
+      C.rcp = small && top + l < H.tail;
       cells += (l == nd - 1 ? 7 : 6) * (size_t)(stripe[l] + 2) * L.ld;
     }
     const size_t nc = (size_t)H.L[nl - 1].nI * H.L[nl - 1].nJ;
-    if (!ok || (cells + nc * nc + nc) * sizeof(T) > kCtSmemCap) continue;
+    if (!ok || (!small && (cells + nc * nc + nc) * sizeof(T) > kCtSmemCap)) continue;
     // One level more, of at least two rows per CTA, where running it in every CTA takes
     // more than one pair per thread, or is FP64 (each CTA's FP64 pipe is the bound): 16
     // batched bubbles 9.1 -> 8.6 ms, the FP64 frame at 128^2 3.65 -> 3.50 ms; in FP32 with
@@ -1666,7 +1673,7 @@ bool plan_ctail(Hierarchy<T>& H, int P) {
     // Not where that moves the finest level's stripes, whose sums of r.z they order.
     short J0top[kClusterMax + 1];
     memcpy(J0top, a.J0[0], sizeof J0top);
-    bool deeper = lb + 1 < nl - 1 && H.L[lb + 1].nJ >= 2 * P && (sizeof(T) == 8 || a.L[nd].pairs * a.L[nd].nJ > kCtThreads) &&
+    bool deeper = !small && lb + 1 < nl - 1 && H.L[lb + 1].nJ >= 2 * P && (sizeof(T) == 8 || a.L[nd].pairs * a.L[nd].nJ > kCtThreads) &&
                   distribute(nd + 1) && (top > 0 || memcmp(J0top, a.J0[0], (size_t)(P + 1) * sizeof(short)) == 0);
     for (int nu = 1; nu <= 3 && deeper; ++nu) deeper = layout_ctail(a, stripe, nu, &H.ct[nu - 1], &H.ct_smem[nu - 1]);
     if (!deeper) {
@@ -1679,6 +1686,18 @@ bool plan_ctail(Hierarchy<T>& H, int P) {
     return true;
   }
   return false;
+}
+
+// The cluster tail: from the levels of 128^2 cells down where whole stripes of them would
+// fit one CTA, else from those of 64^2 down, with the residuals and the dense solve of the
+// launches that it replaces there (tiled levels and the single-CTA tail), whose values it
+// reproduces.  FP64 projection at 511 x 385: 3.07 ms with those launches, 2.76 from the
+// 64 x 49 level down, 2.86 from the 128 x 97 one, whose own two launches fill more SMs.
+template <typename T>
+bool plan_ctail(Hierarchy<T>& H, int P) {
+  H.ctail = -1;
+  if (P < 2 || P > kClusterMax) return false;
+  return plan_ctail_from(H, P, false) || plan_ctail_from(H, P, true);
 }
 
 // Cluster size the part can co-schedule for the cluster tail (16, else 8), or 0.
