@@ -4,8 +4,9 @@
 // gs_update, warp_sum, reduce_scratch, publish_rz, kMaxLevels, kCoarseMax).
 //
 // Every level from the cluster's top level (at most 128^2 cells) down to the dense
-// coarse solve runs inside one launch of a cluster of P CTAs (16 where the part
-// allows it, else 8), each CTA one SM with 512 threads:
+// coarse solve runs inside one launch of a cluster of P CTAs, each CTA one SM with 512
+// threads: 16 where the part allows it, else 8; fewer, down to a single CTA, on
+// hierarchies of too few rows (plan_ctail):
 //
 //   * distributed levels: the rows of a level are split into P contiguous
 //     stripes, one per CTA, nested from level to level (the fine rows of a CTA's
@@ -15,7 +16,7 @@
 //     exchange; halo rows of the right-hand side and of x are pushed into the
 //     neighbours' shared memory (distributed shared memory) when a level is left,
 //     and one cluster barrier per level makes them visible;
-//   * local levels (fewer than P * kCtMinRows rows): the stripes' restricted
+//   * local levels (too few rows for P stripes): the stripes' restricted
 //     residuals are pushed to every CTA, which runs these levels and the dense
 //     coarse solve redundantly, with block barriers only; every CTA computes
 //     identical values (same inputs, same order), and each prolongs from its own.
@@ -71,6 +72,7 @@ struct CtArgs {
   int zero_n; // elements from 0 to clear: every x, b plane
   int inv;    // dense inverse in shared memory, element (m, row) at m * cells + row (doubles), or -1:
               // rows summed in order by one thread each, as the single-CTA tail does
+  int gather; // r.z of all rows summed by the first CTA, as the single-CTA tail sums it
   CtLevel<T> L[kCtMaxLevels];
   short J0[kCtMaxLevels][kClusterMax + 1];  // CTA c owns rows [J0[l][c], J0[l][c+1])
   Scalars* sc;  // set when the top level is the finest: publish r.z and beta
@@ -442,11 +444,18 @@ __device__ __forceinline__ void ct_hand_down(const CtArgs<T>& a, int l, int c, i
 
 // r.z when the top level is the finest: a block sum over 1024 strided partials (two per
 // thread) in block_sum's order; a warp's sum over no elements is the zero it would add up.
-// Valid in the first warp's lane 0.
+// Valid in the first warp's lane 0.  With a.gather the first CTA sums all rows, from global
+// memory, once every CTA's x is there.
 template <typename T>
 __device__ __forceinline__ double ct_rz(const CtArgs<T>& a, int c, const T* sm) {
   const CtLevel<T>& L = a.L[0];
-  const CtWin w = ct_win(a, 0, c);
+  CtWin w = ct_win(a, 0, c);
+  if (a.gather) {
+    cgx::this_cluster().sync();
+    if (c > 0) return 0.0;
+    w.J0 = 0;
+    w.J1 = L.nJ;
+  }
   double* scratch = reduce_scratch();
   const int n = (w.J1 - w.J0) * L.nI, tid = (int)threadIdx.x;
 #pragma unroll
@@ -455,8 +464,9 @@ __device__ __forceinline__ double ct_rz(const CtArgs<T>& a, int c, const T* sm) 
     if ((tid & ~31) + h * kCtThreads < n) {
       for (int u = tid + h * kCtThreads; u < n; u += 2 * kCtThreads) {
         const int lr = u / L.nI, i = u - lr * L.nI, J = w.J0 + lr;
-        const T bv = __ldcg(L.bg + (J + 1) * L.ld + i + 1);
-        const T xv = sm[L.x + (((i + J) & 1) ? L.xplane : 0) + (J - w.w0 + 1) * (L.pairs + 2) + (i >> 1) + 1];
+        const int q = (J + 1) * L.ld + i + 1;
+        const T bv = __ldcg(L.bg + q);
+        const T xv = a.gather ? __ldcg(L.xg + q) : sm[L.x + (((i + J) & 1) ? L.xplane : 0) + (J - w.w0 + 1) * (L.pairs + 2) + (i >> 1) + 1];
         acc = __fma_rn((double)bv, (double)xv, acc);
       }
       acc = warp_sum(acc);
@@ -472,7 +482,7 @@ template <int K, typename T>
 __device__ __forceinline__ void ct_vcycle(const CtArgs<T>& a, int c, int P, const CtDense<T>& dense, T* sm, int nu) {
   const int nl = a.nlev, nd = a.ndist, tid = (int)threadIdx.x;
   for (int l = 0; l < nl; ++l) {
-    if (l >= nd) ct_restrict_local(a, l, sm);
+    if (l >= nd && l > 0) ct_restrict_local(a, l, sm);
     if (l == nl - 1) break;
     const int n = ct_win(a, l, c).R * a.L[l].pairs;
     if (K > 1 && n > kCtThreads)

@@ -1586,7 +1586,7 @@ bool layout_ctail(const CtArgs<T>& base, const int* stripe, int nu, CtArgs<T>* o
   a.res = off;
   off += own;
   a.rg = off;
-  off += a.L[a.ndist - 1].nJ * a.L[a.ndist - 1].pairs;
+  if (a.ndist > 0) off += a.L[a.ndist - 1].nJ * a.L[a.ndist - 1].pairs;
   a.bc = off;
   off += a.L[nl - 1].nI * a.L[nl - 1].nJ;
   if (a.inv >= 0) {  // rows summed in order: the inverse in shared memory, 16-byte aligned
@@ -1602,10 +1602,10 @@ bool layout_ctail(const CtArgs<T>& base, const int* stripe, int nu, CtArgs<T>* o
   return true;
 }
 
-// Lay out the cluster tail: the finest top level whose levels fit in one CTA's
-// shared memory.  Distributed levels have at least P * kCtMinRows rows; the
-// coarsest level is always local.  Returns false (single-CTA tail instead) when
-// no top level qualifies.
+// Lay out a cluster tail of P CTAs: the finest top level whose levels fit in one CTA's
+// shared memory.  Distributed levels have at least kCtMinRows rows per CTA (small: two, and
+// none in a cluster of one); the coarsest level is always local.  False when no top level
+// qualifies.
 template <typename T>
 bool plan_ctail_from(Hierarchy<T>& H, int P, bool small) {
   const int nl = H.nlev;
@@ -1616,20 +1616,22 @@ bool plan_ctail_from(Hierarchy<T>& H, int P, bool small) {
   for (int top = 0; top < nl - 1; ++top) {
     if (nl - top > kCtMaxLevels) continue;
     if ((long)H.L[top].nI * H.L[top].nJ > (small ? (long)kTailCells : top_cells)) continue;
-    if (small && (top == 0 || top > H.tail)) continue;  // levels from the tail down have no tiled launches
+    // Levels from the tail down have no tiled launches, and those sum r.z in another order.
+    if (small && (top > H.tail || (top == 0 && H.tail > 0))) continue;
     int lb = top - 1;
-    while (lb + 1 < nl - 1 && H.L[lb + 1].nJ >= P * (small ? 2 : min_rows)) ++lb;
-    if (lb < top || H.L[lb].nJ > kCtOwnerRows) continue;
+    while (P > 1 && lb + 1 < nl - 1 && H.L[lb + 1].nJ >= P * (small ? 2 : min_rows)) ++lb;
+    if (P > 1 ? lb < top || H.L[lb].nJ > kCtOwnerRows : top != H.tail) continue;
     CtArgs<T> a;
     memset(&a, 0, sizeof a);
     a.inv = small ? 0 : -1;
+    a.gather = small && top == 0;
     a.nlev = nl - top;
     int stripe[kCtMaxLevels];  // rows of each level's widest stripe
     // Stripes of levels 0 .. ndist - 1: the bottom one's rows in equal parts, nested above.
     auto distribute = [&](int ndist) {
       a.ndist = ndist;
       bool ok = true;
-      for (int c = 0; c <= P; ++c) a.J0[ndist - 1][c] = (short)((long)c * H.L[top + ndist - 1].nJ / P);
+      for (int c = 0; c <= P && ndist > 0; ++c) a.J0[ndist - 1][c] = (short)((long)c * H.L[top + ndist - 1].nJ / P);
       for (int l = ndist - 2; l >= 0; --l) {
         for (int c = 0; c < P; ++c) a.J0[l][c] = (short)(2 * a.J0[l + 1][c]);
         a.J0[l][P] = (short)H.L[top + l].nJ;
@@ -1679,7 +1681,7 @@ bool plan_ctail_from(Hierarchy<T>& H, int P, bool small) {
     if (!deeper) {
       distribute(nd);
       for (int nu = 1; nu <= 3 && ok; ++nu) ok = layout_ctail(a, stripe, nu, &H.ct[nu - 1], &H.ct_smem[nu - 1]);
-      if (!ok) continue;
+      if (!ok || (P == 1 && H.ct[0].kpairs > kCtPairs)) continue;  // one CTA: mixed 60 x 50 0.95 -> 1.02 ms
     }
     H.ctail = top;
     H.ct_P = P;
@@ -1689,15 +1691,22 @@ bool plan_ctail_from(Hierarchy<T>& H, int P, bool small) {
 }
 
 // The cluster tail: from the levels of 128^2 cells down where whole stripes of them would
-// fit one CTA, else from those of 64^2 down, with the residuals and the dense solve of the
-// launches that it replaces there (tiled levels and the single-CTA tail), whose values it
-// reproduces.  FP64 projection at 511 x 385: 3.07 ms with those launches, 2.76 from the
-// 64 x 49 level down, 2.86 from the 128 x 97 one, whose own two launches fill more SMs.
+// fit one CTA, else from those of 64^2 down in as many CTAs as leave each two rows, with the
+// residuals, the dense solve and the sum of r.z of the launches that it replaces there
+// (tiled levels and the single-CTA tail), whose values it reproduces.  FP64 projection at
+// 511 x 385: 3.07 ms with those launches, 2.76 from the 64 x 49 level down, 2.86 from the
+// 128 x 97 one, whose own two launches fill more SMs.  Projections with the single-CTA tail
+// / one CTA here / at most 4, 8, 16: FP64 64 x 40 1.28 / 1.53 / 0.93 / 0.82 / 0.83 ms, 40 x 32
+// 0.92 / 0.85 / 0.70 / 0.68 / 0.67, mixed 100 x 40 1.15 / 1.30 / 0.87 / 0.79 / 0.78, 640 x 480
+// (tail from 40 x 30) 1.98 / 1.82 / 1.85 / 1.80 / 1.80.
 template <typename T>
 bool plan_ctail(Hierarchy<T>& H, int P) {
   H.ctail = -1;
   if (P < 2 || P > kClusterMax) return false;
-  return plan_ctail_from(H, P, false) || plan_ctail_from(H, P, true);
+  if (plan_ctail_from(H, P, false)) return true;
+  for (int q : {16, 8, 4, 1})
+    if (q <= P && plan_ctail_from(H, q, true)) return true;
+  return false;
 }
 
 // Cluster size the part can co-schedule for the cluster tail (16, else 8), or 0.
@@ -2415,15 +2424,16 @@ void solver_destroy(Solver* S) {
 }
 
 void solver_layout(const Solver* S, int mixed, int* levels, int* cluster_top, int* cluster_ctas) {
-  if (mixed) {
-    *levels = S->h32.nlev;
-    *cluster_top = S->h32.ctail;
-    *cluster_ctas = S->h32.ctail >= 0 ? S->h32.ct_P : 0;
-  } else {
-    *levels = S->h64.nlev;
-    *cluster_top = S->h64.ctail;
-    *cluster_ctas = S->h64.ctail >= 0 ? S->h64.ct_P : 0;
-  }
+  auto report = [&](const auto& H) {
+    const bool cluster = H.ctail >= 0 && H.ct_P > 1;
+    *levels = H.nlev;
+    *cluster_top = cluster ? H.ctail : -1;
+    *cluster_ctas = cluster ? H.ct_P : 0;
+  };
+  if (mixed)
+    report(S->h32);
+  else
+    report(S->h64);
 }
 
 // Tile shapes of the tiled smoothing levels: plan < 0 restores the default rule

@@ -30,3 +30,30 @@ def test_vcycle_has_the_single_cta_tails_bits(gb, ni, nj):
     for a, b in zip(z[True], z[False]):
         assert np.all(np.isfinite(a)) and np.linalg.norm(a) > 0
         assert np.array_equal(a, b) if small else rel_l2(a, b) <= 1e-11
+
+
+# Grids that the 64^2 form holds whole (r.z summed by its first CTA), over the numbers of CTAs
+# that their rows allow (16, 8, 4, 1), one of more levels with its tail at 40 x 30, and the
+# smallest ones: whole solves, both precisions.  8 x 120 is the larger form's (64 rows and
+# up): its V-cycles to the tolerances of tests/test_gpu_cluster_windows.py.
+@pytest.mark.parametrize("ni,nj", [(64, 48), (65, 63), (40, 32), (41, 31), (63, 17), (100, 15), (16, 9), (24, 8), (9, 9), (8, 120), (640, 480)])
+@pytest.mark.parametrize("prec_name", ["FP64", "MIXED"])
+def test_solve_has_the_single_cta_tails_bits(gb, ni, nj, prec_name):
+    prec = getattr(gb, "PRECISION_" + prec_name)
+    case = case_for(ni, nj, 3)
+    got = {}
+    for cluster in (True, False):
+        c = make(gb, case, cluster)
+        rhs = system(gb, c, 0.5 / (max(ni, nj) - 1))
+        r = rhs + np.random.default_rng(ni * nj).standard_normal((nj, ni)) * np.abs(rhs).max() * 1e-3
+        got[cluster] = [c.preconditioner_apply(r, prec, nu) for nu in (1, 2, 3)]
+        for nu in (1, 2, 3):
+            x, st = c.poisson_solve(rhs, opts=gb.solve_opts(precision=prec, tolerance=1e-9, mg_smooth=nu), allow_max_iters=True)
+            got[cluster] += [x, np.array([st.iterations, st.outer_iterations])]
+        c.close()
+    if (ni, nj) == (8, 120):
+        for a, b in zip(got[True][:3], got[False][:3]):
+            assert np.all(np.isfinite(a)) and rel_l2(a, b) <= (1e-11 if prec_name == "FP64" else 2e-5)
+        return
+    for a, b in zip(got[True], got[False]):
+        assert np.all(np.isfinite(a)) and np.array_equal(a, b)
