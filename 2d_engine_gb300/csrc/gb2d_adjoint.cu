@@ -990,7 +990,8 @@ int adjoint_buffers(gb2d_ctx* c) {
       return GB2D_ERR_CUDA;
     }
   }
-  return GB2D_OK;
+  // Cleared on the legacy stream, which the context's streams do not wait for.
+  return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? GB2D_OK : GB2D_ERR_CUDA;
 }
 
 void launch_weno5_adjoint(cudaStream_t s, gb2d_ctx* c, double dt, double* mu_ua, double* mu_va) {

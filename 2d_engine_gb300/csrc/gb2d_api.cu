@@ -242,6 +242,13 @@ int gb2d_create(const gb2d_grid* grid, const gb2d_params* params, gb2d_ctx** out
     cudaGetLastError();
     return GB2D_ERR_CUDA;
   }
+  // The buffers were cleared on the legacy stream, which the context's non-blocking streams
+  // do not wait for: without this a first upload can be overwritten by a late clear.
+  if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+    cudaGetLastError();
+    free_ctx(c);
+    return GB2D_ERR_CUDA;
+  }
   *out = c;
   return GB2D_OK;
 }

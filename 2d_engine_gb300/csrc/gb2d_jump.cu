@@ -172,6 +172,8 @@ int jump_buffers(gb2d_ctx* c) {
   }
   cudaError_t e = cudaMalloc(&c->jmp_phi, (ni + 4) * (nj + 4) * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&c->jmp_bc, np * sizeof(int));
+  // Cleared on the legacy stream, which the context's streams do not wait for.
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
   return e == cudaSuccess ? GB2D_OK : GB2D_ERR_CUDA;
 }
 
