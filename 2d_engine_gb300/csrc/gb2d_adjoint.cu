@@ -20,61 +20,79 @@ namespace gb2d {
 
 namespace {
 
-// d f / d a_m of one WENO5 side f(a1..a5) = sum_k w_k P_k (ADVECTION_METHOD_2D.h:545-619):
+// x / y for x, y >= 0, y not tiny or huge where the quotient is taken on the integer pipes.
+__device__ __noinline__ double plain_quotient(double x, double y) { return x / y; }
+__device__ __forceinline__ bool mid_positive(double x) { return words(x).hi - ((1023u - 500u) << 20) < (1000u << 20); }
+__device__ __forceinline__ double quotient(double x, double y) {
+  return mid_positive(x) && mid_positive(y) ? div_pos(x, y) : plain_quotient(x, y);
+}
+
+// One WENO5 side f(a_0..a_4) = sum_k w_k P_k (ADVECTION_METHOD_2D.h:545-619) of the
+// differences a_t = os (q_{t+1} - q_t), and its derivative with respect to q_0..q_5:
 //   df/da = sum_k w_k dP_k/da + sum_k (P_k - f) / S * dalpha_k/da,
-//   alpha_k = c_k / (eps + beta_k)^2, S = sum alpha_k, w_k = alpha_k / S.
-__device__ void weno5_side_grad(const double a[5], double eps, double& f, double g[5]) {
-  const double A[3] = {a[0] - 2 * a[1] + a[2], a[1] - 2 * a[2] + a[3], a[2] - 2 * a[3] + a[4]};
-  const double B[3] = {a[0] - 4 * a[1] + 3 * a[2], a[1] - a[3], 3 * a[2] - 4 * a[3] + a[4]};
-  const double dA[3][5] = {{1, -2, 1, 0, 0}, {0, 1, -2, 1, 0}, {0, 0, 1, -2, 1}};
-  const double dB[3][5] = {{1, -4, 3, 0, 0}, {0, 1, 0, -1, 0}, {0, 0, 3, -4, 1}};
-  const double dP[3][5] = {{1.0 / 3, -7.0 / 6, 11.0 / 6, 0, 0}, {0, -1.0 / 6, 5.0 / 6, 1.0 / 3, 0}, {0, 0, 1.0 / 3, 5.0 / 6, -1.0 / 6}};
+//   alpha_k = c_k / (eps + beta_k)^2, S = sum alpha_k, w_k = alpha_k / S,
+// J_m = scale (df/da_{m-1} - df/da_m).
+// The FP64 pipe bounds it (16 cycles of an SM a warp instruction), so: nine quotients,
+// formed beside it, in place of twelve on it; factors 2^k folded into constants; terms
+// that several derivatives share formed once.  About 105 FP64 operations, from some 280.
+__device__ __forceinline__ void weno5_side_grad(const double q[6], double os, double scale, double eps, double& f, double J[6]) {
+  double a[5];
+#pragma unroll
+  for (int t = 0; t < 5; ++t) a[t] = os * (q[t + 1] - q[t]);
+  const double A[3] = {__fma_rn(-2.0, a[1], a[0]) + a[2], __fma_rn(-2.0, a[2], a[1]) + a[3], __fma_rn(-2.0, a[3], a[2]) + a[4]};
+  const double B[3] = {__fma_rn(3.0, a[2], __fma_rn(-4.0, a[1], a[0])), a[1] - a[3], __fma_rn(3.0, a[2], __fma_rn(-4.0, a[3], a[4]))};
+  const double P[3] = {__fma_rn(11.0 / 6, a[2], __fma_rn(-7.0 / 6, a[1], 1.0 / 3 * a[0])),
+                       __fma_rn(1.0 / 3, a[3], __fma_rn(5.0 / 6, a[2], -1.0 / 6 * a[1])),
+                       __fma_rn(-1.0 / 6, a[4], __fma_rn(5.0 / 6, a[3], 1.0 / 3 * a[2]))};
   const double c[3] = {0.1, 0.6, 0.3};
-  double beta[3], al[3], P[3], S = 0;
+  double tA[3], tB[3], h[3], al[3], w[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    beta[k] = 13.0 / 12.0 * A[k] * A[k] + 0.25 * B[k] * B[k];
-    al[k] = c[k] / ((eps + beta[k]) * (eps + beta[k]));
-    S += al[k];
-    P[k] = 0;
-#pragma unroll
-    for (int m = 0; m < 5; ++m) P[k] += dP[k][m] * a[m];
+    tA[k] = 13.0 / 12.0 * A[k];
+    tB[k] = 0.25 * B[k];
+    const double e = __fma_rn(tB[k], B[k], __fma_rn(tA[k], A[k], eps));
+    h[k] = quotient(4.0, e);
+    al[k] = quotient(c[k], e * e);
   }
-  f = 0;
+  const double S = al[0] + al[1] + al[2];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) f += al[k] / S * P[k];
-#pragma unroll
-  for (int m = 0; m < 5; ++m) g[m] = 0;
+  for (int k = 0; k < 3; ++k) w[k] = quotient(al[k], S);
+  f = __fma_rn(w[2], P[2], __fma_rn(w[1], P[1], w[0] * P[0]));
+  double rA[3], rB[3];  // r dbeta_k/dA_k and r dbeta_k/dB_k, r = -2 w_k (P_k - f) / (eps + beta_k)
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const double w = al[k] / S, r = (P[k] - f) / S * (-2 * al[k] / (eps + beta[k]));
-#pragma unroll
-    for (int m = 0; m < 5; ++m) g[m] += w * dP[k][m] + r * (13.0 / 6.0 * A[k] * dA[k][m] + 0.5 * B[k] * dB[k][m]);
+    const double r = (f - P[k]) * w[k] * h[k];
+    rA[k] = r * tA[k];
+    rB[k] = r * tB[k];
   }
+  const double X0 = rA[0] + rB[0], X1 = rA[1] + rB[1], X2 = rA[2] + rB[2];
+  const double g0 = __fma_rn(1.0 / 3, w[0], X0);
+  const double g1 = __fma_rn(-7.0 / 6, w[0], __fma_rn(-2.0, rA[0], __fma_rn(-4.0, rB[0], __fma_rn(-1.0 / 6, w[1], X1))));
+  const double g2 = __fma_rn(11.0 / 6, w[0], __fma_rn(2.0, rB[0], X0)) + __fma_rn(5.0 / 6, w[1], -2.0 * rA[1]) +
+                    __fma_rn(1.0 / 3, w[2], __fma_rn(2.0, rB[2], X2));
+  const double g3 = __fma_rn(1.0 / 3, w[1], rA[1] - rB[1]) + __fma_rn(5.0 / 6, w[2], __fma_rn(-2.0, rA[2], -4.0 * rB[2]));
+  const double g4 = __fma_rn(-1.0 / 6, w[2], X2);
+  J[0] = -scale * g0;
+  J[1] = scale * (g0 - g1);
+  J[2] = scale * (g1 - g2);
+  J[3] = scale * (g2 - g3);
+  J[4] = scale * (g3 - g4);
+  J[5] = scale * g4;
 }
 
 // Derivative of the upwind WENO5 derivative along one line with respect to its seven
-// stencil values q[0..6] (offsets -3..+3): minus side (d0..d4) when up, else plus side
-// (d5..d1); d_k = o (q[k+1] - q[k]).  f receives the derivative itself.
-__device__ void weno5_line_grad(const double q[7], double o, double eps, bool up, double& f, double J[7]) {
-  double d[6], gd[6] = {0, 0, 0, 0, 0, 0}, a[5], g[5];
+// stencil values q[0..6] (offsets -3..+3).  f receives the derivative itself.  The minus
+// side (up) uses q[0..5] with o (q[k+1] - q[k]); the plus side is the same function of the
+// mirrored values q[6..1] with -o.
+__device__ __forceinline__ void weno5_line_grad(const double q[7], double o, double eps, bool up, double& f, double J[7]) {
+  double c[6], H[6];
+  const double os = up ? o : -o;
 #pragma unroll
-  for (int k = 0; k < 6; ++k) d[k] = o * (q[k + 1] - q[k]);
-  if (up) {
+  for (int m = 0; m < 6; ++m) c[m] = up ? q[m] : q[6 - m];
+  weno5_side_grad(c, os, os, eps, f, H);
+  J[up ? 6 : 0] = 0.0;
 #pragma unroll
-    for (int t = 0; t < 5; ++t) a[t] = d[t];
-    weno5_side_grad(a, eps, f, g);
-#pragma unroll
-    for (int t = 0; t < 5; ++t) gd[t] = g[t];
-  } else {
-#pragma unroll
-    for (int t = 0; t < 5; ++t) a[t] = d[5 - t];
-    weno5_side_grad(a, eps, f, g);
-#pragma unroll
-    for (int t = 0; t < 5; ++t) gd[5 - t] = g[t];
-  }
-#pragma unroll
-  for (int m = 0; m < 7; ++m) J[m] = o * ((m > 0 ? gd[m - 1] : 0.0) - (m < 6 ? gd[m] : 0.0));
+  for (int m = 0; m < 6; ++m) J[up ? m : 6 - m] = H[m];
 }
 
 // The seven stencil positions of the ghost-filled copy read clamped positions of the
@@ -88,30 +106,40 @@ struct AdjArgs {
 
 // Per interior node n: C[m] = -dt u_n lam_n dfx/dq_m (m = 0..6) and the same for y
 // (m = 7..13); gv = -dt lam f / 2 per direction (the face-averaged velocity's share).
-__global__ void k_weno5_adj_coef(const double* __restrict__ phi_a, const double* __restrict__ ua_a, const double* __restrict__ va_a,
-                                 const double* __restrict__ lam_a, double* __restrict__ coef, double* __restrict__ gvel, AdjArgs a) {
+// A thread per node and direction (blockIdx.z), blocks of 64: the FP64 pipe is the bound (27
+// of the 30 us that it takes at 256^2), and small blocks spread evenly over the SMs.  With
+// both directions in a thread, blocks of 256 and either side of the upwind switch evaluated
+// where a warp mixes them, the adjoint from host arrays took 238 us; with this, 128.
+constexpr int kCoefThreads = 64;
+__global__ void __launch_bounds__(kCoefThreads) k_weno5_adj_coef(const double* __restrict__ phi_a, const double* __restrict__ ua_a,
+                                                                 const double* __restrict__ va_a, const double* __restrict__ lam_a,
+                                                                 double* __restrict__ coef, double* __restrict__ gvel, AdjArgs a) {
   const int ni = a.ni, nj = a.nj;
   const DField phi = dfield((double*)phi_a, 2, ni, nj), lam = dfield((double*)lam_a, 2, ni, nj);
   const DField ua = dfield((double*)ua_a, 3, ni + 1, nj), va = dfield((double*)va_a, 3, ni, nj + 1);
   const size_t n = (size_t)ni * nj;
+  const bool y = blockIdx.z != 0;
+  if (y) {
+    coef += 7 * n;
+    gvel += n;
+  }
   GB_FOR_IJ(i, j, ni, nj) {
     const size_t t = (size_t)j * ni + i;
-    const double u = (GB_AT(ua, i + 1, j) + GB_AT(ua, i, j)) * 0.5;
-    const double v = (GB_AT(va, i, j + 1) + GB_AT(va, i, j)) * 0.5;
-    const double l = GB_AT(lam, i, j);
-    double q[7], J[7], fx, fy;
+    const double vel = (y ? GB_AT(va, i, j + 1) + GB_AT(va, i, j) : GB_AT(ua, i + 1, j) + GB_AT(ua, i, j)) * 0.5;
+    const double l = GB_AT(lam, i, j), dl = -a.dt * l, o = y ? a.ody : a.odx;
+    const bool up = gtz(vel);
+    const double os = up ? o : -o;
+    double q[6], J[6], f;
 #pragma unroll
-    for (int m = 0; m < 7; ++m) q[m] = GB_AT(phi, clamp_line(i - 3 + m, ni), j);
-    weno5_line_grad(q, a.odx, a.eps, gtz(u), fx, J);
+    for (int m = 0; m < 6; ++m) {
+      const int d = up ? m - 3 : 3 - m;
+      q[m] = y ? GB_AT(phi, i, clamp_line(j + d, nj)) : GB_AT(phi, clamp_line(i + d, ni), j);
+    }
+    weno5_side_grad(q, os, -a.dt * vel * l * os, a.eps, f, J);
+    coef[(up ? 6 : 0) * n + t] = 0.0;
 #pragma unroll
-    for (int m = 0; m < 7; ++m) coef[m * n + t] = -a.dt * u * l * J[m];
-#pragma unroll
-    for (int m = 0; m < 7; ++m) q[m] = GB_AT(phi, i, clamp_line(j - 3 + m, nj));
-    weno5_line_grad(q, a.ody, a.eps, gtz(v), fy, J);
-#pragma unroll
-    for (int m = 0; m < 7; ++m) coef[(7 + m) * n + t] = -a.dt * v * l * J[m];
-    gvel[t] = -a.dt * l * fx * 0.5;
-    gvel[n + t] = -a.dt * l * fy * 0.5;
+    for (int m = 0; m < 6; ++m) coef[(up ? m : 6 - m) * n + t] = J[m];
+    gvel[t] = dl * f * 0.5;
   }
 }
 
@@ -205,6 +233,15 @@ __global__ void k_reinit_adj_coef(const double* __restrict__ phi_a, const double
 __device__ __forceinline__ double line_gather(const double* __restrict__ coef, size_t n, size_t stride, size_t base, int k, int nk,
                                               int mbase) {
   double acc = 0;
+  if (k >= 3 && k <= nk - 4) {  // seven independent loads, added in the loop's order
+    const double* q = coef + base + (size_t)(k - 3) * stride;
+    double v[7];
+#pragma unroll
+    for (int d = 0; d < 7; ++d) v[d] = q[(size_t)(mbase + 6 - d) * n + (size_t)d * stride];
+#pragma unroll
+    for (int d = 0; d < 7; ++d) acc += v[d];
+    return acc;
+  }
   int ps[4] = {k, 0, 0, 0}, np = 1;
   if (k == 1) {
     ps[1] = -1;
@@ -227,28 +264,44 @@ __device__ __forceinline__ double line_gather(const double* __restrict__ coef, s
 
 // mu = lam (identity part) + the stencil coefficients gathered onto each interior
 // node; ghost positions pass lam through (the sweep copies the input's ghost ring).
-__global__ void k_weno5_adj_gather(const double* __restrict__ lam_a, const double* __restrict__ coef, double* __restrict__ mu_a, AdjArgs a) {
+__device__ __forceinline__ void gather_node(const double* __restrict__ lam_a, const double* __restrict__ coef, double* __restrict__ mu_a,
+                                            const AdjArgs& a, int i, int j) {
   const int ni = a.ni, nj = a.nj;
   const DField lam = dfield((double*)lam_a, 2, ni, nj), mu = dfield(mu_a, 2, ni, nj);
   const size_t n = (size_t)ni * nj;
-  GB_FOR_IJ(ii, jj, ni + 4, nj + 4) {
-    const int i = ii - 2, j = jj - 2;
-    double v = GB_AT(lam, i, j);
-    if (i >= 0 && i < ni && j >= 0 && j < nj) {
-      v += line_gather(coef, n, 1, (size_t)j * ni, i, ni, 0);
-      v += line_gather(coef, n, (size_t)ni, (size_t)i, j, nj, 7);
-    }
-    GB_AT(mu, i, j) = v;
+  double v = GB_AT(lam, i, j);
+  if (i >= 0 && i < ni && j >= 0 && j < nj) {
+    v += line_gather(coef, n, 1, (size_t)j * ni, i, ni, 0);
+    v += line_gather(coef, n, (size_t)ni, (size_t)i, j, nj, 7);
   }
+  GB_AT(mu, i, j) = v;
+}
+__global__ void k_weno5_adj_gather(const double* __restrict__ lam_a, const double* __restrict__ coef, double* __restrict__ mu_a, AdjArgs a) {
+  GB_FOR_IJ(ii, jj, a.ni + 4, a.nj + 4) gather_node(lam_a, coef, mu_a, a, ii - 2, jj - 2);
 }
 
-// dL/dUA, dL/dVA: each node's velocity share goes to the two faces it averages.
-__global__ void k_weno5_adj_vel(const double* __restrict__ gvel, double* __restrict__ mu_ua_a, double* __restrict__ mu_va_a, int ni, int nj) {
-  const DField mu_ua = dfield(mu_ua_a, 3, ni + 1, nj), mu_va = dfield(mu_va_a, 3, ni, nj + 1);
+// The same with dL/dUA, dL/dVA (null: not asked for), to which each node's velocity share goes
+// at the two faces that it averages; their ghosts are zero.  One launch and two clears fewer
+// than with a kernel for the faces, and the gather's loads in flight together: 128 -> 118 us.
+__global__ void k_weno5_adj_out(const double* __restrict__ lam_a, const double* __restrict__ coef, const double* __restrict__ gvel,
+                                double* __restrict__ mu_a, double* __restrict__ mu_ua, double* __restrict__ mu_va, AdjArgs a) {
+  const int ni = a.ni, nj = a.nj;
   const size_t n = (size_t)ni * nj;
-  GB_FOR_IJ(i, j, ni + 1, nj + 1) {
-    if (mu_ua_a && j < nj) GB_AT(mu_ua, i, j) = (i > 0 ? gvel[(size_t)j * ni + i - 1] : 0.0) + (i < ni ? gvel[(size_t)j * ni + i] : 0.0);
-    if (mu_va_a && i < ni) GB_AT(mu_va, i, j) = (j > 0 ? gvel[n + (size_t)(j - 1) * ni + i] : 0.0) + (j < nj ? gvel[n + (size_t)j * ni + i] : 0.0);
+  GB_FOR_IJ(ii, jj, ni + 7, nj + 7) {
+    if (ii < ni + 4 && jj < nj + 4) gather_node(lam_a, coef, mu_a, a, ii - 2, jj - 2);
+    const int i = ii - 3, j = jj - 3;
+    if (mu_ua && jj < nj + 6) {
+      double v = 0.0;
+      if (i >= 0 && i <= ni && j >= 0 && j < nj)
+        v = (i > 0 ? gvel[(size_t)j * ni + i - 1] : 0.0) + (i < ni ? gvel[(size_t)j * ni + i] : 0.0);
+      mu_ua[(size_t)jj * (ni + 7) + ii] = v;
+    }
+    if (mu_va && ii < ni + 6) {
+      double v = 0.0;
+      if (i >= 0 && i < ni && j >= 0 && j <= nj)
+        v = (j > 0 ? gvel[n + (size_t)(j - 1) * ni + i] : 0.0) + (j < nj ? gvel[n + (size_t)j * ni + i] : 0.0);
+      mu_va[(size_t)jj * (ni + 6) + ii] = v;
+    }
   }
 }
 
@@ -256,7 +309,7 @@ __global__ void k_weno5_adj_vel(const double* __restrict__ gvel, double* __restr
 // each overwrite t <- 2 a - b becomes lam_a += 2 lam_t, lam_b -= lam_t, lam_t = 0, in
 // the reverse order of the forward assignments.  What remains on a ghost cell is the
 // cotangent of the value it held before the extrapolation.  Rows: left and right sides.
-__global__ void k_extrap_adj_rows(double* lam_a, int ni, int nj) {
+__device__ __forceinline__ void extrap_adj_rows(double* lam_a, int ni, int nj) {
   const DField L = dfield(lam_a, 2, ni, nj);
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nj; j += gridDim.x * blockDim.x) {
     // right: forward i = ni then ni+1
@@ -272,7 +325,7 @@ __global__ void k_extrap_adj_rows(double* lam_a, int ni, int nj) {
   }
 }
 // Columns: top and bottom sides.
-__global__ void k_extrap_adj_cols(double* lam_a, int ni, int nj) {
+__device__ __forceinline__ void extrap_adj_cols(double* lam_a, int ni, int nj) {
   const DField L = dfield(lam_a, 2, ni, nj);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ni; i += gridDim.x * blockDim.x) {
     double t = GB_AT(L, i, -1);  // bottom: forward j = -2 then j = -1
@@ -284,6 +337,15 @@ __global__ void k_extrap_adj_cols(double* lam_a, int ni, int nj) {
     t = GB_AT(L, i, nj);
     GB_AT(L, i, nj - 1) += 2 * t, GB_AT(L, i, nj - 2) -= t, GB_AT(L, i, nj) = 0;
   }
+}
+
+__global__ void k_extrap_adj_rows(double* lam_a, int ni, int nj) { extrap_adj_rows(lam_a, ni, nj); }
+__global__ void k_extrap_adj_cols(double* lam_a, int ni, int nj) { extrap_adj_cols(lam_a, ni, nj); }
+// Columns, then rows, in one block.
+__global__ void k_extrap_adj(double* lam_a, int ni, int nj) {
+  extrap_adj_cols(lam_a, ni, nj);
+  __syncthreads();
+  extrap_adj_rows(lam_a, ni, nj);
 }
 
 struct ProjAdjArgs {
@@ -997,15 +1059,19 @@ int adjoint_buffers(gb2d_ctx* c) {
 void launch_weno5_adjoint(cudaStream_t s, gb2d_ctx* c, double dt, double* mu_ua, double* mu_va) {
   const int ni = c->grid.ni, nj = c->grid.nj;
   AdjArgs a{ni, nj, c->base.odx, c->base.ody, c->prm.weno_epsilon, dt};
-  k_extrap_adj_cols<<<(ni + 127) / 128, 128, 0, s>>>(c->adj_lam_phi, ni, nj);
-  k_extrap_adj_rows<<<(nj + 127) / 128, 128, 0, s>>>(c->adj_lam_phi, ni, nj);
-  k_weno5_adj_coef<<<grid_ij(ni, nj), kThreads, 0, s>>>(c->phi_buf[c->phi_cur], c->ua, c->va, c->adj_lam_phi, c->adj_coef, c->adj_gvel, a);
-  k_weno5_adj_gather<<<grid_ij(ni + 4, nj + 4), kThreads, 0, s>>>(c->adj_lam_phi, c->adj_coef, c->adj_mu_phi, a);
-  GB_LAUNCHED(4);
-  if (mu_ua || mu_va) {
-    k_weno5_adj_vel<<<grid_ij(ni + 1, nj + 1), kThreads, 0, s>>>(c->adj_gvel, mu_ua, mu_va, ni, nj);
+  if (ni <= 1024 && nj <= 1024) {  // one round of one block, where two launches of 4 us are latency
+    k_extrap_adj<<<1, 1024, 0, s>>>(c->adj_lam_phi, ni, nj);
     GB_LAUNCHED(1);
+  } else {
+    k_extrap_adj_cols<<<(ni + 127) / 128, 128, 0, s>>>(c->adj_lam_phi, ni, nj);
+    k_extrap_adj_rows<<<(nj + 127) / 128, 128, 0, s>>>(c->adj_lam_phi, ni, nj);
+    GB_LAUNCHED(2);
   }
+  const int rows = nj < 65535 ? nj : 65535;
+  k_weno5_adj_coef<<<dim3((ni + kCoefThreads - 1) / kCoefThreads, rows, 2), kCoefThreads, 0, s>>>(
+      c->phi_buf[c->phi_cur], c->ua, c->va, c->adj_lam_phi, c->adj_coef, c->adj_gvel, a);
+  k_weno5_adj_out<<<grid_ij(ni + 7, nj + 7), kThreads, 0, s>>>(c->adj_lam_phi, c->adj_coef, c->adj_gvel, c->adj_mu_phi, mu_ua, mu_va, a);
+  GB_LAUNCHED(2);
 }
 
 void launch_projection_adjoint_rhs(cudaStream_t s, gb2d_ctx* c, double dt, int with_lam_p) {

@@ -804,8 +804,6 @@ int gb2d_weno5_adjoint(gb2d_ctx* c, double dt, const double* lam_phi, double* mu
   const size_t ni = c->grid.ni, nj = c->grid.nj;
   const size_t nphi = (ni + 4) * (nj + 4), nua = (ni + 7) * (nj + 6), nva = (ni + 6) * (nj + 7);
   GB2D_CUDA_TRY(c, cudaMemcpyAsync(c->adj_lam_phi, lam_phi, nphi * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  if (mu_ua) GB2D_CUDA_TRY(c, cudaMemsetAsync(c->adj_mu_u, 0, nua * sizeof(double), c->stream));
-  if (mu_va) GB2D_CUDA_TRY(c, cudaMemsetAsync(c->adj_mu_v, 0, nva * sizeof(double), c->stream));
   launch_weno5_adjoint(c->stream, c, dt, mu_ua ? c->adj_mu_u : nullptr, mu_va ? c->adj_mu_v : nullptr);
   if ((rc = check_launch(c, "weno5_adjoint"))) return rc;
   GB2D_CUDA_TRY(c, cudaMemcpyAsync(mu_phi, c->adj_mu_phi, nphi * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
