@@ -1231,11 +1231,13 @@ __global__ void k_end_device(const Scalars* sc, Scalars* fs, int last) {
 // barriers an iteration (residual; the V-cycle's two and r.z; direction; p.Ap), no host.
 // Every number equals the launched kernels': their blocks of 256 threads become the
 // halves of a CTA, with the same elements, the same sums and the same order of partials.
-// Vectors that another CTA wrote are read through L2 (__ldcg). Every CTA computes the same
-// scalars from the same partials, so that all take the same branches; at most max_it
-// iterations.  Measured: the mixed projection at 64^2 0.60 -> 0.49 ms, an iteration 34 -> 19
-// us (the V-cycle 9 of them); a bubble frame at 128^2 (FP64) 3.70 -> 3.65 ms, whose
-// V-cycles are bound by 16 SMs' FP64 pipes.
+// Vectors that another CTA wrote are read through L2 (__ldcg); the partials of the sums go
+// into every CTA's shared memory (64^2: 0.503 -> 0.480 ms against partials in global memory
+// and FP64 divisions).  Every CTA computes the same scalars from the same partials, so that
+// all take the same branches; at most max_it iterations.  Measured: the mixed projection at
+// 64^2 0.60 -> 0.48 ms, an iteration 34 -> 19 us (the V-cycle half of them); a bubble frame at
+// 128^2 (FP64) 3.70 -> 3.62 ms, whose V-cycles are bound by 16 SMs' FP64 pipes.
+constexpr int kCgBlocks = 64;  // 128^2 cells
 template <typename T>
 struct CgArgs {
   CtArgs<T> a;
@@ -1243,8 +1245,7 @@ struct CgArgs {
   double *x, *r, *p, *ap;
   T* rT;
   const double* ainv;
-  double *part_rr, *part_pap;
-  int G, nu;      // virtual blocks
+  int G, nu;      // virtual blocks (at most kCgBlocks)
   Scalars* sc;    // thr2, max_it in; iters, rr, flag out
   int* done;      // nonzero: nothing to do
   double* host;   // [0] ||r||^2, [1] iterations
@@ -1280,18 +1281,26 @@ __device__ __forceinline__ double half_sum_df(DF v, bool active, double* scratch
   x = warp_sum_df(x);
   return widen(x.hi) + widen(x.lo);
 }
+// A virtual block's partial, in the first lane of its half's first warp, to every CTA.
+__device__ __forceinline__ void cluster_share(double blk, double* part, int vb, int G, int P) {
+  const int vt = (int)threadIdx.x & (kThreads - 1);
+  if (vt >= 32 || vb >= G) return;
+  blk = __shfl_sync(0xffffffffu, blk, 0);
+  if (vt < P) *cgx::this_cluster().map_shared_rank(part + vb, vt) = blk;
+}
 // sum_partials by a block of 256 threads; valid in the first warp.
 __device__ __forceinline__ double cluster_total(const double* part, int G, double* scratch) {
   const int t = (int)threadIdx.x;
-  double v = 0.0;
   if (G <= 32) {  // one warp's sum, to which the other warps' zeros add nothing
-    if (t < G) v = __ldcg(part + t);
+    const double v = t < G ? part[t] : 0.0;
     return t < 32 ? warp_sum(v) : 0.0;
   }
-  if (t < kThreads)
-    for (int k = t; k < G; k += kThreads) v += __ldcg(part + k);
-  return half_sum(v, t < G && t < kThreads, scratch);
+  return half_sum(t < G ? part[t] : 0.0, t < G, scratch);
 }
+// a / b, correctly rounded: on the integer pipes where both are positive and far from the
+// ends of the range (one thread's chain of FP64 operations is twice as long).
+__device__ __forceinline__ bool mid_positive(double x) { return (uint32_t)(dbits(x) >> 32) - ((1023u - 500u) << 20) < (1000u << 20); }
+__device__ __forceinline__ double quotient(double a, double b) { return mid_positive(a) && mid_positive(b) ? div_pos(a, b) : a / b; }
 
 template <typename T, int K>
 __global__ void __launch_bounds__(kCtThreads, 1) k_cg_cluster(const __grid_constant__ CgArgs<T> g) {
@@ -1300,7 +1309,7 @@ __global__ void __launch_bounds__(kCtThreads, 1) k_cg_cluster(const __grid_const
   const int P = (int)cl.num_blocks(), c = (int)cl.block_rank(), tid = (int)threadIdx.x;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
-  __shared__ double rz_part[kClusterMax], scratch[16], s_rz, s_scalar;
+  __shared__ double rz_part[kClusterMax], scratch[16], s_rz, s_scalar, part_rr[kCgBlocks], part_pap[kCgBlocks];
   const CtArgs<T>& a = g.a;
   const Level<double>& L = g.L;
   if (*g.done) return;  // uniform over the cluster
@@ -1344,11 +1353,11 @@ __global__ void __launch_bounds__(kCtThreads, 1) k_cg_cluster(const __grid_const
           blk = half_sum_df(DF{acc.s, -acc.c}, any, scratch);
         else
           blk = half_sum(acc.s, any, scratch);
-        if (vt == 0 && vb < G) g.part_rr[vb] = blk;
+        cluster_share(blk, part_rr, vb, G, P);
       }
       cl.sync();
       {
-        const double total = cluster_total(g.part_rr, G, scratch);
+        const double total = cluster_total(part_rr, G, scratch);
         if (tid == 0) s_scalar = total;
         __syncthreads();
         rr = s_scalar;
@@ -1372,7 +1381,7 @@ __global__ void __launch_bounds__(kCtThreads, 1) k_cg_cluster(const __grid_const
       double rz = 0.0;
       for (int o = 0; o < P; ++o) rz += rz_part[o];
       s_rz = rz;
-      s_scalar = it == 0 ? 0.0 : rz / rz_cur;  // in one thread: 512 would hold up the FP64 pipe
+      s_scalar = it == 0 ? 0.0 : quotient(rz, rz_cur);  // in one thread: 512 would hold up the FP64 pipe
     }
     __syncthreads();
     const double rz = s_rz, bt = s_scalar;
@@ -1430,12 +1439,12 @@ __global__ void __launch_bounds__(kCtThreads, 1) k_cg_cluster(const __grid_const
       } else {
         blk = half_sum(acc, any, scratch);
       }
-      if (vt == 0 && vb < G) g.part_pap[vb] = blk;
+      cluster_share(blk, part_pap, vb, G, P);
     }
     cl.sync();
     {
-      const double total = cluster_total(g.part_pap, G, scratch);
-      if (tid == 0) s_scalar = rz / total;
+      const double total = cluster_total(part_pap, G, scratch);
+      if (tid == 0) s_scalar = quotient(rz, total);
       __syncthreads();
       alpha = s_scalar;
     }
@@ -1806,7 +1815,7 @@ bool cluster_cg(const Hierarchy<T>& H, int use_mg) {
     const char* e = getenv("GB2D_CLUSTER_CG");
     return e && e[0] == '0';
   }();
-  return use_mg && H.ctail == 0 && !off;
+  return use_mg && H.ctail == 0 && (long)H.L[0].nI * H.L[0].nJ <= (long)kCgBlocks * kThreads && !off;
 }
 // Runs the CG from the state that k_begin_loop or k_begin_device set.
 template <typename T>
@@ -1821,8 +1830,6 @@ void launch_cg_cluster(cudaStream_t s, Solver* S, const Hierarchy<T>& H, const d
   g.ap = S->ap;
   g.rT = sizeof(T) == 4 ? H.r : nullptr;
   g.ainv = ainv;
-  g.part_rr = slot(S, kSlotRr);
-  g.part_pap = slot(S, kSlotPap);
   g.G = S->G;
   g.nu = nu;
   g.sc = S->sc;
