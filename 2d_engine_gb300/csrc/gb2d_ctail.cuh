@@ -1,7 +1,7 @@
 // gb2d_ctail.cuh — the coarse end of the V-cycle as ONE thread-block cluster.
 //
 // Included by gb2d_solver.cu inside its anonymous namespace (uses Level, Scalars,
-// gs_update, warp_sum, reduce_scratch, publish_rz, kMaxLevels, kCoarseMax).
+// gs_sum, gs_residual, warp_sum, reduce_scratch, publish_rz, kMaxLevels, kCoarseMax).
 //
 // Every level from the cluster's top level (at most 128^2 cells) down to the dense
 // coarse solve runs inside one launch of a cluster of P CTAs, each CTA one SM with 512
@@ -191,8 +191,9 @@ __device__ __forceinline__ void ct_half(T* xp, int xplane, int ps, CtRegs<T, K>&
     }
     const bool right = (g.od[k] != 0) == (COLOR == 0);  // the cell is the pair's right one
     const T own = g.x[1 - COLOR][k], side = xo[right ? ad + 1 : ad - 1], xb = xo[ad - ps], xt = xo[ad + ps];
-    const T v = gs_update(g.b[COLOR][k], g.cl[COLOR][k], right ? own : side, g.cr[COLOR][k], right ? side : own, g.y0[COLOR][k], xb,
-                          g.y1[COLOR][k], xt, g.idg[COLOR][k]);
+    const T v = mulr(gs_sum(g.b[COLOR][k], g.cl[COLOR][k], right ? own : side, g.cr[COLOR][k], right ? side : own, g.y0[COLOR][k], xb,
+                            g.y1[COLOR][k], xt),
+                     g.idg[COLOR][k]);
     g.x[COLOR][k] = v;
     xw[ad] = v;
   }
