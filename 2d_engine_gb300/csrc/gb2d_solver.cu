@@ -18,12 +18,13 @@
 // shared memory, the red and black half sweeps run back to back, halo cells are
 // recomputed redundantly); the pre-smoothing launch also forms the residual and
 // restricts it, the post-smoothing launch also prolongs the coarse correction.
-// The levels from 128^2 down run in one launch of a 16-CTA thread-block cluster
-// (gb2d_ctail.cuh), neighbour rows read from the other CTAs' shared memory; a
-// single-CTA kernel over the levels from 64^2 down is the fallback.  One CG
-// iteration adds three FP64 kernels (direction, operator product with p.Ap,
-// update with r.r), and each iteration is replayed from a CUDA graph whose
-// kernels use programmatic dependent launch.  The loop around the CG recomputes
+// The levels from 128^2 (or 64^2) down run in one launch of a thread-block cluster
+// of up to 16 CTAs (gb2d_ctail.cuh), each working on a stripe of rows and the halo
+// that one side of smoothing uses up; a single-CTA kernel over the levels from 64^2
+// down is the fallback.  One CG iteration adds three FP64 kernels (direction, operator
+// product with p.Ap, update with r.r), and each iteration is replayed from a CUDA
+// graph whose kernels use programmatic dependent launch; where the cluster holds the
+// finest level, one launch runs the whole CG in it.  The loop around the CG recomputes
 // the true FP64 residual and restarts only if the recursive residual drifted.
 //
 // All reductions are two-stage and deterministic: blocks write partial sums,
