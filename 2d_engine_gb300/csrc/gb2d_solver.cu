@@ -963,25 +963,30 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(TailArgs<T> a, const doub
        k < k##_end; k += (size_t)gridDim.x * blockDim.x)
 
 // r = b - A x with the reference's matrix entries, in FP64; its copy for the
-// preconditioner (rT, FP32 or the FP64 r itself); partial ||r||^2 and ||b||^2.
-template <typename T>
+// preconditioner (rT, FP32 or the FP64 r itself); partial ||r||^2 and, on a solve's first
+// pass (BB), ||b||^2, whose partials stay for the later ones.  The FP64 pipe bounds it (eight
+// operations a cell with ||b||^2): one product runs on the integer pipes.  2048^2: 64 us, 74
+// before.
+template <typename T, bool BB>
 __global__ void k_residual64(Level<double> L, const double* __restrict__ x, const double* __restrict__ b, double* __restrict__ r64,
                              T* __restrict__ rT, double* __restrict__ part_rr, double* __restrict__ part_bb) {
   double rr = 0.0, bb = 0.0;
   GB_FLAT_FOR(L, k) {
-    double ax = L.dg[k] * x[k] - L.cx[k] * x[k - 1] - L.cx[k + 1] * x[k + 1] - L.cy[k] * x[k - L.ld] - L.cy[k + L.ld] * x[k + L.ld];
-    double r = b[k] - ax;
+    const double bk = b[k];
+    const double ax = __fma_rn(
+        -L.cy[k + L.ld], x[k + L.ld],
+        __fma_rn(-L.cy[k], x[k - L.ld], __fma_rn(-L.cx[k + 1], x[k + 1], __fma_rn(L.dg[k], x[k], -mul_idg(x[k - 1], L.cx[k])))));
+    const double r = bk - ax;
     r64[k] = r;
     if constexpr (sizeof(T) == 4) rT[k] = narrow(r);
-    rr += r * r;
-    bb += b[k] * b[k];
+    rr = __fma_rn(r, r, rr);
+    if (BB) bb = __fma_rn(bk, bk, bb);
   }
   rr = block_sum(rr);
+  if (threadIdx.x == 0) part_rr[blockIdx.x] = rr;
+  if (!BB) return;
   bb = block_sum(bb);
-  if (threadIdx.x == 0) {
-    part_rr[blockIdx.x] = rr;
-    part_bb[blockIdx.x] = bb;
-  }
+  if (threadIdx.x == 0) part_bb[blockIdx.x] = bb;
 }
 
 __global__ void k_reduce_two(const double* __restrict__ pa, const double* __restrict__ pb, int nparts, double* out) {
@@ -2612,6 +2617,17 @@ bool append_cg_loop(cudaStream_t s, cudaStream_t body, cudaGraphConditionalHandl
   return cudaStreamEndCapture(body, &out) == cudaSuccess;
 }
 
+// The true residual of x; first: with ||b||^2.
+inline void launch_residual(cudaStream_t s, Solver* S, bool mixed, const double* x, bool first) {
+  const auto k32 = first ? k_residual64<float, true> : k_residual64<float, false>;
+  const auto k64 = first ? k_residual64<double, true> : k_residual64<double, false>;
+  if (mixed)
+    k32<<<S->G, kThreads, 0, s>>>(S->h64.L[0], x, S->b64, S->h64.r, S->h32.r, slot(S, kSlotRr), slot(S, kSlotBb));
+  else
+    k64<<<S->G, kThreads, 0, s>>>(S->h64.L[0], x, S->b64, S->h64.r, nullptr, slot(S, kSlotRr), slot(S, kSlotBb));
+  GB_LAUNCHED(1);
+}
+
 // The solve of a device-driven frame (ctx->graph_mode, captured on ctx->stream): the true
 // residual and ||b||^2 into the frame scalars, then two passes of [threshold and done flag
 // on the device, CG init, WHILE over one iteration, true residual] -- the host loop's first
@@ -2625,15 +2641,12 @@ int solve_on_device(gb2d_ctx* c, Solver* S, Hierarchy<T>& H, const double* ainv,
   double* P_rr = slot(S, kSlotRr);
   double* P_bb = slot(S, kSlotBb);
   const bool mixed = sizeof(T) == 4;
-  auto residual = [&]() {
-    if (mixed)
-      k_residual64<float><<<G, kThreads, 0, s>>>(S->h64.L[0], x, S->b64, S->h64.r, S->h32.r, P_rr, P_bb);
-    else
-      k_residual64<double><<<G, kThreads, 0, s>>>(S->h64.L[0], x, S->b64, S->h64.r, nullptr, P_rr, P_bb);
+  auto residual = [&](bool first) {
+    launch_residual(s, S, mixed, x, first);
     k_reduce_two<<<1, kThreads, 0, s>>>(P_rr, P_bb, G, &c->sc->g_rr);
-    GB_LAUNCHED(2);
+    GB_LAUNCHED(1);
   };
-  residual();
+  residual(true);
   if (!joined) cudaStreamWaitEvent(s, join_ev, 0);
   cudaMemsetAsync(&S->sc->flag, 0, sizeof(int), s);
   const bool in_cluster = cluster_cg(H, use_mg);  // one kernel instead of the loop node
@@ -2642,7 +2655,7 @@ int solve_on_device(gb2d_ctx* c, Solver* S, Hierarchy<T>& H, const double* ainv,
     if (in_cluster) {
       k_begin_device<<<1, 1, 0, s>>>(cudaGraphConditionalHandle(), 0, S->sc, S->done, c->sc, tol * tol, max_it, pass == 0);
       launch_cg_cluster<T>(s, S, H, ainv, x, nu);
-      residual();
+      residual(false);
       k_end_device<<<1, 1, 0, s>>>(S->sc, c->sc, pass == 1);
       GB_LAUNCHED(2);
       continue;
@@ -2667,7 +2680,7 @@ int solve_on_device(gb2d_ctx* c, Solver* S, Hierarchy<T>& H, const double* ainv,
       snprintf(c->err, sizeof(c->err), "device-driven solve: the CG loop node was refused");
       return GB2D_ERR_CUDA;
     }
-    residual();
+    residual(false);
     k_end_device<<<1, 1, 0, s>>>(S->sc, c->sc, pass == 1);
     GB_LAUNCHED(1);
   }
@@ -2744,12 +2757,10 @@ int solver_solve(gb2d_ctx* c, const double* /*rhs*/, double* x, const gb2d_solve
   int total = 0, outer = 0;
   double rr = 0, bb = 0;
   int status = GB2D_OK;
+  bool first = true;
   auto residual = [&]() {
-    if (prec)
-      k_residual64<float><<<G, kThreads, 0, s>>>(S->h64.L[0], x, S->b64, S->h64.r, S->h32.r, P_rr, P_bb);
-    else
-      k_residual64<double><<<G, kThreads, 0, s>>>(S->h64.L[0], x, S->b64, S->h64.r, nullptr, P_rr, P_bb);
-    GB_LAUNCHED(1);
+    launch_residual(s, S, prec != 0, x, first);
+    first = false;
   };
   auto join = [&]() {
     if (!joined) cudaStreamWaitEvent(s, join_ev, 0);
