@@ -1068,9 +1068,12 @@ __global__ void k_direction(Level<double> L, const TZ* __restrict__ z, double* _
 
 // One row of A p and the two vector updates, every rounding stated (the cluster CG below
 // performs the same operations).
+// INT: the first product on the integer pipes.
+template <bool INT = false>
 __device__ __forceinline__ double ap_row(double dg, double pc, double cxl, double pl, double cxr, double pr, double cyb, double pb,
                                          double cyt, double pt) {
-  return __fma_rn(-cyt, pt, __fma_rn(-cyb, pb, __fma_rn(-cxr, pr, __fma_rn(dg, pc, -__dmul_rn(cxl, pl)))));
+  const double m = INT ? mul_idg(pl, cxl) : __dmul_rn(cxl, pl);
+  return __fma_rn(-cyt, pt, __fma_rn(-cyb, pb, __fma_rn(-cxr, pr, __fma_rn(dg, pc, -m))));
 }
 // A thread's partial of ||r||^2: r r added to acc.
 __device__ __forceinline__ void add_square(Acc<float>& acc, float f) { acc.add(f * f); }
@@ -1082,8 +1085,11 @@ __device__ __forceinline__ void add_square(Acc<double>& acc, double r) { acc.s =
 // preconditioner (TZ = float, whose r.z and ||r||^2 are FP32 sums already) each
 // thread's FP64 partial is split into two FP32 words (one FP64 subtraction) and
 // the block sum runs in double-float on the FP32 pipe; with the FP64 one the
-// block sum stays FP64.
-template <typename TZ>
+// block sum stays FP64.  INT (grids of 2^21 cells and more under the FP32 preconditioner):
+// one of the six operations a cell moves off the FP64 pipe, which bounds the kernel there
+// (2048^2 frame 12.13 -> 12.00 ms; 1024^2 the same; FP64 511 x 385, whose blocks are short
+// of warps, 2.546 -> 2.572 ms).
+template <typename TZ, bool INT>
 __global__ void k_apply_pap(Level<double> L, const double* __restrict__ p, double* __restrict__ ap, Scalars* sc, double* __restrict__ part,
                             unsigned* __restrict__ counter, const int* __restrict__ done) {
   pdl_enter();
@@ -1095,8 +1101,8 @@ __global__ void k_apply_pap(Level<double> L, const double* __restrict__ p, doubl
       const double2 pc = ld2(p, k), pb = ld2(p, k - ld), pt = ld2(p, k + ld);
       const double2 dg = ld2(L.dg, k), cx = ld2(L.cx, k), cy = ld2(L.cy, k), cyt = ld2(L.cy, k + ld);
       const double pl = p[k - 1], pr = p[k + 2], cx2 = L.cx[k + 2];
-      const double y0 = ap_row(dg.x, pc.x, cx.x, pl, cx.y, pc.y, cy.x, pb.x, cyt.x, pt.x);
-      const double y1 = ap_row(dg.y, pc.y, cx.y, pc.x, cx2, pr, cy.y, pb.y, cyt.y, pt.y);
+      const double y0 = ap_row<INT>(dg.x, pc.x, cx.x, pl, cx.y, pc.y, cy.x, pb.x, cyt.x, pt.x);
+      const double y1 = ap_row<INT>(dg.y, pc.y, cx.y, pc.x, cx2, pr, cy.y, pb.y, cyt.y, pt.y);
       st2(ap, k, y0, y1);
       acc = __fma_rn(pc.x, y0, acc);
       acc = __fma_rn(pc.y, y1, acc);
@@ -1104,7 +1110,7 @@ __global__ void k_apply_pap(Level<double> L, const double* __restrict__ p, doubl
   } else {
     GB_FLAT_FOR(L, k) {
       const double pc = p[k];
-      const double y = ap_row(L.dg[k], pc, L.cx[k], p[k - 1], L.cx[k + 1], p[k + 1], L.cy[k], p[k - L.ld], L.cy[k + L.ld], p[k + L.ld]);
+      const double y = ap_row<INT>(L.dg[k], pc, L.cx[k], p[k - 1], L.cx[k + 1], p[k + 1], L.cy[k], p[k - L.ld], L.cy[k + L.ld], p[k + L.ld]);
       ap[k] = y;
       acc = __fma_rn(pc, y, acc);
     }
@@ -2126,13 +2132,18 @@ void precondition(cudaStream_t s, Solver* S, Hierarchy<T>& H, const double* ainv
   }
 }
 
+template <typename T>
+auto apply_kernel(const Solver* S) {
+  return sizeof(T) == 4 && (long)S->ni * S->nj >= (1L << 21) ? k_apply_pap<T, sizeof(T) == 4> : k_apply_pap<T, false>;
+}
+
 // First direction: z = M r, p = z, Ap, alpha.
 template <typename T>
 void enqueue_init(cudaStream_t s, Solver* S, Hierarchy<T>& H, const double* ainv, int use_mg, int nu, Probe* pr) {
   const Level<double>& L = S->h64.L[0];
   precondition<T>(s, S, H, ainv, use_mg, nu, pr);
   pdl_launch(s, dim3(S->G), dim3(kThreads), 0, k_direction<T>, L, (const T*)H.L[0].x, S->p, (const Scalars*)S->sc, 1, (const int*)S->done);
-  pdl_launch(s, dim3(S->G), dim3(kThreads), 0, k_apply_pap<T>, L, (const double*)S->p, S->ap, S->sc, slot(S, kSlotPap), S->counter,
+  pdl_launch(s, dim3(S->G), dim3(kThreads), 0, apply_kernel<T>(S), L, (const double*)S->p, S->ap, S->sc, slot(S, kSlotPap), S->counter,
              (const int*)S->done);
   GB_LAUNCHED(2);
 }
@@ -2148,7 +2159,7 @@ void enqueue_iter(cudaStream_t s, Solver* S, Hierarchy<T>& H, const double* ainv
   GB_LAUNCHED(1);
   precondition<T>(s, S, H, ainv, use_mg, nu, pr);
   pdl_launch(s, dim3(S->G), dim3(kThreads), 0, k_direction<T>, L, (const T*)H.L[0].x, S->p, (const Scalars*)S->sc, 0, (const int*)S->done);
-  pdl_launch(s, dim3(S->G), dim3(kThreads), 0, k_apply_pap<T>, L, (const double*)S->p, S->ap, S->sc, slot(S, kSlotPap), S->counter,
+  pdl_launch(s, dim3(S->G), dim3(kThreads), 0, apply_kernel<T>(S), L, (const double*)S->p, S->ap, S->sc, slot(S, kSlotPap), S->counter,
              (const int*)S->done);
   GB_LAUNCHED(2);
 }
