@@ -1034,26 +1034,13 @@ int density_gradient(gb2d_ctx* c, double dt, double* d_water, double* d_air) {
 int adjoint_buffers(gb2d_ctx* c) {
   if (c->adj_coef) return GB2D_OK;
   const size_t ni = c->grid.ni, nj = c->grid.nj;
-  struct A {
-    double** p;
-    size_t n;
-  } allocs[] = {
-      {&c->adj_coef, 14 * ni * nj},           {&c->adj_gvel, 2 * ni * nj},
-      {&c->adj_lam_phi, (ni + 4) * (nj + 4)}, {&c->adj_mu_phi, (ni + 4) * (nj + 4)},
-      {&c->adj_lam_u, (ni + 5) * (nj + 4)},   {&c->adj_lam_v, (ni + 4) * (nj + 5)},
-      {&c->adj_mu_u, (ni + 7) * (nj + 6)},    {&c->adj_mu_v, (ni + 6) * (nj + 7)},
-      {&c->adj_lam_p, (ni + 2) * (nj + 2)},    {&c->adj_eno, 16 * ((ni + 1) * nj + ni * (nj + 1))},
-  };
-  for (auto& a : allocs) {
-    cudaError_t e = cudaMalloc(a.p, a.n * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemset(*a.p, 0, a.n * sizeof(double));
-    if (e != cudaSuccess) {
-      snprintf(c->err, sizeof(c->err), "adjoint buffers: %s", cudaGetErrorString(e));
-      return GB2D_ERR_CUDA;
-    }
-  }
-  // Cleared on the legacy stream, which the context's streams do not wait for.
-  return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? GB2D_OK : GB2D_ERR_CUDA;
+  auto buf = [](double*& p, size_t n) { return Buffer{(void**)&p, n * sizeof(double)}; };
+  return make_buffers(c, "adjoint buffers",
+                      {buf(c->adj_coef, 14 * ni * nj), buf(c->adj_gvel, 2 * ni * nj), buf(c->adj_lam_phi, (ni + 4) * (nj + 4)),
+                       buf(c->adj_mu_phi, (ni + 4) * (nj + 4)), buf(c->adj_lam_u, (ni + 5) * (nj + 4)),
+                       buf(c->adj_lam_v, (ni + 4) * (nj + 5)), buf(c->adj_mu_u, (ni + 7) * (nj + 6)),
+                       buf(c->adj_mu_v, (ni + 6) * (nj + 7)), buf(c->adj_lam_p, (ni + 2) * (nj + 2)),
+                       buf(c->adj_eno, 16 * ((ni + 1) * nj + ni * (nj + 1)))});
 }
 
 void launch_weno5_adjoint(cudaStream_t s, gb2d_ctx* c, double dt, double* mu_ua, double* mu_va) {

@@ -29,6 +29,24 @@ Space make_space(int ires, int jres, double x_min, double y_min, double x_max, d
   return s;
 }
 
+int make_buffers(gb2d_ctx* c, const char* what, std::initializer_list<Buffer> set) {
+  cudaError_t e = cudaSuccess;
+  for (const Buffer& b : set) {
+    if (e == cudaSuccess) e = cudaMalloc(b.p, b.bytes);
+    if (e == cudaSuccess) e = cudaMemset(*b.p, 0, b.bytes);
+  }
+  // Cleared on the legacy stream, which the context's streams do not wait for.
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+  if (e == cudaSuccess) return GB2D_OK;
+  snprintf(c->err, sizeof(c->err), "%s: %s", what, cudaGetErrorString(e));
+  for (const Buffer& b : set) {
+    if (*b.p) cudaFree(*b.p);
+    *b.p = nullptr;
+  }
+  cudaGetLastError();  // the next launch check is about its own launch
+  return GB2D_ERR_CUDA;
+}
+
 }  // namespace gb2d
 
 using namespace gb2d;
@@ -842,10 +860,7 @@ int gb2d_jump_poisson_solve(gb2d_ctx* c, const double* density, const int* bc, c
                             double* normal_y, const gb2d_solve_opts* o, gb2d_solve_stats* st) {
   if (!c || !density || !bc || !div || !levelset || !jc_solution || !jc_derivative || !pressure || !o) return GB2D_ERR_ARG;
   int rc = jump_buffers(c);
-  if (rc) {
-    snprintf(c->err, sizeof(c->err), "jump_poisson_solve: device allocation failed");
-    return rc;
-  }
+  if (rc) return rc;
   const size_t ni = c->grid.ni, nj = c->grid.nj, np = (ni + 2) * (nj + 2), nphi = (ni + 4) * (nj + 4);
   const cudaMemcpyKind h2d = cudaMemcpyHostToDevice;
   GB2D_CUDA_TRY(c, cudaMemcpyAsync(c->jmp_dens, density, np * sizeof(double), h2d, c->stream));

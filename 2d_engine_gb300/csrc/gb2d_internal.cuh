@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <initializer_list>
 #include <utility>
 
 #include "gb2d.h"
@@ -269,6 +270,14 @@ void launch_frame_dt(cudaStream_t s, gb2d_ctx* c, double cfl);
 int frame_capture(gb2d_ctx* c, double cfl, const gb2d_solve_opts* o);
 
 // ---- gb2d_adjoint.cu ----
+// Device buffers that a context makes on first use.  All of them, cleared, or none: on a
+// failure every pointer of the set is null again, so that any one of them says whether the
+// set stands, and a later call tries again.  Defined in gb2d_api.cu.
+struct Buffer {
+  void** p;
+  size_t bytes;
+};
+int make_buffers(gb2d_ctx* c, const char* what, std::initializer_list<Buffer> set);
 int adjoint_buffers(gb2d_ctx* c);
 // VJP of one level-set advection sweep at the current PHI, UA, VA: adj_lam_phi (consumed)
 // -> adj_mu_phi; velocity cotangents into mu_ua / mu_va (UA/VA layout) when non-null.

@@ -164,17 +164,10 @@ __global__ void k_jump_assemble(JumpIn in, double* __restrict__ bx, double* __re
 int jump_buffers(gb2d_ctx* c) {
   if (c->jmp_dens) return GB2D_OK;
   const size_t ni = c->grid.ni, nj = c->grid.nj, np = (ni + 2) * (nj + 2);
-  double** bufs[] = {&c->jmp_dens, &c->jmp_div, &c->jmp_js, &c->jmp_jd, &c->jmp_nx, &c->jmp_ny};
-  for (double** b : bufs) {
-    cudaError_t e = cudaMalloc(b, np * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemset(*b, 0, np * sizeof(double));
-    if (e != cudaSuccess) return GB2D_ERR_CUDA;
-  }
-  cudaError_t e = cudaMalloc(&c->jmp_phi, (ni + 4) * (nj + 4) * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&c->jmp_bc, np * sizeof(int));
-  // Cleared on the legacy stream, which the context's streams do not wait for.
-  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
-  return e == cudaSuccess ? GB2D_OK : GB2D_ERR_CUDA;
+  auto buf = [](double*& p, size_t n) { return Buffer{(void**)&p, n * sizeof(double)}; };
+  return make_buffers(c, "jump-Poisson buffers",
+                      {buf(c->jmp_dens, np), buf(c->jmp_div, np), buf(c->jmp_js, np), buf(c->jmp_jd, np), buf(c->jmp_nx, np),
+                       buf(c->jmp_ny, np), buf(c->jmp_phi, (ni + 4) * (nj + 4)), Buffer{(void**)&c->jmp_bc, np * sizeof(int)}});
 }
 
 void launch_jump_assemble(cudaStream_t s, gb2d_ctx* c) {
