@@ -94,6 +94,10 @@ void pdl_launch(cudaStream_t s, dim3 grid, dim3 block, size_t smem, void (*k)(P.
   cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
+// Iterations of one pass of a device-side CG loop: the caller's cap, and 2^20 in any case (a
+// kernel or graph launch cannot be left from the host; the host starts another pass).
+__host__ __device__ constexpr int pass_cap(int max_it) { return max_it < (1 << 20) ? max_it : 1 << 20; }
+
 // ---- level construction -----------------------------------------------------
 
 // Grid-stride loop over an nI x nJ index space on a 2D grid (x: columns, y:

@@ -1203,13 +1203,13 @@ __global__ void k_begin_loop(Scalars* sc, int* done, double thr2, int max_it) {
 // Last node of the loop body: counts the iteration, hands the count and the latest
 // ||r||^2 to the host, and continues the loop only while the run has not converged
 // and is under its cap.  It never returns early: every pass sets the condition, so the
-// loop ends after at most max_it passes (and after 1 << 20 in any case).
+// loop ends after at most pass_cap(max_it) passes.
 __global__ void k_loop_cond(cudaGraphConditionalHandle h, Scalars* sc, const int* __restrict__ done, double* host_out) {
   pdl_enter();
   const int n = ++sc->iters;
   host_out[0] = sc->rr;
   host_out[1] = (double)n;
-  const bool more = *done == 0 && n < sc->max_it && n < (1 << 20);
+  const bool more = *done == 0 && n < pass_cap(sc->max_it);
   cudaGraphSetConditional(h, more ? 1u : 0u);
 }
 
@@ -1266,7 +1266,7 @@ __global__ void k_end_device(const Scalars* sc, Scalars* fs, int last) {
 // Vectors that another CTA wrote are read through L2 (__ldcg); the partials of the sums go
 // into every CTA's shared memory (64^2: 0.503 -> 0.480 ms against partials in global memory
 // and FP64 divisions).  Every CTA computes the same scalars from the same partials, so that
-// all take the same branches; at most max_it iterations.  Measured: the mixed projection at
+// all take the same branches; at most pass_cap(max_it) iterations.  Measured: the mixed projection at
 // 64^2 0.60 -> 0.48 ms, an iteration 34 -> 19 us (the V-cycle half of them); a bubble frame at
 // 128^2 (FP64) 3.70 -> 3.62 ms, whose V-cycles are bound by 16 SMs' FP64 pipes.
 constexpr int kCgBlocks = 64;  // 128^2 cells
@@ -1348,7 +1348,7 @@ __global__ void __launch_bounds__(kCtThreads, 1) k_cg_cluster(const __grid_const
   const CtDense<T> dense = ct_dense_load(a, g.ainv, sm);
   for (int u = tid; u < a.zero_n; u += kCtThreads) sm[u] = (T)0;
   const double thr2 = g.sc->thr2;
-  const int max_it = g.sc->max_it, G = g.G;
+  const int max_it = pass_cap(g.sc->max_it), G = g.G;
   const size_t ld = L.ld, end = ld * (L.nJ + 1), pair_end = (end + 1) & ~(size_t)1;
   const int vt = tid & (kThreads - 1), vb0 = c + P * (tid / kThreads), rounds = (G + 2 * P - 1) / (2 * P);
   cl.sync();
