@@ -318,7 +318,9 @@ __global__ void __launch_bounds__(2 * kExX * kExY, 5) k_reinit_sweep_exact(const
   const bool in = i < a.ni && j < a.nj;
   const double s = in ? __ldg(&S[i + (size_t)j * a.ni]) : 0.0;
   const long long smag = mag_bits(s);
-  const bool sfast = smag >= ((1023LL - 100) << 52) && smag <= kInfBits;  // |s| >= 2^-100
+  // 2^-100 <= |s| < 2^100: S is the caller's in gb2d_reinit_sweep_apply, and mul_rn below takes
+  // finite operands whose product stays in the normal range (dtau is in [2^-331, 2^300], |h| below 2^106).
+  const bool sfast = smag >= ((1023LL - 100) << 52) && smag < ((1023LL + 100) << 52);
   int pick = in ? 3 : 2;
   if (in && fast && sfast) {
     float d[6];
