@@ -96,6 +96,7 @@ struct LSArgs {
   float odx_f, ody_f, eps_f;  // the same in FP32 for the FP32 flux path
   int fast_f;                 // FP32 epsilon is in mx_sign's range
   int fast;                   // epsilon is in weno5_side_fast's range (and dx in [2^-300, 2^300], for dtau s h)
+  int row0, rows;             // the launch's first tile row; tile rows of the grid (row `rows` copies the ghost ring)
 };
 
 // Reads phi's interior at (i, j), where positions outside it hold the second interior
@@ -194,11 +195,12 @@ __global__ void __launch_bounds__(2 * kExX* kExY) k_weno5_advect_exact(const dou
   __shared__ ExactTile t;
   __shared__ double vfy[NN];
   const DField src = dfield((double*)src_a, 2, a.ni, a.nj), dst = dfield(dst_a, 2, a.ni, a.nj);
-  if (blockIdx.y == gridDim.y - 1) {
+  const int by = a.row0 + (int)blockIdx.y;
+  if (by == a.rows) {
     copy_ring(src, dst, blockIdx.x * (2 * NN) + threadIdx.x, gridDim.x * (2 * NN));
     return;
   }
-  const int i0 = (int)blockIdx.x * kExX, j0 = (int)blockIdx.y * kExY;
+  const int i0 = (int)blockIdx.x * kExX, j0 = by * kExY;
   const bool fast = stage_exact(t, src, a, i0, j0);
   const int node = threadIdx.x & (NN - 1), dir = threadIdx.x / NN;
   const int c = node & (kExX - 1), r = node / kExX, i = i0 + c, j = j0 + r;
@@ -287,9 +289,9 @@ __device__ __forceinline__ int godunov_case(int ss, int sm, int sp) {
 // settle the signs almost everywhere; a thread evaluates the chosen side of one
 // direction of its node exactly, and the few that need both values (shocks, flat
 // directions) put the second evaluation on the block's list, which the block works
-// off densely.  The update has the bits of evaluating all four derivatives.  ring: the
-// grid's last block row copies src's ghost ring (needed until both buffers of the
-// sweeps hold it).
+// off densely.  The update has the bits of evaluating all four derivatives.  A block row
+// after the tiles', where the launch has one, copies src's ghost ring (needed until both
+// buffers of the sweeps hold it).
 // One level-set TVD-RK3 with its 75 sweeps at 512^2: 22.6 ms with four derivatives per
 // node in FP64 divisions and products (578 FP64 instructions per node), 6.4 ms with the
 // chosen sides, the differences shared and the divisions on the integer pipes (160), 3.5
@@ -298,7 +300,7 @@ __device__ __forceinline__ int godunov_case(int ss, int sm, int sp) {
 // 3.97.  Tiles of 32 x 8 nodes are 3% slower, and 1.3 times as slow on small grids, where
 // they leave SMs idle; 32 x 2 ones are no faster there.
 __global__ void __launch_bounds__(2 * kExX * kExY, 5) k_reinit_sweep_exact(const double* __restrict__ src_a, double* __restrict__ dst_a,
-                                                                     const double* __restrict__ S, LSArgs a, double dtau, int ring) {
+                                                                     const double* __restrict__ S, LSArgs a, double dtau) {
   pdl_enter();
   constexpr int NN = kExX * kExY, NT = 2 * NN;  // nodes and threads: thread dir NN + node
   __shared__ ExactTile t;
@@ -307,11 +309,12 @@ __global__ void __launch_bounds__(2 * kExX * kExY, 5) k_reinit_sweep_exact(const
   __shared__ signed char dy_pick[NN];
   __shared__ int count;
   const DField src = dfield((double*)src_a, 2, a.ni, a.nj), dst = dfield(dst_a, 2, a.ni, a.nj);
-  if (ring && blockIdx.y == gridDim.y - 1) {
+  const int by = a.row0 + (int)blockIdx.y;
+  if (by == a.rows) {
     copy_ring(src, dst, blockIdx.x * NT + threadIdx.x, gridDim.x * NT);
     return;
   }
-  const int tid = threadIdx.x, i0 = (int)blockIdx.x * kExX, j0 = (int)blockIdx.y * kExY;
+  const int tid = threadIdx.x, i0 = (int)blockIdx.x * kExX, j0 = by * kExY;
   if (tid == 0) count = 0;
   const bool fast = stage_exact(t, src, a, i0, j0);
   const int node = tid & (NN - 1), dir = tid / NN, c = node & (kExX - 1), r = node / kExX, i = i0 + c, j = j0 + r;
@@ -461,11 +464,12 @@ __global__ void __launch_bounds__(kMxX* kMxY, 8) k_weno5_advect_mixed(const doub
   __shared__ MixedTile t;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const DField src = dfield((double*)src_a, 2, a.ni, a.nj), dst = dfield(dst_a, 2, a.ni, a.nj);
-  if (blockIdx.y == gridDim.y - 1) {
+  const int by = a.row0 + (int)blockIdx.y;
+  if (by == a.rows) {
     copy_ring(src, dst, blockIdx.x * NT + ty * kMxX + tx, gridDim.x * NT);
     return;
   }
-  const int i0 = (int)blockIdx.x * kMxX, j0 = (int)blockIdx.y * kMxY, i = i0 + tx, j = j0 + ty;
+  const int i0 = (int)blockIdx.x * kMxX, j0 = by * kMxY, i = i0 + tx, j = j0 + ty;
   const bool fast = stage_mixed(t, src, a, i0, j0);
   if (i >= a.ni || j >= a.nj) return;
   const DField ua = dfield((double*)ua_a, 3, a.ni + 1, a.nj), va = dfield((double*)va_a, 3, a.ni, a.nj + 1);
@@ -491,14 +495,14 @@ __global__ void __launch_bounds__(kMxX* kMxY, 8) k_weno5_advect_mixed(const doub
 // derivatives is certain (almost everywhere) the update uses one of the two, and only that
 // one is evaluated; the other nodes put the second evaluation on the block's list, which
 // the block works off densely.  The results equal k_reinit_sweep_mixed's bit for bit.
-// ring: as k_reinit_sweep_exact.
+// The ghost ring: as k_reinit_sweep_exact.
 // Level-set TVD-RK3 with its 75 sweeps at 1024^2: 1.98 ms with four derivatives per node
 // (703 instructions a node), 1.64 ms with the chosen ones, 1.55 ms with the six differences
 // of a direction read once and weno5_side_f32 (507), 1.43 ms with 8 blocks per SM instead
 // of 6 (32 registers; staging, FP64 differences and evaluation of different blocks overlap).
 // Tiles of 32 x 16: 1.72 ms, of 32 x 4: 1.57.
 __global__ void __launch_bounds__(kMxX* kMxY, 8) k_reinit_sweep_tiled(const double* __restrict__ src_a, double* __restrict__ dst_a,
-                                                                   const double* __restrict__ S, LSArgs a, double dtau, int ring) {
+                                                                   const double* __restrict__ S, LSArgs a, double dtau) {
   constexpr int NT = kMxX * kMxY;
   pdl_enter();
   __shared__ MixedTile t;
@@ -507,12 +511,13 @@ __global__ void __launch_bounds__(kMxX* kMxY, 8) k_reinit_sweep_tiled(const doub
   __shared__ int count;
   const int ni = a.ni, nj = a.nj, tx = threadIdx.x, ty = threadIdx.y, tid = ty * kMxX + tx;
   const DField src = dfield((double*)src_a, 2, ni, nj), dst = dfield(dst_a, 2, ni, nj);
-  if (ring && blockIdx.y == gridDim.y - 1) {
+  const int by = a.row0 + (int)blockIdx.y;
+  if (by == a.rows) {
     copy_ring(src, dst, blockIdx.x * NT + tid, gridDim.x * NT);
     return;
   }
   if (tid == 0) count = 0;
-  const int i0 = (int)blockIdx.x * kMxX, j0 = (int)blockIdx.y * kMxY, i = i0 + tx, j = j0 + ty;
+  const int i0 = (int)blockIdx.x * kMxX, j0 = by * kMxY, i = i0 + tx, j = j0 + ty;
   const bool fast = stage_mixed(t, src, a, i0, j0);
   const bool in = i < ni && j < nj;
   const double sv = in ? __ldg(&S[i + (size_t)j * ni]) : 0.0;
@@ -590,6 +595,7 @@ struct EnoArgs {
   // FP32 path, per face grid: 1/h, 1/(2h), 1/(3h), h for x ([0..3]) and y ([4..7])
   float xs_f[8], ys_f[8];
   int fast;  // cell sizes in [2^-30, 2^30]
+  int row0;  // the launch's first tile row
 };
 
 // x / 4, exact but for subnormal results, without the FP64 pipe.
@@ -662,7 +668,7 @@ __global__ void __launch_bounds__(kEnX* kEnY) k_eno3(double* __restrict__ u_a, d
   __shared__ EnoTile<R> t;
   const bool xc = blockIdx.z == 0;
   const int nI = a.ni + (xc ? 1 : 0), nJ = a.nj + (xc ? 0 : 1);
-  const int i0 = (int)blockIdx.x * kEnX, j0 = (int)blockIdx.y * kEnY;
+  const int i0 = (int)blockIdx.x * kEnX, j0 = (a.row0 + (int)blockIdx.y) * kEnY;
   if (i0 >= nI || j0 >= nJ) return;
   const DField ua = dfield((double*)ua_a, 3, a.ni + 1, a.nj), va = dfield((double*)va_a, 3, a.ni, a.nj + 1);
   const DField& g = xc ? ua : va;
@@ -1096,12 +1102,13 @@ __global__ void k_fsm_sweep(double* phi_a, const double* __restrict__ fixed, int
 
 inline dim3 grid2d(int W, int H, dim3 blk) { return dim3((W + blk.x - 1) / blk.x, (H + blk.y - 1) / blk.y); }
 
-LSArgs ls_args(const gb2d_ctx* c) {
+LSArgs ls_args(const gb2d_ctx* c, int tile_y) {
   return LSArgs{c->grid.ni, c->grid.nj, c->base.odx, c->base.ody, c->prm.weno_epsilon,
                 (float)c->base.odx, (float)c->base.ody, (float)c->prm.weno_epsilon,
                 c->prm.weno_epsilon >= 1e-15 && c->prm.weno_epsilon <= 1e8,
                 c->prm.weno_epsilon >= 0x1p-100 && c->prm.weno_epsilon <= 0x1p100 &&
-                    c->base.dx >= 0x1p-300 && c->base.dx <= 0x1p300};
+                    c->base.dx >= 0x1p-300 && c->base.dx <= 0x1p300,
+                0, (c->grid.nj + tile_y - 1) / tile_y};
 }
 
 AsmArgs asm_args(const gb2d_ctx* c, double dt) {
@@ -1192,15 +1199,17 @@ void launch_extrapolate_ghosts(cudaStream_t s, double* f, int g, int nI, int nJ)
 }
 
 void launch_weno5_advect(cudaStream_t s, const gb2d_ctx* c, const double* src, double* dst, double dt, int mixed) {
-  const int ni = c->grid.ni, nj = c->grid.nj;
-  if (mixed) {
-    const dim3 grd((ni + kMxX - 1) / kMxX, (nj + kMxY - 1) / kMxY + 1);
-    pdl_launch(s, grd, dim3(kMxX, kMxY), 0, k_weno5_advect_mixed, src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
-  } else {
-    const dim3 grd((ni + kExX - 1) / kExX, (nj + kExY - 1) / kExY + 1);
-    pdl_launch(s, grd, 2 * kExX * kExY, 0, k_weno5_advect_exact, src, dst, c->ua, c->va, ls_args(c), DtArg{dt, c->dt_dev});
-  }
-  GB_LAUNCHED(1);
+  const unsigned cols = (unsigned)((c->grid.ni + 31) / 32);
+  static_assert(kMxX == 32 && kExX == 32, "tile widths");
+  LSArgs a = ls_args(c, mixed ? kMxY : kExY);
+  for_tile_rows(a.rows + 1, [&](int first, unsigned n) {
+    a.row0 = first;
+    if (mixed)
+      pdl_launch(s, dim3(cols, n), dim3(kMxX, kMxY), 0, k_weno5_advect_mixed, src, dst, c->ua, c->va, a, DtArg{dt, c->dt_dev});
+    else
+      pdl_launch(s, dim3(cols, n), 2 * kExX * kExY, 0, k_weno5_advect_exact, src, dst, c->ua, c->va, a, DtArg{dt, c->dt_dev});
+    GB_LAUNCHED(1);
+  });
 }
 
 void launch_reinit_sign(cudaStream_t s, const gb2d_ctx* c, const double* phi, double* S) {
@@ -1217,17 +1226,22 @@ void launch_reinit_sweep(cudaStream_t s, const gb2d_ctx* c, const double* src, d
     const char* e = getenv("GB2D_REINIT_UNTILED");
     return e && e[0] == '1';
   }();
-  if (mixed && !untiled) {
-    const dim3 g((ni + kMxX - 1) / kMxX, (nj + kMxY - 1) / kMxY + (ring ? 1 : 0));
-    pdl_launch(s, g, dim3(kMxX, kMxY), 0, k_reinit_sweep_tiled, src, dst, S, ls_args(c), dtau, ring);
-  } else if (mixed) {
+  LSArgs a = ls_args(c, mixed ? kMxY : kExY);
+  if (mixed && untiled) {
     const dim3 blk(32, 8);
-    pdl_launch(s, grid2d(ni + 4, nj + 4, blk), blk, 0, k_reinit_sweep_mixed, src, dst, S, ls_args(c), dtau);
-  } else {
-    const dim3 g((ni + kExX - 1) / kExX, (nj + kExY - 1) / kExY + (ring ? 1 : 0));
-    pdl_launch(s, g, 2 * kExX * kExY, 0, k_reinit_sweep_exact, src, dst, S, ls_args(c), dtau, ring);
+    pdl_launch(s, grid2d(ni + 4, nj + 4, blk), blk, 0, k_reinit_sweep_mixed, src, dst, S, a, dtau);
+    GB_LAUNCHED(1);
+    return;
   }
-  GB_LAUNCHED(1);
+  const unsigned cols = (unsigned)((ni + 31) / 32);
+  for_tile_rows(a.rows + (ring ? 1 : 0), [&](int first, unsigned n) {
+    a.row0 = first;
+    if (mixed)
+      pdl_launch(s, dim3(cols, n), dim3(kMxX, kMxY), 0, k_reinit_sweep_tiled, src, dst, S, a, dtau);
+    else
+      pdl_launch(s, dim3(cols, n), 2 * kExX * kExY, 0, k_reinit_sweep_exact, src, dst, S, a, dtau);
+    GB_LAUNCHED(1);
+  });
 }
 
 void launch_blend(cudaStream_t s, const gb2d_ctx* c, const double* keep, double* phi, double c0, double c1) {
@@ -1252,12 +1266,15 @@ void launch_eno3(cudaStream_t s, const gb2d_ctx* c, double dt) {
   }
   auto mid = [](double x) { return x >= 0x1p-30 && x <= 0x1p30; };
   a.fast = mid(c->xs.dx) && mid(c->xs.dy) && mid(c->ys.dx) && mid(c->ys.dy);
-  const dim3 grd((c->grid.ni + kEnX) / kEnX, (c->grid.nj + kEnY) / kEnY, 2);  // covers ni + 1 and nj + 1 faces
-  if (c->prm.advection_precision == GB2D_PRECISION_MIXED)
-    pdl_launch(s, grd, kEnX * kEnY, 0, k_eno3<true>, c->u, c->v, c->ua, c->va, a, DtArg{dt, c->dt_dev});
-  else
-    pdl_launch(s, grd, kEnX * kEnY, 0, k_eno3<false>, c->u, c->v, c->ua, c->va, a, DtArg{dt, c->dt_dev});
-  GB_LAUNCHED(1);
+  for_tile_rows((c->grid.nj + kEnY) / kEnY, [&](int first, unsigned n) {  // covers ni + 1 and nj + 1 faces
+    a.row0 = first;
+    const dim3 grd((c->grid.ni + kEnX) / kEnX, n, 2);
+    if (c->prm.advection_precision == GB2D_PRECISION_MIXED)
+      pdl_launch(s, grd, kEnX * kEnY, 0, k_eno3<true>, c->u, c->v, c->ua, c->va, a, DtArg{dt, c->dt_dev});
+    else
+      pdl_launch(s, grd, kEnX * kEnY, 0, k_eno3<false>, c->u, c->v, c->ua, c->va, a, DtArg{dt, c->dt_dev});
+    GB_LAUNCHED(1);
+  });
 }
 
 void launch_curvature(cudaStream_t s, const gb2d_ctx* c, const double* phi, double* kappa, int* flag) {

@@ -50,6 +50,7 @@ struct FlowArgs {
   float odx_f, ody_f, eps_f, oe_f, dt_f, coef0_f, coef1_f;
   SmearF rho_f, mu_f;
   int fast;            // densities, viscosities and cell sizes are in the fast products' range
+  int row0;            // the viscous launch's first tile row
 };
 
 // FP32 forms for the viscous flux of the mixed path.
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(kFlX* kFlY) k_flow_visc(const double* __restri
   __shared__ FlowTile<R> t;
   __shared__ FlowStep<R> st;
   const int ni = a.ni, nj = a.nj, tid = threadIdx.x;
-  const int i0 = (int)blockIdx.x * kFlX, j0 = (int)blockIdx.y * kFlY;
+  const int i0 = (int)blockIdx.x * kFlX, j0 = (a.row0 + (int)blockIdx.y) * kFlY;
   const DField phi = dfield((double*)phi_a, 2, ni, nj);
   const DField ui = dfield((double*)u_in, 2, ni + 1, nj), vi = dfield((double*)v_in, 2, ni, nj + 1);
   if (tid == 0) {
@@ -429,11 +430,16 @@ void launch_flow(cudaStream_t s, gb2d_ctx* c, double dt, int grav, int visc, int
     auto mid = [](double x) { return x == 0 || (std::fabs(x) >= 0x1p-60 && std::fabs(x) <= 0x1p60); };
     a.fast = mid(a.mu.lo) && mid(a.mu.at0) && mid(a.mu.at1) && mid(a.rho.at0) && mid(a.rho.at1) && mid(a.odx) && mid(a.ody) && a.odx > 0 &&
              a.ody > 0 && mid(c->prm.water_density) && mid(c->prm.air_density);
-    const dim3 grd((ni + kFlX) / kFlX, (nj + kFlY) / kFlY);  // covers ni + 1 and nj + 1 faces
-    if (mixed)
-      pdl_launch(s, grd, kFlX * kFlY, 0, k_flow_visc<float>, phi, (const double*)c->u, (const double*)c->v, c->u_alt, c->v_alt, density, a);
-    else
-      pdl_launch(s, grd, kFlX * kFlY, 0, k_flow_visc<double>, phi, (const double*)c->u, (const double*)c->v, c->u_alt, c->v_alt, density, a);
+    const double *u = c->u, *v = c->v;
+    for_tile_rows((nj + kFlY) / kFlY, [&](int first, unsigned n) {  // covers ni + 1 and nj + 1 faces
+      a.row0 = first;
+      const dim3 grd((ni + kFlX) / kFlX, n);
+      if (mixed)
+        pdl_launch(s, grd, kFlX * kFlY, 0, k_flow_visc<float>, phi, u, v, c->u_alt, c->v_alt, density, a);
+      else
+        pdl_launch(s, grd, kFlX * kFlY, 0, k_flow_visc<double>, phi, u, v, c->u_alt, c->v_alt, density, a);
+      GB_LAUNCHED(1);
+    });
     double* t = c->u;
     c->u = c->u_alt;
     c->u_alt = t;
@@ -441,10 +447,10 @@ void launch_flow(cudaStream_t s, gb2d_ctx* c, double dt, int grav, int visc, int
     c->v = c->v_alt;
     c->v_alt = t;
   } else {
-    a.fast = 0;
+    a.fast = a.row0 = 0;
     pdl_launch(s, grid_ij(ni + 1, nj + 1), kThreads, 0, k_flow, phi, c->u, c->v, density, a);
+    GB_LAUNCHED(1);
   }
-  GB_LAUNCHED(1);
 }
 
 void launch_face_blend(cudaStream_t s, gb2d_ctx* c, double c0, double c1) {

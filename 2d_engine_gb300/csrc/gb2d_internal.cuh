@@ -116,6 +116,13 @@ inline dim3 grid_ij(int nI, int nJ) {
   return dim3(gx, gy);
 }
 
+// Launches over tile rows, at most 65535 (a grid's y extent) at a time: f(first row, rows).  A
+// 4-row tile would otherwise refuse grids of more than 262140 rows.
+template <typename F>
+void for_tile_rows(int rows, F f) {
+  for (int r = 0; r < rows; r += 65535) f(r, (unsigned)(rows - r < 65535 ? rows - r : 65535));
+}
+
 // One multigrid level (cell-centred view of the node grid), padded with a zero
 // ring: cell (i, j) at (i+1) + (j+1)*ld, ld = nI + 2.  cx at the same index is the
 // conductance of the face between (i-1, j) and (i, j) (i = 0..nI), cy the face
