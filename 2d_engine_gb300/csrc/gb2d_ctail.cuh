@@ -38,7 +38,13 @@ constexpr int kCtThreads = 512;
 constexpr int kCtMaxLevels = 10;
 constexpr int kCtMinRows = 4;           // rows per CTA on the coarsest distributed level
 constexpr int kCtOwnerRows = 256;       // rows of the bottom distributed level at most
-constexpr int kCtPairs = 2, kCtPairsMax = 6;  // cell pairs per thread: the usual and the largest kernel
+// Cell pairs per thread of the usual and of the largest kernel.  FP64: three fill the 128
+// registers that a thread of 512 may have (72 bytes of spills; with four 548, with six 2080,
+// which cost more than the launches that the cluster replaces: 121 x 132 to 1e-10 2.05 ms
+// before the pairs were in registers, 2.38 with the kernel of six, 1.69 with that of three).
+constexpr int kCtPairs = 2;
+template <typename T>
+constexpr int kCtPairsMax = sizeof(T) == 8 ? 3 : 6;
 constexpr size_t kCtSmemCap = 220 * 1024;
 // Largest top level: a 256^2 FP32 level fits in the cluster's shared memory, but
 // measured at 1024^2 the projection is faster with 256^2 in the tiled kernels

@@ -1656,7 +1656,7 @@ bool layout_ctail(const CtArgs<T>& base, const int* stripe, int nu, CtArgs<T>* o
     off += nc * nc * (int)(sizeof(double) / sizeof(T));
   }
   a.kpairs = (items + kCtThreads - 1) / kCtThreads;
-  if ((size_t)off * sizeof(T) > kCtSmemCap || a.kpairs > kCtPairsMax) return false;
+  if ((size_t)off * sizeof(T) > kCtSmemCap || a.kpairs > kCtPairsMax<T>) return false;
   *out = a;
   *bytes = (size_t)off * sizeof(T);
   return true;
@@ -1741,7 +1741,11 @@ bool plan_ctail_from(Hierarchy<T>& H, int P, bool small) {
     if (!deeper) {
       distribute(nd);
       for (int nu = 1; nu <= 3 && ok; ++nu) ok = layout_ctail(a, stripe, nu, &H.ct[nu - 1], &H.ct_smem[nu - 1]);
-      if (!ok || (P == 1 && H.ct[0].kpairs > kCtPairs)) continue;  // one CTA: mixed 60 x 50 0.95 -> 1.02 ms
+      // Not with more than two pairs a thread where that is one CTA's (mixed 60 x 50 0.95 -> 1.02 ms)
+      // or FP64: a wide level of few rows, most of whose window every CTA repeats (1000 x 16 to
+      // 1e-10, 500 x 8 in four CTAs: 1.10 ms with the single-CTA tail, 1.25 here).  From the finest
+      // level down the cluster holds the whole CG and wins all the same (171 x 13: 0.87, 0.67 here).
+      if (!ok || (P == 1 && H.ct[0].kpairs > kCtPairs) || (small && top > 0 && sizeof(T) == 8 && H.ct[1].kpairs > kCtPairs)) continue;
     }
     H.ctail = top;
     H.ct_P = P;
@@ -1778,10 +1782,14 @@ int ctail_cluster_size() {
   static int cached = -1;
   if (cached >= 0) return cached;
   cached = 0;
-  const void* kernels[8] = {(const void*)k_ctail<float, kCtPairs>,         (const void*)k_ctail<double, kCtPairs>,
-                            (const void*)k_ctail<float, kCtPairsMax>,      (const void*)k_ctail<double, kCtPairsMax>,
-                            (const void*)k_cg_cluster<float, kCtPairs>,    (const void*)k_cg_cluster<double, kCtPairs>,
-                            (const void*)k_cg_cluster<float, kCtPairsMax>, (const void*)k_cg_cluster<double, kCtPairsMax>};
+  const void* kernels[8] = {(const void*)k_ctail<float, kCtPairs>,
+                            (const void*)k_ctail<double, kCtPairs>,
+                            (const void*)k_ctail<float, kCtPairsMax<float>>,
+                            (const void*)k_ctail<double, kCtPairsMax<double>>,
+                            (const void*)k_cg_cluster<float, kCtPairs>,
+                            (const void*)k_cg_cluster<double, kCtPairs>,
+                            (const void*)k_cg_cluster<float, kCtPairsMax<float>>,
+                            (const void*)k_cg_cluster<double, kCtPairsMax<double>>};
   bool attr_ok = true;
   for (const void* k : kernels)
     attr_ok = attr_ok && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
@@ -1837,7 +1845,7 @@ void launch_ctail(cudaStream_t s, const Hierarchy<T>& H, const double* ainv, int
   cfg.stream = s;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, a.kpairs <= kCtPairs ? k_ctail<T, kCtPairs> : k_ctail<T, kCtPairsMax>, a, ainv, nu, done);
+  cudaLaunchKernelEx(&cfg, a.kpairs <= kCtPairs ? k_ctail<T, kCtPairs> : k_ctail<T, kCtPairsMax<T>>, a, ainv, nu, done);
 }
 
 // The cluster CG serves grids whose finest level the cluster tail holds.
@@ -1879,7 +1887,7 @@ void launch_cg_cluster(cudaStream_t s, Solver* S, const Hierarchy<T>& H, const d
   cfg.stream = s;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, g.a.kpairs <= kCtPairs ? k_cg_cluster<T, kCtPairs> : k_cg_cluster<T, kCtPairsMax>, g);
+  cudaLaunchKernelEx(&cfg, g.a.kpairs <= kCtPairs ? k_cg_cluster<T, kCtPairs> : k_cg_cluster<T, kCtPairsMax<T>>, g);
   GB_LAUNCHED(1);
 }
 
