@@ -495,14 +495,14 @@ __global__ void __launch_bounds__(kMxX* kMxY, 8) k_weno5_advect_mixed(const doub
 // derivatives is certain (almost everywhere) the update uses one of the two, and only that
 // one is evaluated; the other nodes put the second evaluation on the block's list, which
 // the block works off densely.  The results equal k_reinit_sweep_mixed's bit for bit.
-// The ghost ring: as k_reinit_sweep_exact.
+// ring: the grid's last block row copies src's ghost ring.
 // Level-set TVD-RK3 with its 75 sweeps at 1024^2: 1.98 ms with four derivatives per node
 // (703 instructions a node), 1.64 ms with the chosen ones, 1.55 ms with the six differences
 // of a direction read once and weno5_side_f32 (507), 1.43 ms with 8 blocks per SM instead
 // of 6 (32 registers; staging, FP64 differences and evaluation of different blocks overlap).
 // Tiles of 32 x 16: 1.72 ms, of 32 x 4: 1.57.
 __global__ void __launch_bounds__(kMxX* kMxY, 8) k_reinit_sweep_tiled(const double* __restrict__ src_a, double* __restrict__ dst_a,
-                                                                   const double* __restrict__ S, LSArgs a, double dtau) {
+                                                                   const double* __restrict__ S, LSArgs a, double dtau, int ring) {
   constexpr int NT = kMxX * kMxY;
   pdl_enter();
   __shared__ MixedTile t;
@@ -511,13 +511,12 @@ __global__ void __launch_bounds__(kMxX* kMxY, 8) k_reinit_sweep_tiled(const doub
   __shared__ int count;
   const int ni = a.ni, nj = a.nj, tx = threadIdx.x, ty = threadIdx.y, tid = ty * kMxX + tx;
   const DField src = dfield((double*)src_a, 2, ni, nj), dst = dfield(dst_a, 2, ni, nj);
-  const int by = a.row0 + (int)blockIdx.y;
-  if (by == a.rows) {
+  if (ring && blockIdx.y == gridDim.y - 1) {
     copy_ring(src, dst, blockIdx.x * NT + tid, gridDim.x * NT);
     return;
   }
   if (tid == 0) count = 0;
-  const int i0 = (int)blockIdx.x * kMxX, j0 = by * kMxY, i = i0 + tx, j = j0 + ty;
+  const int i0 = (int)blockIdx.x * kMxX, j0 = (int)blockIdx.y * kMxY, i = i0 + tx, j = j0 + ty;
   const bool fast = stage_mixed(t, src, a, i0, j0);
   const bool in = i < ni && j < nj;
   const double sv = in ? __ldg(&S[i + (size_t)j * ni]) : 0.0;
@@ -1234,12 +1233,14 @@ void launch_reinit_sweep(cudaStream_t s, const gb2d_ctx* c, const double* src, d
     return;
   }
   const unsigned cols = (unsigned)((ni + 31) / 32);
+  if (mixed) {  // one launch, up to 524280 rows: an offset of the tile rows costs it 0.5%
+    pdl_launch(s, dim3(cols, a.rows + (ring ? 1 : 0)), dim3(kMxX, kMxY), 0, k_reinit_sweep_tiled, src, dst, S, a, dtau, ring);
+    GB_LAUNCHED(1);
+    return;
+  }
   for_tile_rows(a.rows + (ring ? 1 : 0), [&](int first, unsigned n) {
     a.row0 = first;
-    if (mixed)
-      pdl_launch(s, dim3(cols, n), dim3(kMxX, kMxY), 0, k_reinit_sweep_tiled, src, dst, S, a, dtau);
-    else
-      pdl_launch(s, dim3(cols, n), 2 * kExX * kExY, 0, k_reinit_sweep_exact, src, dst, S, a, dtau);
+    pdl_launch(s, dim3(cols, n), 2 * kExX * kExY, 0, k_reinit_sweep_exact, src, dst, S, a, dtau);
     GB_LAUNCHED(1);
   });
 }

@@ -24,9 +24,10 @@ def run(gb, f, ni, nj, prec, what):
     c.set_flow_params(water_viscosity=1.0, air_viscosity=0.01, viscosity=True)
     for k, a in f.items():
         c.set(getattr(gb, "FIELD_" + k), np.ascontiguousarray(a))
-    if what == "levelset":
+    if what in ("levelset", "advection"):
         c.levelset_advection(0.2 * H)
-        c.reinitialization()
+        if what == "levelset":
+            c.reinitialization()
         out = [c.get(gb.FIELD_PHI)]
     else:
         c.velocity_advection(0.1 * H)
@@ -36,8 +37,8 @@ def run(gb, f, ni, nj, prec, what):
     return out
 
 
-# 262140 rows are 65535 tiles of 4, 524280 of 8.
-@pytest.mark.parametrize("what,prec,nj", [("levelset", 0, 262140), ("levelset", 0, 262141), ("levelset", 0, 300001), ("levelset", 1, 524281),
+# 262140 rows are 65535 tiles of 4, 524280 of 8 (the mixed reinitialisation's limit).
+@pytest.mark.parametrize("what,prec,nj", [("levelset", 0, 262140), ("levelset", 0, 262141), ("levelset", 0, 300001), ("advection", 1, 524281), ("levelset", 1, 262141),
                                           ("velocity", 0, 524281), ("velocity", 1, 524400)])
 def test_rows_beyond_one_launch(gb, what, prec, nj):
     ni, short = 5, 600
@@ -46,4 +47,4 @@ def test_rows_beyond_one_launch(gb, what, prec, nj):
     ref = run(gb, {k: a[nj - short:] for k, a in f.items()}, ni, short, prec, what)
     for a, b in zip(tall, ref):
         np.testing.assert_array_equal(a[nj - short:][40:], b[40:])
-        assert not np.array_equal(a[nj - short:][40:-40], f["PHI" if what == "levelset" else "U"][nj - short:][40:-40])
+        assert not np.array_equal(a[nj - short:][40:-40], f["U" if what == "velocity" else "PHI"][nj - short:][40:-40])
