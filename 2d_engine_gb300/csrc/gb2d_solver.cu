@@ -2142,7 +2142,11 @@ void precondition(cudaStream_t s, Solver* S, Hierarchy<T>& H, const double* ainv
 
 template <typename T>
 auto apply_kernel(const Solver* S) {
-  return sizeof(T) == 4 && (long)S->ni * S->nj >= (1L << 21) ? k_apply_pap<T, sizeof(T) == 4> : k_apply_pap<T, false>;
+  static const bool off = [] {  // GB2D_APPLY_INT=0 (read once): the plain product on every grid, for comparison
+    const char* e = getenv("GB2D_APPLY_INT");
+    return e && e[0] == '0';
+  }();
+  return sizeof(T) == 4 && !off && (long)S->ni * S->nj >= (1L << 21) ? k_apply_pap<T, sizeof(T) == 4> : k_apply_pap<T, false>;
 }
 
 // First direction: z = M r, p = z, Ap, alpha.
