@@ -135,8 +135,10 @@ __global__ void __launch_bounds__(kCoefThreads) k_weno5_adj_coef(const double* _
       const int d = up ? m - 3 : 3 - m;
       q[m] = y ? GB_AT(phi, i, clamp_line(j + d, nj)) : GB_AT(phi, clamp_line(i + d, ni), j);
     }
-    weno5_side_grad(q, os, -a.dt * vel * l * os, a.eps, f, J);
-    coef[(up ? 6 : 0) * n + t] = 0.0;
+    const double w = -a.dt * vel * l;
+    weno5_side_grad(q, os, w * os, a.eps, f, J);
+    // The unused end of the stencil: w times zero, NaN where w is not finite.
+    coef[(up ? 6 : 0) * n + t] = from_words(0u, (words(w).hi & 0x7ff00000u) == 0x7ff00000u ? 0x7ff80000u : 0u);
 #pragma unroll
     for (int m = 0; m < 6; ++m) coef[(up ? m : 6 - m) * n + t] = J[m];
     gvel[t] = dl * f * 0.5;
