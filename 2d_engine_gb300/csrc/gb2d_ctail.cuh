@@ -46,9 +46,9 @@ constexpr int kCtPairs = 2;
 template <typename T>
 constexpr int kCtPairsMax = sizeof(T) == 8 ? 3 : 6;
 constexpr size_t kCtSmemCap = 220 * 1024;
-// Largest top level: a 256^2 FP32 level fits in the cluster's shared memory, but
-// measured at 1024^2 the projection is faster with 256^2 in the tiled kernels
-// (one launch per smoothing side, no cluster barriers) and the cluster from 128^2.
+// Largest top level.  From 64^2 instead, the mixed projection at 1024^2 takes 1.96 ms
+// against 1.94 (at 256^2 0.81 against 0.79); a 256^2 level in 16 CTAs would take seven pairs
+// a thread with three sweeps a side, more than the largest kernel has.
 constexpr int kCtMaxTopCells = 128 * 128;
 
 // Shared-memory offsets are in elements of T.  A plane holds one colour of a level's

@@ -1259,16 +1259,18 @@ __global__ void k_end_device(const Scalars* sc, Scalars* fs, int last) {
 // Where the cluster tail holds the finest level (at most 128^2 cells), a CG iteration was
 // four launches of a few microseconds each around vectors of some 100 KB: launch and
 // reduction latency (64^2: 28 us of kernels and 6 of gaps). This kernel runs the whole
-// iteration loop in the tail's cluster: vectors in global memory (L2), five cluster
-// barriers an iteration (residual; the V-cycle's two and r.z; direction; p.Ap), no host.
+// iteration loop in the tail's cluster: vectors in global memory (L2), no host.  Cluster
+// barriers an iteration: four (residual, r.z, direction, p.Ap), one a distributed level, and
+// one where the first CTA sums r.z: 5 at 64^2 mixed, 7 at 128^2 FP64.
 // Every number equals the launched kernels': their blocks of 256 threads become the
 // halves of a CTA, with the same elements, the same sums and the same order of partials.
 // Vectors that another CTA wrote are read through L2 (__ldcg); the partials of the sums go
 // into every CTA's shared memory (64^2: 0.503 -> 0.480 ms against partials in global memory
 // and FP64 divisions).  Every CTA computes the same scalars from the same partials, so that
-// all take the same branches; at most pass_cap(max_it) iterations.  Measured: the mixed projection at
-// 64^2 0.60 -> 0.48 ms, an iteration 34 -> 19 us (the V-cycle half of them); a bubble frame at
-// 128^2 (FP64) 3.70 -> 3.62 ms, whose V-cycles are bound by 16 SMs' FP64 pipes.
+// all take the same branches; at most pass_cap(max_it) iterations.  Against the launched
+// kernels (GB2D_CLUSTER_CG=0): the mixed projection at 64^2 0.52 -> 0.40 ms, an FP64 one at
+// 128^2 1.13 -> 1.04, a bubble frame at 128^2 (FP64) 3.70 -> 3.50.  At 128^2 the 16 SMs' FP64
+// pipes are busy 45% of the time, the rest is barriers and waits for dependent results.
 constexpr int kCgBlocks = 64;  // 128^2 cells
 template <typename T>
 struct CgArgs {
@@ -1708,7 +1710,13 @@ bool plan_ctail_from(Hierarchy<T>& H, int P, bool small) {
     };
     const int nd = lb - top + 1;
     bool ok = distribute(nd);
-    size_t cells = 0;  // six padded stripes per level must fit in one CTA's shared memory
+    // The 128^2 form's size bound: six padded stripes per level within one CTA's shared memory.
+    // layout_ctail below checks what the windows need, which is less; the bound keeps wide FP64
+    // levels in the tiled launches, which fill more SMs (128 x 97, see plan_ctail), and each
+    // grid's choice of form, which fixes its sums' order, where it was.  It is not the fastest
+    // choice for every grid that it turns away: those between 64^2 and 128^2 cells in FP64 were
+    // not measured in the other form.
+    size_t cells = 0;
     for (int l = 0; l < a.nlev; ++l) {
       const Level<T>& L = H.L[top + l];
       CtLevel<T>& C = a.L[l];
@@ -1743,7 +1751,7 @@ bool plan_ctail_from(Hierarchy<T>& H, int P, bool small) {
       for (int nu = 1; nu <= 3 && ok; ++nu) ok = layout_ctail(a, stripe, nu, &H.ct[nu - 1], &H.ct_smem[nu - 1]);
       // Not with more than two pairs a thread where that is one CTA's (mixed 60 x 50 0.95 -> 1.02 ms)
       // or FP64: a wide level of few rows, most of whose window every CTA repeats (1000 x 16 to
-      // 1e-10, 500 x 8 in four CTAs: 1.10 ms with the single-CTA tail, 1.25 here).  From the finest
+      // 1e-10, 500 x 8 in four CTAs: 1.01 ms with that level in the tiled launches, 1.25 here).  From the finest
       // level down the cluster holds the whole CG and wins all the same (171 x 13: 0.87, 0.67 here).
       if (!ok || (P == 1 && H.ct[0].kpairs > kCtPairs) || (small && top > 0 && sizeof(T) == 8 && H.ct[1].kpairs > kCtPairs)) continue;
     }

@@ -165,8 +165,8 @@ int gb2d_check_exact_division(unsigned long long n, unsigned long long seed, uns
 
 /* Multigrid layout of the pressure solver for one precision (GB2D_PRECISION_FP64
  * or GB2D_PRECISION_MIXED, whose V-cycles run in FP32): the number of levels, the
- * first level handled by the thread-block-cluster tail kernel (-1 when the
- * single-CTA tail is used instead) and that cluster's CTA count.  No counterpart
+ * first level handled by the thread-block-cluster tail kernel (-1 when one CTA
+ * handles the coarse levels, by whichever kernel) and that cluster's CTA count.  No counterpart
  * in the reference (diagnostics). */
 int gb2d_solver_layout(gb2d_ctx* ctx, int precision, int* levels, int* cluster_top, int* cluster_ctas);
 
